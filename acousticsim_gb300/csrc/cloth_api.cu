@@ -128,8 +128,12 @@ struct Batch
     bool persist_ok = false;
     bool persist_sm = false; // own-row state in shared memory
     bool persist_1b = false; // single-barrier variant (shared memory, every halo staged)
+    bool persist_team = false; // k_pcg_team: the matrix on chip
+    int team_chunks = 1;       // its chunks per warp
     TeamBlock *d_work = nullptr;
-    int grid_persist = 0;
+    char *d_sync = nullptr;    // behind the work list: arrival counts or team sums
+    size_t sync_bytes = 0;
+    int grid_persist = 0, block_persist = kPBlock;
     int halo_cap = 0, rows_cap = 0;
     size_t smem_persist = 0;
     SpinCfg spin = {kSpinLimitDefault, 0u}; // the context's setting when the set was built
@@ -818,12 +822,139 @@ int make_batch(cloth_ctx *ctx, const std::vector<cloth_s *> &members,
 // The persistent kernel a plan launches.
 const void *persistent_kernel(const Batch *b)
 {
+    if (b->persist_team)
+        return team_kernel(b->team_chunks, b->skew);
     if (b->persist_1b)
         return (const void *)k_pcg1_persistent;
     if (b->skew)
         return b->persist_sm ? (const void *)k_pcg_persistent_sm_skew
                              : (const void *)k_pcg_persistent_gm_skew;
     return b->persist_sm ? (const void *)k_pcg_persistent_sm : (const void *)k_pcg_persistent_gm;
+}
+
+// The persistent kernels' arguments (k_pcg_team takes fewer).
+struct PersistArgs
+{
+    void *team[4], *two[5];
+    explicit PersistArgs(Batch *b)
+        : team{&b->d_descs, &b->d_work, &b->d_sync, &b->spin},
+          two{&b->d_descs, &b->d_work, &b->halo_cap, &b->rows_cap, &b->spin}
+    {
+    }
+    void **of(const Batch *b) { return b->persist_team ? team : two; }
+};
+
+// The work list of a persistent launch, and behind it per_block bytes for
+// every block, zeroed before each launch.
+int upload_work(Batch *b, const std::vector<TeamBlock> &work, size_t per_block, size_t align)
+{
+    const size_t at = align_up(work.size() * sizeof(TeamBlock), align);
+    b->sync_bytes = work.size() * per_block;
+    CK(cudaMalloc(&b->d_work, at + b->sync_bytes));
+    b->d_sync = reinterpret_cast<char *>(b->d_work) + at;
+    CK(cudaMemcpy(b->d_work, work.data(), work.size() * sizeof(TeamBlock),
+                  cudaMemcpyHostToDevice));
+    b->grid_persist = int(work.size());
+    b->persist_ok = true;
+    return CLOTH_OK;
+}
+
+// One block's rows [r0, r1) and the columns they touch.
+TeamBlock team_block(const Tables &t, int inst, int rank, int r0, int r1)
+{
+    TeamBlock w{inst, rank, 1, r0, r1, r0, r1, 0};
+    int lo = r0, hi = r1 - 1;
+    for (int v = r0; v < r1; v++)
+    {
+        lo = std::min(lo, t.cols[t.rowptr[v]]);
+        hi = std::max(hi, t.cols[t.rowptr[v + 1] - 1]);
+    }
+    w.halo0 = lo;
+    w.halo1 = hi + 1;
+    return w;
+}
+
+// Plan of k_pcg_team: every block's rows, their blocks and p over their
+// columns in its shared memory.  False when the set does not fit that way.
+bool plan_team(cloth_ctx *ctx, const Batch *b, std::vector<TeamBlock> &work, size_t &smem,
+               int &chunks)
+{
+    const int G = std::min(ctx->num_sms, kTeamMaxBlocks);
+    const int n = int(b->members.size());
+    if (n > G)
+        return false;
+    const size_t cap = size_t(ctx->max_smem_optin) - 4096;
+    // the split of instance i into blocks of `rows` rows: its blocks, or none
+    // when one does not fit
+    auto split = [&](int i, int rows, std::vector<TeamBlock> &out, size_t &bytes) {
+        const cloth_s *c = b->members[i];
+        const Tables &t = c->tab;
+        out.clear();
+        bytes = 0;
+        for (int r0 = 0; r0 < t.nv; r0 += rows)
+        {
+            out.push_back(team_block(t, i, int(out.size()), r0, std::min(t.nv, r0 + rows)));
+            const TeamBlock &w = out.back();
+            bytes = std::max(bytes, team_smem_bytes(w.halo1 - w.halo0, w.row1 - w.row0,
+                                                    c->h.width, c->h.Aw != nullptr));
+            if (bytes > cap || w.halo1 - w.halo0 > 65535)
+                return false;
+        }
+        for (auto &w : out)
+            w.nblk = int(out.size());
+        return int(out.size()) <= G;
+    };
+    auto rows_of = [](int nv, int blocks) {
+        return ((nv + blocks - 1) / blocks + kRedRows - 1) / kRedRows * kRedRows;
+    };
+    long long total = 0;
+    for (auto *c : b->members)
+        total += c->tab.nv;
+    std::vector<std::vector<TeamBlock>> teams(n);
+    std::vector<size_t> bytes(n);
+    int used = 0;
+    for (int i = 0; i < n; i++)
+    {
+        const int nv = b->members[i]->tab.nv;
+        long long share = std::max(1ll, (long long)(G - (n - 1)) * nv / std::max(1ll, total));
+        if (nv <= kTeamSingleRows && split(i, rows_of(nv, 1), teams[i], bytes[i]))
+        {
+            used++;
+            continue;
+        }
+        const int want = std::max(1, std::min<int>(int(share), (nv + kTeamMinRows - 1) / kTeamMinRows));
+        const int rows = rows_of(nv, want);
+        if (rows > 2 * kTeamWorkers || !split(i, rows, teams[i], bytes[i]))
+            return false;
+        used += int(teams[i].size());
+    }
+    if (used > G)
+        return false;
+    smem = 0;
+    int most = 0;
+    work.clear();
+    for (int i = 0; i < n; i++)
+    {
+        smem = std::max(smem, bytes[i]);
+        for (const auto &w : teams[i])
+        {
+            most = std::max(most, w.row1 - w.row0);
+            work.push_back(w);
+        }
+    }
+    chunks = most > kTeamWorkers ? 2 : 1;
+    const void *f = team_kernel(chunks, b->skew);
+    int occ = 0;
+    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, int(cap)) !=
+            cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, f, kTeamThreads, smem) !=
+            cudaSuccess ||
+        occ * ctx->num_sms < int(work.size()))
+    {
+        cudaGetLastError();
+        return false;
+    }
+    return true;
 }
 
 // Team plan of the persistent solver: every instance gets blocks in
@@ -836,6 +967,15 @@ int plan_persistent(cloth_ctx *ctx, Batch *b)
     if (ctx->solver != CLOTH_SOLVER_PERSISTENT && ctx->solver != CLOTH_SOLVER_PERSISTENT_1B &&
         ctx->solver != CLOTH_SOLVER_PERSISTENT_2B)
         return CLOTH_OK;
+    std::vector<TeamBlock> work;
+    if (ctx->solver != CLOTH_SOLVER_PERSISTENT_1B &&
+        plan_team(ctx, b, work, b->smem_persist, b->team_chunks))
+    {
+        b->persist_team = true;
+        b->block_persist = kTeamThreads;
+        return upload_work(b, work, sizeof(TeamSync), alignof(TeamSync) * 64);
+    }
+    work.clear();
     const size_t smem_cap_bytes =
         std::min<size_t>(size_t(std::max(ctx->max_smem_optin, 48 * 1024)) - 4096,
                          200 * 1024);
@@ -912,7 +1052,6 @@ int plan_persistent(cloth_ctx *ctx, Batch *b)
         nb[worst]--;
         used--;
     }
-    std::vector<TeamBlock> work;
     int max_entries = 0, max_rows = 0;
     bool all_staged = true;
     for (int i = 0; i < n; i++)
@@ -927,21 +1066,7 @@ int plan_persistent(cloth_ctx *ctx, Batch *b)
         std::vector<TeamBlock> team;
         for (int r0 = 0; r0 < t.nv; r0 += chunk)
         {
-            TeamBlock w;
-            w.inst = i;
-            w.rank = rank++;
-            w.row0 = r0;
-            w.row1 = std::min(t.nv, r0 + chunk);
-            int lo = w.row0, hi = w.row1 - 1;
-            for (int v = w.row0; v < w.row1; v++)
-            {
-                lo = std::min(lo, t.cols[t.rowptr[v]]);
-                hi = std::max(hi, t.cols[t.rowptr[v + 1] - 1]);
-            }
-            w.halo0 = lo;
-            w.halo1 = hi + 1;
-            w.p_global = 0;
-            team.push_back(w);
+            team.push_back(team_block(t, i, rank++, r0, std::min(t.nv, r0 + chunk)));
         }
         bool team_staged = true;
         for (auto &w : team)
@@ -999,14 +1124,10 @@ int plan_persistent(cloth_ctx *ctx, Batch *b)
         cudaGetLastError();
         return CLOTH_OK;
     }
-    // the work list, then one arrival count per block slot (the team barrier
-    // of the two-barrier kernels), zeroed before every launch
-    CK(cudaMalloc(&b->d_work, work.size() * (sizeof(TeamBlock) + sizeof(unsigned long long))));
-    CK(cudaMemcpy(b->d_work, work.data(), work.size() * sizeof(TeamBlock),
-                  cudaMemcpyHostToDevice));
-    b->grid_persist = int(work.size());
-    b->persist_ok = true;
-    return CLOTH_OK;
+    // one arrival count per block slot (the team barrier of the two-barrier
+    // kernels) behind the work list
+    b->block_persist = kPBlock;
+    return upload_work(b, work, sizeof(unsigned long long), sizeof(TeamBlock));
 }
 
 int add_kernel(cudaGraph_t g, cudaGraphNode_t *node, const cudaGraphNode_t *deps,
@@ -1082,16 +1203,16 @@ int build_graph(Batch *b, bool full, cudaGraphExec_t *exec)
     if (b->persist_ok)
     {
         b->spin = b->ctx->spin;
-        void *a_per[] = {&b->d_descs, &b->d_work, &b->halo_cap, &b->rows_cap, &b->spin};
+        PersistArgs a_per(b);
         if (rc == CLOTH_OK)
         {
-            // the team barriers' arrival counts start at zero
+            // the team barriers' arrival counts (or team sums) start at zero
             cudaMemsetParams mp;
             std::memset(&mp, 0, sizeof(mp));
-            mp.dst = b->d_work + b->grid_persist;
+            mp.dst = b->d_sync;
             mp.value = 0;
             mp.elementSize = 4;
-            mp.width = size_t(b->grid_persist) * 2;
+            mp.width = b->sync_bytes / 4;
             mp.height = 1;
             if (cudaGraphAddMemsetNode(&n, g, last ? &last : nullptr, last ? 1 : 0, &mp) !=
                 cudaSuccess)
@@ -1105,9 +1226,9 @@ int build_graph(Batch *b, bool full, cudaGraphExec_t *exec)
             std::memset(&p, 0, sizeof(p));
             p.func = const_cast<void *>(persistent_kernel(b));
             p.gridDim = dim3(b->grid_persist);
-            p.blockDim = dim3(kPBlock);
+            p.blockDim = dim3(b->block_persist);
             p.sharedMemBytes = unsigned(b->smem_persist);
-            p.kernelParams = a_per;
+            p.kernelParams = a_per.of(b);
             if (cudaGraphAddKernelNode(&n, g, last ? &last : nullptr, last ? 1 : 0, &p) !=
                 cudaSuccess)
                 rc = fail(CLOTH_ERR_CUDA, "cudaGraphAddKernelNode(persistent) failed");
@@ -1209,12 +1330,11 @@ int launch_persistent(Batch *b)
     cloth_ctx *ctx = b->ctx;
     PhaseTimer t(ctx, PH_SPMV);
     b->spin = ctx->spin;
-    void *args[] = {&b->d_descs, &b->d_work, &b->halo_cap, &b->rows_cap, &b->spin};
-    CK(cudaMemsetAsync(b->d_work + b->grid_persist, 0,
-                       size_t(b->grid_persist) * sizeof(unsigned long long), ctx->stream));
-    CK(cudaLaunchCooperativeKernel(persistent_kernel(b),
-                                   dim3(b->grid_persist), dim3(kPBlock), args,
-                                   b->smem_persist, ctx->stream));
+    PersistArgs args(b);
+    CK(cudaMemsetAsync(b->d_sync, 0, b->sync_bytes, ctx->stream));
+    CK(cudaLaunchCooperativeKernel(persistent_kernel(b), dim3(b->grid_persist),
+                                   dim3(b->block_persist), args.of(b), b->smem_persist,
+                                   ctx->stream));
     return CLOTH_OK;
 }
 

@@ -247,6 +247,26 @@ struct SpinCfg
     unsigned extra;
 };
 
+// k_pcg_team: worker threads (one row each, or two) and the control warp; a
+// team's sum words, four iterations deep (p.q in words 0-2, r.z and r.r in
+// words 4-9), zeroed before every launch.
+constexpr int kTeamWorkers = 512;
+constexpr int kTeamThreads = kTeamWorkers + 32;
+constexpr int kTeamSingleRows = 640; // instances up to this size: a team of one block
+constexpr int kTeamMinRows = 64;     // rows a block of a larger team gets at least
+constexpr int kTeamMaxBlocks = 255; // a word counts its team's arrivals in one byte
+struct TeamSync
+{
+    unsigned long long words[4][16];
+};
+// Dynamic shared memory of a k_pcg_team block: p over its halo, and width
+// planes of blocks (skew parts), and local column indices over its rows.
+__host__ __device__ inline size_t team_smem_bytes(int halo, int rows, int width, bool skew)
+{
+    const size_t rp = size_t((rows + 31) / 32) * 32;
+    return size_t(halo) * 16 + size_t(width) * rp * (skew ? 42 : 26);
+}
+
 // One variant of a graph-loop kernel: R rows per thread (blocks of kTile / R
 // threads), U ELL slots whose loads are issued together (SpMV only), TPB
 // consecutive tiles taken by a block at a time.

@@ -20,85 +20,13 @@
 //
 // Reference kernels: src/sim/cloth/BaraffClothGpu.cu, src/sim/cloth/gpu_solvers/PCGSolver.cu.
 #include "device.cuh"
+#include "pcg_math.cuh"
 
 #include <type_traits>
 
 namespace cloth {
 
 namespace {
-
-__device__ __forceinline__ float3 operator+(float3 a, float3 b)
-{
-    return make_float3(a.x + b.x, a.y + b.y, a.z + b.z);
-}
-__device__ __forceinline__ float3 operator-(float3 a, float3 b)
-{
-    return make_float3(a.x - b.x, a.y - b.y, a.z - b.z);
-}
-__device__ __forceinline__ float3 operator*(float s, float3 a)
-{
-    return make_float3(s * a.x, s * a.y, s * a.z);
-}
-__device__ __forceinline__ float3 xyz(float4 v) { return make_float3(v.x, v.y, v.z); }
-__device__ __forceinline__ float4 f4(float3 v, float w = 0.f)
-{
-    return make_float4(v.x, v.y, v.z, w);
-}
-// Row-level products stay in FP32; sums from 32 rows upward are FP64 (GB300's
-// FP64 pipe is narrow, so FP64 work is kept per warp, not per row).
-__device__ __forceinline__ float fdot(float3 a, float3 b)
-{
-    return fmaf(a.z, b.z, fmaf(a.y, b.y, a.x * b.x));
-}
-__device__ __forceinline__ float warp_sum(float v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-        v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-// sum of squares in component order, as tCudaMatrix::norm (CudaMatrix.h:314-320)
-__device__ __forceinline__ float norm3(float3 a)
-{
-    float s = a.x * a.x;
-    s = s + a.y * a.y;
-    s = s + a.z * a.z;
-    return sqrtf(s);
-}
-// symmetric 3x3 (00 01 02 11 12 22) times vector
-// (explicit fused multiply-adds: device code is built without implicit
-// contraction, so every kernel variant rounds the same way)
-__device__ __forceinline__ float3 symv(const float *s, float3 v)
-{
-    return make_float3(fmaf(s[2], v.z, fmaf(s[1], v.y, s[0] * v.x)),
-                       fmaf(s[4], v.z, fmaf(s[3], v.y, s[1] * v.x)),
-                       fmaf(s[5], v.z, fmaf(s[4], v.y, s[2] * v.x)));
-}
-// p = z + beta p_old with one rounding per component (the persistent
-// kernels' form, so every PCG driver forms the same p)
-__device__ __forceinline__ float3 pform(float3 z, float beta, float3 po)
-{
-    return make_float3(fmaf(beta, po.x, z.x), fmaf(beta, po.y, z.y), fmaf(beta, po.z, z.z));
-}
-// w x p: the skew part of a block of the dihedral-bending model (an upper
-// block is S p + w x p, its transposed lower block S p - w x p)
-__device__ __forceinline__ float3 skewv(float4 w, float3 p)
-{
-    return make_float3(fmaf(w.y, p.z, -(w.z * p.y)), fmaf(w.z, p.x, -(w.x * p.z)),
-                       fmaf(w.x, p.y, -(w.y * p.x)));
-}
-__device__ __forceinline__ void load_sym(const float4 *a0, const float2 *a1,
-                                         size_t o, float *s)
-{
-    float4 u = a0[o];
-    float2 w = a1[o];
-    s[0] = u.x;
-    s[1] = u.y;
-    s[2] = u.z;
-    s[3] = u.w;
-    s[4] = w.x;
-    s[5] = w.y;
-}
 
 // Symmetric 3x3 inverse by the adjugate, as tCudaMatrix::inverse
 // (CudaMatrix.h:362-398) evaluates it for a symmetric block.
@@ -242,17 +170,6 @@ __device__ bool tile_reduce(const InstDesc &d, int tile_idx, const float (&vf)[N
     return true;
 }
 
-__device__ __forceinline__ bool test_converged(const InstDesc &d,
-                                               const InstState &s, double rr)
-{
-    bool ok = false;
-    if (d.rel_tol2 > 0.0 && rr <= d.rel_tol2 * s.bb)
-        ok = true;
-    if (d.abs_tol2 > 0.0 && rr <= d.abs_tol2)
-        ok = true;
-    return ok;
-}
-
 // PCG start bookkeeping of one instance (thread 0 of its last tile): FP64
 // scalars from the start sums tot = (r.z, r.r, b.b), counters, the team
 // barrier and team-sum buffers of the persistent solver, the active flag.
@@ -294,69 +211,6 @@ __device__ __forceinline__ void begin_solve(const InstDesc &d, const double (&to
         st.active = 1;
         atomicAdd(&ctl->n_active, 1);
     }
-}
-
-// round(v * 2^s) as a signed 128-bit integer, returned as H * 2^32 + L with
-// 0 <= L < 2^32 (integer operations only).  Exact addition of these limbs
-// makes a team sum independent of how the rows are split over blocks.
-__device__ __forceinline__ void fx_split(float v, int s, long long &H,
-                                         unsigned long long &L)
-{
-    const unsigned bits = __float_as_uint(v);
-    const int e = int((bits >> 23) & 0xffu);
-    H = 0;
-    L = 0;
-    if (e == 0 || e == 255)
-        return; // zero, subnormal (below any scale in use) or Inf/NaN (check sum)
-    const unsigned long long m = (bits & 0x7fffffu) | 0x800000u;
-    const int sh = e - 150 + s; // |v| = m * 2^(e - 150)
-    unsigned long long fh = 0ull, fl = 0ull;
-    if (sh >= 104)
-    {
-        fh = 0x3fffffffffffffffull; // saturate; the check sum flags it
-        fl = ~0ull;
-    }
-    else if (sh >= 64)
-        fh = m << (sh - 64);
-    else if (sh > 0)
-    {
-        fl = m << sh;
-        fh = m >> (64 - sh);
-    }
-    else if (sh == 0)
-        fl = m;
-    else if (sh > -25)
-        fl = (m + (1ull << (-sh - 1))) >> (-sh);
-    if (bits & 0x80000000u)
-    {
-        fl = ~fl + 1ull;
-        fh = ~fh + (fl == 0ull ? 1ull : 0ull);
-    }
-    L = fl & 0xffffffffull;
-    H = (long long)((fh << 32) | (fl >> 32));
-}
-
-// Scale exponent for an estimate of a sum (from the double's exponent bits).
-__device__ __forceinline__ int fx_scale(double est)
-{
-    const long long b = __double_as_longlong(est);
-    const int e = int((b >> 52) & 0x7ff);
-    if (e == 0 || e == 0x7ff)
-        return 100;
-    const int s = kFxTop - (e - 1023);
-    return max(-900, min(900, s));
-}
-
-// 2^e for |e| < 1000, built from the exponent field
-__device__ __forceinline__ double pow2(int e)
-{
-    return __longlong_as_double((long long)(1023 + e) << 52);
-}
-
-__device__ __forceinline__ double fx_value(unsigned long long H, unsigned long long L,
-                                           int s)
-{
-    return double((long long)H) * pow2(32 - s) + double(L) * pow2(-s);
 }
 
 // An instance leaves the loop: the thread that brings the active count down
