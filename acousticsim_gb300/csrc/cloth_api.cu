@@ -129,7 +129,8 @@ struct Batch
     bool persist_sm = false; // own-row state in shared memory
     bool persist_1b = false; // single-barrier variant (shared memory, every halo staged)
     bool persist_team = false; // k_pcg_team: the matrix on chip
-    int team_chunks = 1;       // its chunks per warp
+    int team_rows = 1;         // its rows per thread
+    int team_cluster = 0;      // its teams are clusters of this many blocks (0: not clusters)
     TeamBlock *d_work = nullptr;
     char *d_sync = nullptr;    // behind the work list: arrival counts or team sums
     size_t sync_bytes = 0;
@@ -823,7 +824,7 @@ int make_batch(cloth_ctx *ctx, const std::vector<cloth_s *> &members,
 const void *persistent_kernel(const Batch *b)
 {
     if (b->persist_team)
-        return team_kernel(b->team_chunks, b->skew);
+        return team_kernel(b->team_rows, b->skew, b->team_cluster > 0);
     if (b->persist_1b)
         return (const void *)k_pcg1_persistent;
     if (b->skew)
@@ -843,6 +844,26 @@ struct PersistArgs
     }
     void **of(const Batch *b) { return b->persist_team ? team : two; }
 };
+
+// How a persistent launch keeps its teams together: all blocks resident, or
+// every team a cluster.
+cudaLaunchAttribute persist_attribute(const Batch *b)
+{
+    cudaLaunchAttribute at;
+    std::memset(&at, 0, sizeof(at));
+    if (b->persist_team && b->team_cluster > 0)
+    {
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = unsigned(b->team_cluster);
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    }
+    else
+    {
+        at.id = cudaLaunchAttributeCooperative;
+        at.val.cooperative = 1;
+    }
+    return at;
+}
 
 // The work list of a persistent launch, and behind it per_block bytes for
 // every block, zeroed before each launch.
@@ -874,76 +895,115 @@ TeamBlock team_block(const Tables &t, int inst, int rank, int r0, int r1)
     return w;
 }
 
-// Plan of k_pcg_team: every block's rows, their blocks and p over their
-// columns in its shared memory.  False when the set does not fit that way.
-bool plan_team(cloth_ctx *ctx, const Batch *b, std::vector<TeamBlock> &work, size_t &smem,
-               int &chunks)
+// Adds instance i of b to a k_pcg_team work list in at most `blocks` blocks (K
+// rows a thread, rows in 32-aligned chunks); false when one does not fit its SM.
+bool team_split(const Batch *b, int i, int blocks, int K, bool cluster, size_t cap,
+                std::vector<TeamBlock> &work, size_t &smem)
+{
+    const cloth_s *c = b->members[i];
+    const Tables &t = c->tab;
+    const size_t first = work.size();
+    const int rows =
+        ((t.nv + blocks - 1) / blocks + kRedRows - 1) / kRedRows * kRedRows;
+    if (rows > K * kTeamWorkers)
+        return false;
+    size_t most = 0;
+    for (int r0 = 0; r0 < t.nv; r0 += rows)
+    {
+        work.push_back(team_block(t, i, int(work.size() - first), r0, std::min(t.nv, r0 + rows)));
+        const TeamBlock &w = work.back();
+        most = std::max(most, team_smem_bytes(w.halo1 - w.halo0, w.row1 - w.row0, c->h.width,
+                                              c->h.Aw != nullptr, team_reg_slots(K, b->skew),
+                                              cluster));
+        if (most > cap || w.halo1 - w.halo0 > 65535)
+        {
+            work.resize(first);
+            return false;
+        }
+    }
+    for (size_t k = first; k < work.size(); k++)
+        work[k].nblk = int(work.size() - first);
+    smem = std::max(smem, most);
+    return true;
+}
+
+// Plan of k_pcg_team whose teams are clusters of C blocks (at_once: all of them
+// resident together).
+bool plan_cluster(cloth_ctx *ctx, const Batch *b, int K, int C, std::vector<TeamBlock> &work,
+                  size_t &smem, bool at_once)
+{
+    const size_t cap = size_t(ctx->max_smem_optin) - 6144;
+    const int n = int(b->members.size());
+    smem = 0;
+    work.clear();
+    // the largest first: clusters start in this order as SMs come free
+    std::vector<int> order(n);
+    for (int i = 0; i < n; i++)
+        order[i] = i;
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
+        return b->members[x]->tab.nv > b->members[y]->tab.nv;
+    });
+    for (int i : order)
+    {
+        if (!team_split(b, i, C, K, true, cap, work, smem))
+            return false;
+        while (work.size() % size_t(C))
+            work.push_back(TeamBlock{-1, 0, 0, 0, 0, 0, 0, 0});
+    }
+    const void *f = team_kernel(K, b->skew, true);
+    cudaLaunchConfig_t cfg;
+    std::memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3(unsigned(work.size()));
+    cfg.blockDim = dim3(kTeamThreads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = unsigned(C);
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int active = 0;
+    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, int(cap)) !=
+            cudaSuccess ||
+        cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
+            cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&active, f, &cfg) != cudaSuccess ||
+        active < (at_once ? n : 1))
+    {
+        cudaGetLastError();
+        return false;
+    }
+    return true;
+}
+
+// Plan of k_pcg_team with K rows per thread and teams of any number of blocks,
+// all resident at once: every block's rows, their blocks and p over their
+// columns on its SM.  False when the set does not fit.
+bool plan_team(cloth_ctx *ctx, const Batch *b, int K, std::vector<TeamBlock> &work, size_t &smem)
 {
     const int G = std::min(ctx->num_sms, kTeamMaxBlocks);
     const int n = int(b->members.size());
     if (n > G)
         return false;
     const size_t cap = size_t(ctx->max_smem_optin) - 4096;
-    // the split of instance i into blocks of `rows` rows: its blocks, or none
-    // when one does not fit
-    auto split = [&](int i, int rows, std::vector<TeamBlock> &out, size_t &bytes) {
-        const cloth_s *c = b->members[i];
-        const Tables &t = c->tab;
-        out.clear();
-        bytes = 0;
-        for (int r0 = 0; r0 < t.nv; r0 += rows)
-        {
-            out.push_back(team_block(t, i, int(out.size()), r0, std::min(t.nv, r0 + rows)));
-            const TeamBlock &w = out.back();
-            bytes = std::max(bytes, team_smem_bytes(w.halo1 - w.halo0, w.row1 - w.row0,
-                                                    c->h.width, c->h.Aw != nullptr));
-            if (bytes > cap || w.halo1 - w.halo0 > 65535)
-                return false;
-        }
-        for (auto &w : out)
-            w.nblk = int(out.size());
-        return int(out.size()) <= G;
-    };
-    auto rows_of = [](int nv, int blocks) {
-        return ((nv + blocks - 1) / blocks + kRedRows - 1) / kRedRows * kRedRows;
-    };
     long long total = 0;
     for (auto *c : b->members)
         total += c->tab.nv;
-    std::vector<std::vector<TeamBlock>> teams(n);
-    std::vector<size_t> bytes(n);
-    int used = 0;
-    for (int i = 0; i < n; i++)
-    {
-        const int nv = b->members[i]->tab.nv;
-        long long share = std::max(1ll, (long long)(G - (n - 1)) * nv / std::max(1ll, total));
-        if (nv <= kTeamSingleRows && split(i, rows_of(nv, 1), teams[i], bytes[i]))
-        {
-            used++;
-            continue;
-        }
-        const int want = std::max(1, std::min<int>(int(share), (nv + kTeamMinRows - 1) / kTeamMinRows));
-        const int rows = rows_of(nv, want);
-        if (rows > 2 * kTeamWorkers || !split(i, rows, teams[i], bytes[i]))
-            return false;
-        used += int(teams[i].size());
-    }
-    if (used > G)
-        return false;
     smem = 0;
-    int most = 0;
     work.clear();
     for (int i = 0; i < n; i++)
     {
-        smem = std::max(smem, bytes[i]);
-        for (const auto &w : teams[i])
-        {
-            most = std::max(most, w.row1 - w.row0);
-            work.push_back(w);
-        }
+        const int nv = b->members[i]->tab.nv;
+        const long long share =
+            std::max(1ll, (long long)(G - (n - 1)) * nv / std::max(1ll, total));
+        const int want =
+            std::max(1, std::min<int>(int(share), (nv + kTeamMinRows - 1) / kTeamMinRows));
+        if (!team_split(b, i, want, K, false, cap, work, smem))
+            return false;
     }
-    chunks = most > kTeamWorkers ? 2 : 1;
-    const void *f = team_kernel(chunks, b->skew);
+    if (int(work.size()) > G)
+        return false;
+    const void *f = team_kernel(K, b->skew, false);
     int occ = 0;
     if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, int(cap)) !=
             cudaSuccess ||
@@ -968,12 +1028,32 @@ int plan_persistent(cloth_ctx *ctx, Batch *b)
         ctx->solver != CLOTH_SOLVER_PERSISTENT_2B)
         return CLOTH_OK;
     std::vector<TeamBlock> work;
-    if (ctx->solver != CLOTH_SOLVER_PERSISTENT_1B &&
-        plan_team(ctx, b, work, b->smem_persist, b->team_chunks))
+    if (ctx->solver != CLOTH_SOLVER_PERSISTENT_1B)
     {
         b->persist_team = true;
         b->block_persist = kTeamThreads;
-        return upload_work(b, work, sizeof(TeamSync), alignof(TeamSync) * 64);
+        int most = 0;
+        for (auto *c : b->members)
+            most = std::max(most, c->tab.nv);
+        // Clusters where the set's cloths fit them and all run at once.  Up to
+        // 320 rows a block alone is fastest (16^2: 2.3 us per iteration, 2.8
+        // in a cluster of 16; 20^2: 2.7 alone, 2.7 in 8), above it 16 blocks
+        // (32^2: 2.6 us, 2.9 as two blocks), while one row a thread is enough
+        // (64^2: 2.9 us, 3.3 over the whole GPU; 90^2, two rows: 4.8 and 3.4)
+        const int C = most <= kTeamAloneRows ? 1 : kClusterMax;
+        if (plan_cluster(ctx, b, 1, C, work, b->smem_persist, true))
+        {
+            b->team_rows = 1;
+            b->team_cluster = C;
+            return upload_work(b, work, sizeof(unsigned long long), sizeof(TeamBlock));
+        }
+        for (int K = 1; K <= 2; K++)
+            if (plan_team(ctx, b, K, work, b->smem_persist))
+            {
+                b->team_rows = K;
+                return upload_work(b, work, sizeof(TeamSync), alignof(TeamSync) * 64);
+            }
+        b->persist_team = false;
     }
     work.clear();
     const size_t smem_cap_bytes =
@@ -1234,12 +1314,9 @@ int build_graph(Batch *b, bool full, cudaGraphExec_t *exec)
                 rc = fail(CLOTH_ERR_CUDA, "cudaGraphAddKernelNode(persistent) failed");
             else
             {
-                cudaLaunchAttributeValue v;
-                std::memset(&v, 0, sizeof(v));
-                v.cooperative = 1;
-                if (cudaGraphKernelNodeSetAttribute(n, cudaLaunchAttributeCooperative, &v) !=
-                    cudaSuccess)
-                    rc = fail(CLOTH_ERR_CUDA, "cooperative attribute on graph node failed");
+                const cudaLaunchAttribute at = persist_attribute(b);
+                if (cudaGraphKernelNodeSetAttribute(n, at.id, &at.val) != cudaSuccess)
+                    rc = fail(CLOTH_ERR_CUDA, "launch attribute on graph node failed");
                 last = n;
             }
         }
@@ -1332,9 +1409,16 @@ int launch_persistent(Batch *b)
     b->spin = ctx->spin;
     PersistArgs args(b);
     CK(cudaMemsetAsync(b->d_sync, 0, b->sync_bytes, ctx->stream));
-    CK(cudaLaunchCooperativeKernel(persistent_kernel(b), dim3(b->grid_persist),
-                                   dim3(b->block_persist), args.of(b), b->smem_persist,
-                                   ctx->stream));
+    cudaLaunchAttribute at = persist_attribute(b);
+    cudaLaunchConfig_t cfg;
+    std::memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3(b->grid_persist);
+    cfg.blockDim = dim3(b->block_persist);
+    cfg.dynamicSmemBytes = b->smem_persist;
+    cfg.stream = ctx->stream;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    CK(cudaLaunchKernelExC(&cfg, persistent_kernel(b), args.of(b)));
     return CLOTH_OK;
 }
 

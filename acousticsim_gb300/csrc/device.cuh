@@ -247,25 +247,43 @@ struct SpinCfg
     unsigned extra;
 };
 
-// k_pcg_team: worker threads (one row each, or two) and the control warp; a
-// team's sum words, four iterations deep (p.q in words 0-2, r.z and r.r in
-// words 4-9), zeroed before every launch.
-constexpr int kTeamWorkers = 512;
+// k_pcg_team: worker threads (one row each, or two) and the control warp - 16
+// warps, four on each quarter of an SM, so a thread may have 128 registers; a
+// team's sum words, four iterations deep (p.q in words 0-3, r.z in 4-7, r.r in
+// 8-11), zeroed before every launch.
+constexpr int kTeamWorkers = 480;
 constexpr int kTeamThreads = kTeamWorkers + 32;
-constexpr int kTeamSingleRows = 640; // instances up to this size: a team of one block
-constexpr int kTeamMinRows = 64;     // rows a block of a larger team gets at least
+constexpr int kTeamAloneRows = 320; // instances up to this size: a team of one block
+constexpr int kTeamMinRows = 64;    // rows a block of a larger team gets at least
 constexpr int kTeamMaxBlocks = 255; // a word counts its team's arrivals in one byte
 struct TeamSync
 {
     unsigned long long words[4][16];
 };
-// Dynamic shared memory of a k_pcg_team block: p over its halo, and width
-// planes of blocks (skew parts), and local column indices over its rows.
-__host__ __device__ inline size_t team_smem_bytes(int halo, int rows, int width, bool skew)
+// Slots of a row whose blocks k_pcg_team holds in registers (K rows a thread).
+__host__ __device__ constexpr int team_reg_slots(int k, bool skew_kernel)
+{
+    return k > 1 ? 0 : skew_kernel ? 4 : 8;
+}
+// Dynamic shared memory of a k_pcg_team block: p over its halo; blocks (skew
+// parts) and local column indices of the rows' other slots; in a cluster, z
+// over the halo rows of other blocks.
+__host__ __device__ inline size_t team_smem_bytes(int halo, int rows, int width, bool skew,
+                                                  int reg_slots, bool cluster)
 {
     const size_t rp = size_t((rows + 31) / 32) * 32;
-    return size_t(halo) * 16 + size_t(width) * rp * (skew ? 42 : 26);
+    const size_t planes = width > reg_slots ? width - reg_slots : 0;
+    return (size_t(halo) + (cluster ? halo - rows : 0)) * 16 + planes * rp * (skew ? 42 : 26);
 }
+// A team that is one thread-block cluster: its most blocks, and a block whose
+// halo holds rows [row0, row1) of this one (row i of z goes to z + 16 i in the
+// cluster's shared memory, counted on its barrier bar).
+constexpr int kClusterMax = 16;
+struct TeamPeer
+{
+    int row0, row1;
+    unsigned z, bar;
+};
 
 // One variant of a graph-loop kernel: R rows per thread (blocks of kTile / R
 // threads), U ELL slots whose loads are issued together (SpMV only), TPB

@@ -24,8 +24,8 @@
 //
 // Measured (one GB300, us per PCG iteration over a whole step, before: the
 // kernel that reads the matrix from L2 and forms the scalars in FP64): 20x20
-// 11.8 -> 4.6, 97x61 11.8 -> 4.5, 193x255 12.4 -> 4.9, 128x128 with dihedral
-// bending 14.1 -> 5.1.
+// 11.8 -> 3.8, 64x64 12.2 -> 3.2, 97x61 11.8 -> 3.7, 193x255 12.4 -> 4.4,
+// 128x128 with dihedral bending 14.1 -> 4.9.
 #include "internal.h"
 #include "pcg_math.cuh"
 
@@ -85,136 +85,211 @@ __device__ __forceinline__ float3 poll_row(const float4 *p, unsigned tag, unsign
                        __uint_as_float(unsigned(hi)));
 }
 
-// ---- team sums.  A sum is the exact total of fixed-point chunk sums, 96 bits
-// and a sign, in units of 2^-s (fx_split).  Three words carry it: bits 0-31,
-// 32-63 and the rest (biased), each with the number of blocks that added to
-// it in its top byte, and the number of blocks that saw a chunk out of range
-// (or Inf / NaN) in bits 40-55 of the second.
-typedef __int128 i128;
-constexpr int kCountShift = 56;
-constexpr unsigned long long kOne = 1ull << kCountShift;
-constexpr unsigned long long kBias = 1ull << 44;
-constexpr unsigned long long kBad = 1ull << 40;
-
-__device__ __forceinline__ i128 shl(long long v, int n)
+// ---- a team that is one thread-block cluster exchanges through its blocks'
+// shared memory: 16-byte remote stores that count on the receiver's mbarrier
+__device__ __forceinline__ unsigned smem_u32(const void *p)
 {
-    return i128((unsigned __int128)(i128(v)) << n);
+    return unsigned(__cvta_generic_to_shared(p));
 }
-
-struct Total
+__device__ __forceinline__ unsigned peer_addr(unsigned addr, unsigned rank)
 {
-    long long H;          // bits 32.. (wraps where the sum is out of range)
-    unsigned long long L; // bits 0-31
-    int s;
-    bool bad;
-};
-
-__device__ __forceinline__ double total_value(const Total &t) { return fx_value(t.H, t.L, t.s); }
-
-// The block's chunk sums c[0 .. n) at scale s: 24-bit digits per lane, added
-// over the warp by the integer reduce instructions.
-__device__ __forceinline__ i128 fold(const float *c, int n, int s, bool &bad)
+    unsigned a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ void cluster_sync()
 {
-    unsigned d0 = 0, d1 = 0, d2 = 0, b = 0;
-    int d3 = 0;
-    for (int ch = threadIdx.x & 31; ch < n; ch += 32)
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ void peer_store(unsigned addr, unsigned bar, int a, int b, int c, int d)
+{
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], "
+                 "{%1, %2, %3, %4}, [%5];" ::"r"(addr),
+                 "r"(a), "r"(b), "r"(c), "r"(d), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void mbar_expect(unsigned bar, unsigned bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
+                 : "memory");
+}
+// Waits for a phase; false when the bounded wait gave up.
+__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, unsigned limit)
+{
+    for (unsigned n = 0;;)
     {
-        const float v = c[ch];
-        long long h;
-        unsigned long long l;
-        fx_split(v, s, h, l);
-        const int e = int((__float_as_uint(v) >> 23) & 0xffu);
-        if (e == 255 || e - 127 + s >= 95)
-            b = 1u;
-        d0 += unsigned(l) & 0xffffffu;
-        d1 += (unsigned(l) >> 24) | (unsigned(h) & 0xffffu) << 8;
-        d2 += unsigned(h >> 16) & 0xffffffu;
-        d3 += int(h >> 40);
-    }
-    d0 = __reduce_add_sync(kFull, d0);
-    d1 = __reduce_add_sync(kFull, d1);
-    d2 = __reduce_add_sync(kFull, d2);
-    d3 = __reduce_add_sync(kFull, d3);
-    bad = __any_sync(kFull, b) != 0;
-    return i128(d0) + (i128(d1) << 24) + (i128(d2) << 48) + shl(d3, 72);
-}
-
-__device__ __forceinline__ Total make_total(i128 v, int s, bool bad)
-{
-    Total t;
-    t.H = (long long)(v >> 32);
-    t.L = (unsigned long long)v & 0xffffffffull;
-    t.s = s;
-    t.bad = bad || (v >> 95) != ((v >> 95) ? i128(-1) : i128(0));
-    return t;
-}
-
-// Word k (0-2) of a block's contribution.
-__device__ __forceinline__ unsigned long long sum_word(i128 v, bool bad, int k)
-{
-    if (k == 0)
-        return kOne + ((unsigned long long)v & 0xffffffffull);
-    if (k == 1)
-        return kOne + ((unsigned long long)(v >> 32) & 0xffffffffull) + (bad ? kBad : 0ull);
-    return kOne + kBias + (unsigned long long)(long long)(v >> 64);
-}
-
-// Team total of NQ quantities: lanes 0 .. 3 NQ - 1 add one word each and poll
-// it until every block's arrival is in.  Returns false when the wait gave up.
-template <int NQ>
-__device__ __forceinline__ bool team_total(unsigned long long *words, const i128 (&v)[NQ],
-                                           const bool (&bad)[NQ], const int (&s)[NQ], int nblk,
-                                           const SpinCfg &sc, Total (&out)[NQ])
-{
-    const int lane = threadIdx.x & 31;
-    unsigned long long w = 0ull;
-    if (lane < 3 * NQ)
-    {
-        const int q = NQ == 1 ? 0 : lane / 3, k = lane - 3 * q;
-        i128 vq = v[0];
-        bool bq = bad[0];
-        if (NQ > 1 && q)
-        {
-            vq = v[NQ - 1];
-            bq = bad[NQ - 1];
-        }
-        w = sum_word(vq, bq, k);
-        asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(words + lane), "l"(w)
+        unsigned done;
+        asm volatile("{ .reg .pred p; mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, "
+                     "[%1], %2; "
+                     "selp.u32 %0, 1, 0, p; }"
+                     : "=r"(done)
+                     : "r"(bar), "r"(parity)
                      : "memory");
-    }
-    const unsigned long long target = (unsigned long long)nblk + sc.extra;
-    unsigned n = 0;
-    for (;;)
-    {
-        bool here = true;
-        if (lane < 3 * NQ)
-        {
-            asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];"
-                         : "=l"(w)
-                         : "l"(words + lane)
-                         : "memory");
-            here = (w >> kCountShift) >= target;
-        }
-        if (__all_sync(kFull, here))
-            break;
-        if (++n > sc.limit)
+        if (done)
+            return true;
+        if (++n > limit)
             return false;
-        if (n > 256)
+        if (n > 4096)
             __nanosleep(32);
     }
-    w &= kOne - 1;
-#pragma unroll
-    for (int q = 0; q < NQ; q++)
-    {
-        const unsigned long long w0 = __shfl_sync(kFull, w, 3 * q),
-                                 w1 = __shfl_sync(kFull, w, 3 * q + 1),
-                                 w2 = __shfl_sync(kFull, w, 3 * q + 2);
-        const long long hi = (long long)(w2 - (unsigned long long)nblk * kBias);
-        const i128 t = i128(w0) + (i128(w1 & (kBad - 1)) << 32) + shl(hi, 64);
-        out[q] = make_total(t, s[q], (w1 >> 40) != 0);
-    }
-    return true;
 }
+
+// ---- team sums.  A sum is the exact total V of fixed-point chunk sums, in
+// units of 2^-s, kept as signed 24-bit digits d0 .. d3 (each chunk adds to two
+// of them).  Four words carry it, one per digit: the digit's sum, biased per
+// block, with the number of blocks that added to the word in its top byte;
+// bits 44-55 of the first count the blocks that saw a chunk out of range (or
+// Inf / NaN).
+constexpr int kCountShift = 56, kBadShift = 44;
+constexpr unsigned long long kOne = 1ull << kCountShift;
+constexpr unsigned long long kBias = 1ull << 32;
+constexpr unsigned long long kSumMask = (1ull << kBadShift) - 1;
+
+// V = hi 2^48 + lo, 0 <= lo < 2^48.
+struct Raw
+{
+    long long hi;
+    unsigned long long lo;
+    int s;
+};
+__device__ __forceinline__ Raw raw(double d)
+{
+    Raw r;
+    const unsigned long long b = (unsigned long long)__double_as_longlong(d);
+    const int e = int((b >> 52) & 0x7ff);
+    long long m = e ? (long long)((b & 0xfffffffffffffull) | 0x10000000000000ull) : 0ll;
+    if (b >> 63)
+        m = -m;
+    r.hi = m >> 48;
+    r.lo = (unsigned long long)m & 0xffffffffffffull;
+    r.s = e ? 1075 - e : 0;
+    return r;
+}
+// The FP64 value the drivers that sum 64-bit limbs decode.
+__device__ __forceinline__ double value(const Raw &r)
+{
+    return fx_value((unsigned long long)r.hi << 16 | r.lo >> 32, r.lo & 0xffffffffull, r.s);
+}
+
+// Adds 32-row chunks' FP32 sums to the block's digits: lanes 8 q .. 8 q + 4 add
+// quantity q's (v and its scale s are theirs), dig[8 q .. 8 q + 3] being its
+// digits and dig[8 q + 4] the count of sums out of range.  NQ quantities.
+template <int NQ> __device__ __forceinline__ void chunk_add(int *dig, float v, int s)
+{
+    const unsigned bits = __float_as_uint(v);
+    const int e = int((bits >> 23) & 0xffu), lane = threadIdx.x & 31, j = lane & 7;
+    unsigned m = e ? (bits & 0x7fffffu) | 0x800000u : 0u; // (subnormal: below any scale in use)
+    int sh = e - 150 + s;                                 // |v| = m 2^sh units
+    const bool bad = e == 255 || (e != 0 && sh >= 72);
+    if (sh < 0)
+    {
+        m = sh > -25 ? (m + (1u << (-sh - 1))) >> -sh : 0u;
+        sh = 0;
+    }
+    const int k = (sh * 43) >> 10, off = sh - 24 * k; // sh / 24, sh % 24
+    int x = j == k ? int((m << off) & 0xffffffu) : j == k + 1 ? int(m >> (24 - off)) : 0;
+    if (bits & 0x80000000u)
+        x = -x;
+    if (bad)
+        x = j == 4 ? 1 : 0;
+    else if (j > 3)
+        x = 0;
+    if (x != 0 && lane < 8 * NQ)
+        atomicAdd(dig + lane, x);
+}
+
+// V from its digits; true when it is out of the 96-bit range.
+__device__ __forceinline__ bool combine(long long d0, long long d1, long long d2, long long d3,
+                                        int s, Raw &r)
+{
+    const long long lo = d0 + d1 * (1ll << 24);
+    r.hi = d2 + d3 * (1ll << 24) + (lo >> 48);
+    r.lo = (unsigned long long)lo & 0xffffffffffffull;
+    r.s = s;
+    return r.hi >= (1ll << 47) || r.hi < -(1ll << 47);
+}
+
+// A block's digits dig[0 .. 4], read and cleared by the control warp.
+struct Digits
+{
+    int4 d;
+    int bad;
+};
+__device__ __forceinline__ Digits take(int *dig)
+{
+    const volatile int *v = dig;
+    Digits r{make_int4(v[0], v[1], v[2], v[3]), v[4]};
+    __syncwarp();
+    if ((threadIdx.x & 31) < 5)
+        dig[threadIdx.x & 31] = 0;
+    return r;
+}
+__device__ __forceinline__ bool decode(const Digits &v, int s, Raw &r)
+{
+    return combine(v.d.x, v.d.y, v.d.z, v.d.w, s, r) || v.bad != 0;
+}
+
+// The same digits carried into [0, 2^24) (the last one signed), bit 31 of the
+// first marking a sum out of range: a cluster's 16 add up in 32 bits.
+__device__ __forceinline__ int4 carried(const Digits &v)
+{
+    int4 c = v.d;
+    c.y += c.x >> 24;
+    c.x = (c.x & 0xffffff) | (v.bad ? int(0x80000000u) : 0);
+    c.z += c.y >> 24;
+    c.y &= 0xffffff;
+    c.w += c.z >> 24;
+    c.z &= 0xffffff;
+    return c;
+}
+// Total of a cluster's nblk records.
+__device__ __forceinline__ bool decode(const int4 *rec, int nblk, int s, Raw &r)
+{
+    int4 c = make_int4(0, 0, 0, 0);
+    if ((threadIdx.x & 31) < nblk)
+        c = rec[threadIdx.x & 31];
+    const bool bad = __any_sync(kFull, c.x < 0) != 0;
+    const int d0 = __reduce_add_sync(kFull, c.x & 0xffffff), d1 = __reduce_add_sync(kFull, c.y),
+              d2 = __reduce_add_sync(kFull, c.z), d3 = __reduce_add_sync(kFull, c.w);
+    return combine(d0, d1, d2, d3, s, r) || bad;
+}
+
+// Word k of a block's sum: added to the team's by lane k.
+__device__ __forceinline__ void word_add(unsigned long long *words, const Digits &v, int k)
+{
+    const int d = k == 0 ? v.d.x : k == 1 ? v.d.y : k == 2 ? v.d.z : v.d.w;
+    const unsigned long long w = kOne + kBias + (unsigned long long)(long long)d +
+                                 (k == 0 && v.bad ? 1ull << kBadShift : 0ull);
+    asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(words + k), "l"(w)
+                 : "memory");
+}
+// A team's sum words, the same in every lane (one 32-byte request a poll: the
+// team's polls and reductions queue at one L2 slice).
+struct Words
+{
+    unsigned long long w[4];
+    __device__ __forceinline__ void load(const unsigned long long *p)
+    {
+        asm volatile("ld.relaxed.gpu.global.v4.u64 {%0, %1, %2, %3}, [%4];"
+                     : "=l"(w[0]), "=l"(w[1]), "=l"(w[2]), "=l"(w[3])
+                     : "l"(p)
+                     : "memory");
+    }
+    // every block's contribution is in
+    __device__ __forceinline__ bool all_in(unsigned long long target) const
+    {
+        return min(min(w[0] >> kCountShift, w[1] >> kCountShift),
+                   min(w[2] >> kCountShift, w[3] >> kCountShift)) >= target;
+    }
+    __device__ __forceinline__ bool decode(int nblk, int s, Raw &r) const
+    {
+        const unsigned long long b = (unsigned long long)nblk * kBias;
+        return combine((long long)((w[0] & kSumMask) - b), (long long)((w[1] & kSumMask) - b),
+                       (long long)((w[2] & kSumMask) - b), (long long)((w[3] & kSumMask) - b), s,
+                       r) ||
+               ((w[0] >> kBadShift) & 0xfffu) != 0;
+    }
+};
 
 // ---- scalars without the FP64 pipe.  |value| = (hi + lo 2^-24) 2^e with hi
 // in [2^23, 2^24): its top 48 bits, the rest dropped (relative error 2^-47).
@@ -224,33 +299,28 @@ struct Top48
     int e;
     bool neg;
 };
-__device__ __forceinline__ Top48 top48(const Total &t)
+__device__ __forceinline__ Top48 top48(const Raw &v)
 {
     Top48 r;
-    i128 v = shl(t.H, 32) + i128(t.L);
-    r.neg = v < 0;
+    unsigned long long hi = (unsigned long long)v.hi, lo = v.lo;
+    r.neg = v.hi < 0;
     if (r.neg)
-        v = -v;
-    const unsigned long long vh = (unsigned long long)(v >> 64), vl = (unsigned long long)v;
-    const int nb = vh ? 128 - __clzll((long long)vh) : 64 - __clzll((long long)vl);
-    const int sh = nb - 48;
-    const unsigned long long m =
-        sh > 0 ? (unsigned long long)((unsigned __int128)v >> sh) : vl << -sh;
-    r.hi = unsigned(m >> 24);
-    r.lo = unsigned(m) & 0xffffffu;
-    r.e = nb - 24 - t.s;
-    return r;
-}
-__device__ __forceinline__ Top48 top48(double d)
-{
-    Top48 r;
-    const unsigned long long b = (unsigned long long)__double_as_longlong(d);
-    const unsigned long long m = ((b & 0xfffffffffffffull) | 0x10000000000000ull) >> 5;
-    const int e = int((b >> 52) & 0x7ff);
-    r.neg = (b >> 63) != 0;
-    r.hi = e ? unsigned(m >> 24) : 0u;
-    r.lo = unsigned(m) & 0xffffffu;
-    r.e = e - 1023 - 23;
+    {
+        lo = (0ull - lo) & 0xffffffffffffull;
+        hi = 0ull - hi - (lo != 0ull ? 1ull : 0ull);
+    }
+    int base = 48;
+    if (hi == 0ull)
+    {
+        hi = lo;
+        lo = 0ull;
+        base = 0;
+    }
+    const int nb = 64 - __clzll((long long)hi); // bits of hi
+    const unsigned long long t = nb <= 48 ? hi << (48 - nb) | lo >> nb : hi >> (nb - 48);
+    r.hi = unsigned(t >> 24);
+    r.lo = unsigned(t) & 0xffffffu;
+    r.e = base + nb - 24 - v.s;
     return r;
 }
 // An order of the magnitudes that a relative difference above 2^-22 decides.
@@ -258,18 +328,28 @@ __device__ __forceinline__ long long key(const Top48 &t)
 {
     return ((long long)t.e << 24) + (long long)(t.hi - 0x800000u);
 }
+// fx_scale of the FP64 value: from its exponent, unless the rounding to FP64
+// could have carried into it (or the sum left the range where it rounds once).
+__device__ __forceinline__ int scale_of(const Raw &v, const Top48 &t)
+{
+    if (t.hi == 0u || (t.hi == 0xffffffu && t.lo == 0xffffffu) || v.hi >= (1ll << 37) ||
+        v.hi <= -(1ll << 37))
+        return fx_scale(value(v));
+    return max(-900, min(900, kFxTop - (t.e + 23)));
+}
 
 // float(a / b), the quotient of the FP64 values rounded to FP64 and then to
 // FP32, as the drivers that divide in FP64 form it.  The quotient is formed
 // as q1 + q2 (FP32 quotient, then its remainder over b): within 2^-43 of the
 // exact one.  Where that leaves the rounding to FP32 open (the sum lies
 // within 2^-38 of a midpoint: one time in ~10,000), or the result is not in
-// the normal range, *ok = false and the caller divides in FP64.
-__device__ __forceinline__ float ratio(const Top48 &a, const Top48 &b, bool *ok)
+// the normal range, *ok = false and the caller divides in FP64.  rb: about
+// 1 / b.hi.
+__device__ __forceinline__ float recip(const Top48 &b) { return __fdividef(1.f, float(b.hi)); }
+__device__ __forceinline__ float ratio(const Top48 &a, const Top48 &b, float rb, bool *ok)
 {
     const float ah = float(a.hi), al = float(a.lo) * 0x1p-24f;
     const float bh = float(b.hi), bl = float(b.lo) * 0x1p-24f;
-    const float rb = __fdividef(1.f, bh);
     const float q1 = ah * rb;
     const float rem = fmaf(-q1, bl, fmaf(-q1, bh, ah) + al);
     const float q2 = rem * rb;
@@ -285,43 +365,84 @@ __device__ __forceinline__ float ratio(const Top48 &a, const Top48 &b, bool *ok)
     return __uint_as_float(r);
 }
 
+__device__ __forceinline__ float3 pick(bool on, float3 a, float3 b)
+{
+    return make_float3(on ? a.x : b.x, on ? a.y : b.y, on ? a.z : b.z);
+}
+
 } // namespace
 
 // K: chunks of 32 rows per warp (a block owns at most K * kTeamWorkers rows).
 // SKEW: the launch set holds a dihedral-bending instance; skew block parts
 // are kept and applied where an instance has them.
-template <int K, bool SKEW>
+// Of each row the first kRegSlots blocks are in registers where a thread has
+// one row, the others in shared memory: its bandwidth (11 wavefronts per slot
+// and warp, 5 of them for p and the column) bounds the SpMV of a full block.
+// CLUSTER: every team is one thread-block cluster (the launch's cluster size,
+// idle blocks included) and exchanges sums and z rows through its blocks'
+// shared memory: ~400 cycles a sum instead of ~1,500.  Teams are independent,
+// so a launch may have more of them than fit on the GPU at once.
+template <int K, bool SKEW, bool CLUSTER>
 __global__ void __launch_bounds__(kTeamThreads, 1)
     k_pcg_team(InstDesc *const *descs, const TeamBlock *work, TeamSync *sync, SpinCfg sc)
 {
     constexpr int kAll = kTeamThreads;
+    constexpr int RW = team_reg_slots(K, SKEW);
     extern __shared__ float4 sm_dyn[];
     __shared__ InstDesc d;
-    __shared__ float cpart[3][K * kWarps]; // FP32 sums of the 32-row chunks: p.q, r.z, r.r
+    __shared__ int s_dig[3][8];  // digits of the block's sums: p.q, r.z, r.r
+    __shared__ int s_scale[3];   // and their scales
     __shared__ float s_af, s_bf;
     __shared__ int s_stop, s_err, s_go;
+    // cluster: the blocks' sum records (p.q; r.z; r.r), the barriers they and
+    // the z rows are counted on, and where a row of z goes: the blocks whose
+    // columns touch rows of this one
+    __shared__ alignas(16) int4 s_rec[CLUSTER ? 3 : 1][kClusterMax];
+    __shared__ alignas(8) unsigned long long s_bar[3];
+    __shared__ TeamPeer s_peer[CLUSTER ? kClusterMax : 1];
+    __shared__ int s_npeer;
     const TeamBlock w = work[blockIdx.x];
     if (threadIdx.x == 0)
     {
-        d = *descs[w.inst];
         s_stop = 0;
         s_err = 0;
-        s_go = __ldcg(&d.st->active);
+        s_go = 0;
+        if (!CLUSTER || w.inst >= 0)
+        {
+            d = *descs[w.inst];
+            s_go = __ldcg(&d.st->active);
+        }
+        if (CLUSTER)
+        {
+            for (int i = 0; i < 3; i++)
+                asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(s_bar + i))
+                             : "memory");
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        }
     }
     __syncthreads();
+    if (CLUSTER)
+        cluster_sync();
     InstState *st = d.st;
     if (!s_go)
+    {
+        if (CLUSTER)
+            cluster_sync();
         return;
+    }
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nrow = w.row1 - w.row0, nch = (nrow + 31) >> 5, rp = nch << 5;
-    const int nh = w.halo1 - w.halo0, W = d.width;
+    const int nh = w.halo1 - w.halo0, W = max(d.width - RW, 0); // slots in shared memory
     const bool skew = SKEW && d.Aw;
     // the test hook's extra arrivals make a team of one wait too
     const bool multi = w.nblk > 1 || sc.extra != 0u;
     const int it0 = __ldcg(&st->iter);
-    // shared memory: p over the halo, then the rows' blocks by slot
+    // shared memory: p over the halo (z of its rows that other blocks own),
+    // then the rows' blocks by slot
+    const int nhalo = nh - nrow;
     float4 *sp = sm_dyn;
-    float4 *sA0 = sp + nh;
+    float4 *sz = sp + nh;
+    float4 *sA0 = CLUSTER ? sz + nhalo : sz;
     float4 *sAw = sA0 + size_t(W) * rp;
     float2 *sA1 = reinterpret_cast<float2 *>(skew ? sAw + size_t(W) * rp : sAw);
     unsigned short *scol = reinterpret_cast<unsigned short *>(sA1 + size_t(W) * rp);
@@ -329,10 +450,23 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
     if (warp == kWarps)
     {
         // ------------------------------------------------ control warp
-        unsigned long long(*words)[16] = sync[blockIdx.x - w.rank].words;
-        double rho = __ldcg(&st->rho), rr = __ldcg(&st->rr), pq = __ldcg(&st->pq);
+        unsigned long long(*words)[16] = CLUSTER ? nullptr : sync[blockIdx.x - w.rank].words;
+        const unsigned bar_p = smem_u32(s_bar), bar_z = smem_u32(s_bar + 1);
+        // this lane's peer: block lane % 16, sum lane / 16 (r.z, r.r)
+        const int pr_ = lane & (kClusterMax - 1), pq_ = lane / kClusterMax;
+        unsigned to_p = 0, to_z = 0, at_p = 0, at_z = 0;
+        if (CLUSTER && pr_ < w.nblk)
+        {
+            to_p = peer_addr(bar_p, pr_);
+            to_z = peer_addr(bar_z, pr_);
+            at_p = peer_addr(smem_u32(&s_rec[0][w.rank]), pr_);
+            at_z = peer_addr(smem_u32(&s_rec[CLUSTER ? 1 + pq_ : 0][w.rank]), pr_);
+        }
+        unsigned phase = 0;
+        // the scalars as exact sums: what alpha and beta were formed from too
+        Raw pq = raw(__ldcg(&st->pq)), rho = raw(__ldcg(&st->rho)), rr = raw(__ldcg(&st->rr));
+        Raw rho_b = rho, rho_a = rho, pq_a = pq;
         const double alpha0 = __ldcg(&st->alpha), beta0 = __ldcg(&st->beta);
-        double rho_prev = 0.0, rho_alpha = 0.0, pq_alpha = 0.0; // what beta and alpha came from
         bool have_a = false, have_b = false;
         // the convergence threshold on ||r||^2
         const double bb = __ldcg(&st->bb);
@@ -342,43 +476,90 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
         if (d.abs_tol2 > 0.0)
             thr = fmax(thr, d.abs_tol2);
         const bool tests = d.rel_tol2 > 0.0 || d.abs_tol2 > 0.0;
-        const Top48 thr48 = top48(thr);
+        const Top48 thr48 = top48(raw(thr));
         const long long thr_key = key(thr48) + 2;
+        const int check_every = d.check_every, max_iters = d.max_iters;
+        int to_check = check_every - 1 - (it0 + check_every - 1) % check_every;
         Top48 rho48 = top48(rho);
-        int s_pq = fx_scale(pq), s_rho = fx_scale(rho), s_rr = fx_scale(rr);
-        int it = it0, status = 0;
+        float rb_rho = recip(rho48);
+        int s_pq = fx_scale(__ldcg(&st->pq)), s_rho = fx_scale(__ldcg(&st->rho)),
+            s_rr = fx_scale(__ldcg(&st->rr));
+        const unsigned long long target = (unsigned long long)w.nblk + sc.extra;
+        int it = it0, stop = 0;
+        if (lane == 0)
+        {
+            s_scale[0] = s_pq;
+            s_scale[1] = s_rho;
+            s_scale[2] = s_rr;
+        }
+        if (lane < 24)
+            s_dig[lane >> 3][lane & 7] = 0;
+        // the end of the solve is told at the next alpha (the workers' step
+        // towards it changes nothing that is kept)
         bar_sync(6, kAll); // the workers have filled shared memory
         for (;;)
         {
-            unsigned long long *wd = words[it & 3];
+            unsigned long long *wd = CLUSTER ? nullptr : words[it & 3];
             // ---- p.q and alpha
             bar_sync(2, kAll);
-            int stop = *(volatile int *)&s_err ? 9 : 0;
-            Total tq[1];
-            if (!stop)
-            {
-                bool bad[1];
-                i128 v[1];
-                v[0] = fold(cpart[0], nch, s_pq, bad[0]);
-                const int s[1] = {s_pq};
-                if (!multi)
-                    tq[0] = make_total(v[0], s_pq, bad[0]);
-                else if (!team_total<1>(wd, v, bad, s, w.nblk, sc, tq))
-                    stop = 9;
-            }
+            if (*(volatile int *)&s_err)
+                stop = 9;
             float af = 0.f;
+            Top48 pq48 = rho48;
             if (!stop)
             {
-                if (tq[0].bad)
-                    stop = 6;
-                else if (tq[0].H == 0 && tq[0].L == 0ull)
-                    stop = 7;
+                const Digits v = take(s_dig[0]);
+                bool bad = false;
+                if (!multi)
+                    bad = decode(v, s_pq, pq);
+                else if (CLUSTER)
+                {
+                    const int4 c = carried(v);
+                    if (lane == 0)
+                        mbar_expect(bar_p, 16u * (unsigned(w.nblk) + sc.extra));
+                    __syncwarp();
+                    if (lane < w.nblk)
+                        peer_store(at_p, to_p, c.x, c.y, c.z, c.w);
+                    if (mbar_wait(bar_p, phase, sc.limit))
+                        bad = decode(s_rec[0], w.nblk, s_pq, pq);
+                    else
+                        stop = 9;
+                    __syncwarp();
+                }
                 else
                 {
+                    if (lane < 4)
+                        word_add(wd, v, lane);
+                    Words x;
+                    unsigned n = 0;
+                    for (;;)
+                    {
+                        x.load(wd);
+                        if (x.all_in(target))
+                        {
+                            bad = x.decode(w.nblk, s_pq, pq);
+                            break;
+                        }
+                        if (++n > sc.limit)
+                        {
+                            stop = 9;
+                            break;
+                        }
+                        if (n > 256)
+                            __nanosleep(32);
+                    }
+                }
+                if (!stop)
+                {
+                    pq48 = top48(pq);
                     bool ok;
-                    af = ratio(rho48, top48(tq[0]), &ok);
-                    if (!ok)
-                        af = float(rho / total_value(tq[0]));
+                    af = ratio(rho48, pq48, recip(pq48), &ok);
+                    if (bad)
+                        stop = 6;
+                    else if (pq48.hi == 0u)
+                        stop = 7;
+                    else if (!ok)
+                        af = float(value(rho) / value(pq));
                 }
             }
             if (lane == 0)
@@ -388,124 +569,178 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
             }
             __syncwarp();
             bar_arrive(3, kAll);
-            if (stop != 9)
-                pq = total_value(tq[0]);
             if (stop)
-            {
-                status = stop;
                 break;
-            }
-            rho_alpha = rho;
-            pq_alpha = pq;
+            rho_a = rho;
+            pq_a = pq;
             have_a = true;
-            const int s_pq_next = fx_scale(pq);
-            // the buffer of iteration it + 2 was last polled in iteration
-            // it - 2, which every block of the team has left: cleared here,
-            // ordered before this block's next arrivals by the fence below
-            if (w.rank == 0 && lane < 16)
-                words[(it + 2) & 3][lane] = 0ull;
-            const bool check = (it % d.check_every) == 0 || it + 1 >= d.max_iters;
+            s_pq = scale_of(pq, pq48);
+            if (lane == 0)
+                s_scale[0] = s_pq;
             // ---- r.z, r.r and beta
             bar_sync(4, kAll);
-            stop = *(volatile int *)&s_err ? 9 : 0;
-            Total tz[2];
-            if (!stop)
-            {
-                bool bad[2];
-                i128 v[2];
-                v[0] = fold(cpart[1], nch, s_rho, bad[0]);
-                v[1] = fold(cpart[2], nch, s_rr, bad[1]);
-                const int s[2] = {s_rho, s_rr};
-                if (!multi)
-                {
-                    tz[0] = make_total(v[0], s_rho, bad[0]);
-                    tz[1] = make_total(v[1], s_rr, bad[1]);
-                }
-                else if (!team_total<2>(wd + 4, v, bad, s, w.nblk, sc, tz))
-                    stop = 9;
-            }
+            if (*(volatile int *)&s_err)
+                stop = 9;
             float bf = 0.f;
+            Raw rz = rho;
             Top48 new48 = rho48;
-            bool tested = false;
+            Digits v2;
+            Words x, y;
+            bool bad = false;
+            unsigned n = 0;
             if (!stop)
             {
-                new48 = top48(tz[0]);
-                bool ok;
-                bf = ratio(new48, rho48, &ok);
-                if (!ok)
-                    bf = rho == 0.0 ? 0.f : float(total_value(tz[0]) / rho);
-                if (tz[0].bad || tz[1].bad)
-                    stop = 6;
+                const Digits v1 = take(s_dig[1]);
+                v2 = take(s_dig[2]);
+                if (!multi)
+                    bad = decode(v1, s_rho, rz);
+                else if (CLUSTER)
+                {
+                    const int4 c1 = carried(v1), c2 = carried(v2);
+                    const int4 c = pq_ ? c2 : c1;
+                    if (lane == 0)
+                        mbar_expect(bar_z, 32u * (unsigned(w.nblk) + sc.extra));
+                    __syncwarp();
+                    if (pr_ < w.nblk)
+                        peer_store(at_z, to_z, c.x, c.y, c.z, c.w);
+                    if (mbar_wait(bar_z, phase, sc.limit))
+                        bad = decode(s_rec[CLUSTER ? 1 : 0], w.nblk, s_rho, rz);
+                    else
+                        stop = 9;
+                    __syncwarp();
+                }
                 else
                 {
-                    if (check && tests)
+                    if (lane < 8)
+                        word_add(wd + 4 + (lane & 4), lane < 4 ? v1 : v2, lane & 3);
+                    for (;;)
                     {
-                        const bool zero = tz[1].H == 0 && tz[1].L == 0ull;
-                        if (zero || thr48.hi == 0u || key(top48(tz[1])) <= thr_key)
-                            tested = true;
+                        x.load(wd + 4);
+                        if (x.all_in(target))
+                        {
+                            bad = x.decode(w.nblk, s_rho, rz);
+                            break;
+                        }
+                        if (++n > sc.limit)
+                        {
+                            stop = 9;
+                            break;
+                        }
+                        if (n > 256)
+                            __nanosleep(32);
                     }
-                    if (tested)
-                    {
-                        const double v = total_value(tz[1]);
-                        if ((d.rel_tol2 > 0.0 && v <= d.rel_tol2 * bb) ||
-                            (d.abs_tol2 > 0.0 && v <= d.abs_tol2))
-                            stop = 1;
-                    }
-                    if (!stop && it + 1 >= d.max_iters)
-                        stop = 8;
+                }
+                if (!stop)
+                {
+                    new48 = top48(rz);
+                    bool ok;
+                    bf = ratio(new48, rho48, rb_rho, &ok);
+                    if (!ok)
+                        bf = rho48.hi == 0u ? 0.f : float(value(rz) / value(rho));
                 }
             }
             if (lane == 0)
-            {
                 s_bf = bf;
-                s_stop = stop;
-            }
             __syncwarp();
             bar_arrive(5, kAll);
-            if (stop == 9)
-            {
-                status = 9;
-                break;
-            }
-            it++;
-            // FP64 scalars: the next scales, and the state that is reported
-            rho_prev = rho;
-            have_b = true;
-            rho = total_value(tz[0]);
-            rr = total_value(tz[1]);
-            rho48 = new48;
-            s_pq = s_pq_next;
-            s_rho = fx_scale(rho);
-            s_rr = fx_scale(rr);
+            // ---- r.r, the convergence test and the next scales, while the
+            // workers form p and A p
+            phase ^= 1u;
+            if (!stop && multi && !CLUSTER)
+                for (;;)
+                {
+                    y.load(wd + 8);
+                    if (y.all_in(target))
+                        break;
+                    if (++n > sc.limit)
+                    {
+                        stop = 9;
+                        break;
+                    }
+                }
             if (stop)
+                continue; // a wait gave up: told at the next alpha
+            bad |= !multi    ? decode(v2, s_rr, rr)
+                   : CLUSTER ? decode(s_rec[CLUSTER ? 2 : 0], w.nblk, s_rr, rr)
+                             : y.decode(w.nblk, s_rr, rr);
+            it++;
+            rho_b = rho;
+            have_b = true;
+            rho = rz;
+            rho48 = new48;
+            rb_rho = recip(rho48);
+            const Top48 r48 = top48(rr);
+            s_rho = scale_of(rho, rho48);
+            s_rr = scale_of(rr, r48);
+            if (lane == 0)
             {
-                status = stop == 1 ? 0 : stop;
-                break;
+                s_scale[1] = s_rho;
+                s_scale[2] = s_rr;
             }
-            if (multi && w.rank == 0)
-                __threadfence();
+            const bool check = to_check == 0 || it >= max_iters;
+            to_check = to_check == 0 ? check_every - 1 : to_check - 1;
+            if (bad)
+                stop = 6;
+            else
+            {
+                if (check && tests &&
+                    (r48.hi == 0u || thr48.hi == 0u || key(r48) <= thr_key))
+                {
+                    const double v = value(rr);
+                    if ((d.rel_tol2 > 0.0 && v <= d.rel_tol2 * bb) ||
+                        (d.abs_tol2 > 0.0 && v <= d.abs_tol2))
+                        stop = 1;
+                }
+                if (!stop && it >= max_iters)
+                    stop = 8;
+            }
         }
         if (lane == 0)
         {
-            if (status == 9)
+            if (stop == 9)
                 atomicExch(&st->bar_err, 1);
             if (w.rank == 0)
             {
+                const double rho_d = value(rho), b_d = value(rho_b);
                 st->iter = it;
-                st->status = status;
-                st->rho = rho;
-                st->rr = rr;
-                st->pq = pq;
-                st->alpha = have_a ? rho_alpha / pq_alpha : alpha0;
-                st->beta = have_b ? (rho_prev == 0.0 ? 0.0 : rho / rho_prev) : beta0;
+                st->status = stop == 1 ? 0 : stop;
+                st->rho = rho_d;
+                st->rr = value(rr);
+                st->pq = value(pq);
+                st->alpha = have_a ? value(rho_a) / value(pq_a) : alpha0;
+                st->beta = have_b ? (b_d == 0.0 ? 0.0 : rho_d / b_d) : beta0;
                 st->active = 0;
             }
         }
+        if (CLUSTER)
+            cluster_sync();
         return;
     }
 
     // ---------------------------------------------------- workers
-    const int own0 = w.row0 - w.halo0, nhalo = nh - nrow;
+    const int own0 = w.row0 - w.halo0;
+    const unsigned bar_h = smem_u32(s_bar + 2);
+    if (CLUSTER && tid == 0)
+    {
+        int n = 0;
+        for (int j = 0; j < w.nblk; j++)
+        {
+            const TeamBlock o = work[blockIdx.x - w.rank + j];
+            if (j == w.rank || o.halo0 >= w.row1 || o.halo1 <= w.row0)
+                continue;
+            // row i of this block is entry i - halo0 of block j's range, and
+            // that less its own rows in front of it in its z buffer
+            const int own = o.row0 < w.row0 ? o.row1 - o.row0 : 0;
+            const unsigned z_of_j = smem_u32(sm_dyn) + 16u * unsigned(o.halo1 - o.halo0);
+            s_peer[n++] = TeamPeer{max(o.halo0, w.row0), min(o.halo1, w.row1),
+                                   peer_addr(z_of_j, j) - 16u * unsigned(o.halo0 + own),
+                                   peer_addr(bar_h, j)};
+        }
+        s_npeer = n;
+        if (nhalo > 0)
+            mbar_expect(bar_h, 16u * unsigned(nhalo));
+    }
+    unsigned hphase = 0;
     float3 x[K], r[K], z[K], p[K];
     float M[K][6];
     int len[K];
@@ -536,44 +771,82 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
                 const int j = i < own0 ? i : i + nrow;
                 sp[j] = __ldcg(pold + w.halo0 + j);
             }
-        // the rows' blocks: lower slots from their transposed position
-        const int wl = d.width_lo, wu = d.width_up;
+    }
+    // the rows' blocks: lower slots from their transposed position
+    const int wl = d.width_lo, wu = d.width_up;
+    auto block_of = [&](int s, int row, int info, uint32_t &oa) -> int {
+        if (s < ((info >> 8) & 255))
+        {
+            const uint32_t ref = d.lref[lo_idx(s, row, wl)];
+            oa = lref_block(ref, wu);
+            return lref_col(ref) - w.halo0;
+        }
+        oa = up_idx(s - ((info >> 8) & 255), row, wu);
+        return d.colu[oa] - w.halo0;
+    };
+    float rA[RW + 1][6], rw[RW + 1][3];
+    unsigned rc[RW + 1];
+    if (RW > 0)
+    {
+        const int li = warp * 32 + lane, row = w.row0 + li;
+        const int info = li < nrow ? d.rowinfo[row] : 0;
+#pragma unroll
+        for (int s = 0; s < RW; s++)
+        {
+            rc[s] = 0u;
+#pragma unroll
+            for (int i = 0; i < 6; i++)
+                rA[s][i] = 0.f;
+            rw[s][0] = rw[s][1] = rw[s][2] = 0.f;
+            if (s < (info & 255))
+            {
+                uint32_t oa;
+                rc[s] = unsigned(block_of(s, row, info, oa)) * 16u;
+                load_sym(d.A0, d.A1, oa, rA[s]);
+                if (SKEW && skew)
+                {
+                    const float4 aw = d.Aw[oa];
+                    rw[s][0] = aw.x;
+                    rw[s][1] = aw.y;
+                    rw[s][2] = aw.z;
+                }
+            }
+        }
+    }
+    const int ds0 = RW > 0 && warp * 32 + lane < nrow
+                        ? (d.rowinfo[w.row0 + warp * 32 + lane] >> 8) & 255
+                        : 0;
+    {
 #pragma unroll 2
         for (int u = warp; u < W * nch; u += kWarps)
         {
             const int s = u / nch, li = (u - s * nch) * 32 + lane, row = w.row0 + li;
-            if (li >= nrow)
-                continue;
-            const int info = d.rowinfo[row], ds = (info >> 8) & 255;
-            if (s >= (info & 255))
-                continue;
-            uint32_t oa;
-            int c;
-            if (s < ds)
-            {
-                const uint32_t ref = d.lref[lo_idx(s, row, wl)];
-                oa = lref_block(ref, wu);
-                c = lref_col(ref);
-            }
-            else
-            {
-                oa = up_idx(s - ds, row, wu);
-                c = d.colu[oa];
-            }
+            const int info = li < nrow ? d.rowinfo[row] : 0, slot = s + RW;
             const size_t o = size_t(s) * rp + li;
+            if (slot >= (info & 255))
+            {
+                scol[o] = 0; // read where another row of the warp has the slot
+                continue;
+            }
+            uint32_t oa;
+            const int c = block_of(slot, row, info, oa);
             sA0[o] = d.A0[oa];
             sA1[o] = d.A1[oa];
             if (SKEW && skew)
             {
                 float4 aw = d.Aw[oa];
-                aw.w = s < ds ? -1.f : 1.f; // the transposed block's skew part changes sign
+                aw.w = slot < ((info >> 8) & 255) ? -1.f : 1.f; // the transposed block's skew part changes sign
                 sAw[o] = aw;
             }
-            scol[o] = (unsigned short)(c - w.halo0);
+            scol[o] = (unsigned short)c;
         }
     }
     // halo rows of z of the first iteration (written before this launch)
     float3 hz[kHaloAhead];
+    if (CLUSTER)
+        for (int i = tid; i < nhalo; i += kWorkers)
+            sz[i] = __ldcg(d.z + w.halo0 + (i < own0 ? i : i + nrow));
+    else
 #pragma unroll
     for (int u = 0; u < kHaloAhead; u++)
     {
@@ -591,7 +864,9 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
         {
             const int j = i < own0 ? i : i + nrow;
             float3 zz;
-            if (u < kHaloAhead)
+            if (CLUSTER)
+                zz = xyz(sz[i]);
+            else if (u < kHaloAhead)
                 zz = u == 0 ? hz[0] : hz[1];
             else if (tag == unsigned(it0))
                 zz = xyz(__ldcg(d.z + w.halo0 + j));
@@ -622,30 +897,76 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
                 const float4 *a0 = sA0 + li;
                 const float2 *a1 = sA1 + li;
                 const unsigned short *cc = scol + li;
-                // the next slots' blocks and columns are in flight while the
-                // products of these form
-#pragma unroll 4
-                for (int s = 0; s < len[k]; s++)
+                // kAhead slots at a time, loads first and products selected, not
+                // branched around (a branch per slot made the walk three times
+                // as long); a row's planes past its last slot hold column 0
+                constexpr int kAhead = 4;
+                const int n = len[k];
+#pragma unroll
+                for (int s0 = 0; s0 < RW; s0 += kAhead)
                 {
-                    const size_t o = size_t(s) * rp;
-                    const float4 u = a0[o];
-                    const float2 v = a1[o];
-                    const float3 pc = xyz(sp[cc[o]]);
-                    const float A[6] = {u.x, u.y, u.z, u.w, v.x, v.y};
-                    q[k] = q[k] + symv(A, pc);
-                    if (SKEW && skew)
+                    float4 pc[kAhead];
+#pragma unroll
+                    for (int i = 0; i < kAhead; i++)
+                        pc[i] = *reinterpret_cast<const float4 *>(
+                            reinterpret_cast<const char *>(sp) + rc[s0 + i]);
+#pragma unroll
+                    for (int i = 0; i < kAhead; i++)
                     {
-                        const float4 aw = sAw[o + li];
-                        const float3 cw = skewv(aw, pc);
-                        q[k] = aw.w < 0.f ? q[k] - cw : q[k] + cw;
+                        const int s = s0 + i;
+                        float3 t = q[k] + symv(rA[s], xyz(pc[i]));
+                        if (SKEW && skew)
+                        {
+                            const float3 cw = skewv(
+                                make_float4(rw[s][0], rw[s][1], rw[s][2], 0.f), xyz(pc[i]));
+                            t = s < ds0 ? t - cw : t + cw;
+                        }
+                        q[k] = pick(s < n, t, q[k]);
                     }
                 }
-                const float part = warp_sum(li < nrow ? fdot(p[k], q[k]) : 0.f);
-                if (lane == 0)
-                    cpart[0][ch] = part;
+                const int top = __reduce_max_sync(kFull, n - RW);
+                for (int s0 = 0; s0 < top; s0 += kAhead)
+                {
+                    float4 u[kAhead];
+                    float2 v[kAhead];
+                    float4 pc[kAhead];
+                    int o[kAhead];
+#pragma unroll
+                    for (int i = 0; i < kAhead; i++)
+                    {
+                        o[i] = min(s0 + i, top - 1) * rp;
+                        pc[i] = sp[cc[o[i]]];
+                        u[i] = a0[o[i]];
+                        v[i] = a1[o[i]];
+                    }
+#pragma unroll
+                    for (int i = 0; i < kAhead; i++)
+                    {
+                        const float A[6] = {u[i].x, u[i].y, u[i].z, u[i].w, v[i].x, v[i].y};
+                        float3 t = q[k] + symv(A, xyz(pc[i]));
+                        if (SKEW && skew)
+                        {
+                            const float4 aw = sAw[o[i] + li];
+                            const float3 cw = skewv(aw, xyz(pc[i]));
+                            t = aw.w < 0.f ? t - cw : t + cw;
+                        }
+                        q[k] = pick(s0 + i < n - RW, t, q[k]);
+                    }
+                }
+                chunk_add<1>(s_dig[0], warp_sum(li < nrow ? fdot(p[k], q[k]) : 0.f), s_scale[0]);
             }
         }
         bar_arrive(2, kAll);
+        // the sum words of iteration it + 2 were last polled in iteration
+        // it - 2, which every block of the team has left (its r.z words of
+        // it - 1 are in): cleared here, and ordered before this block's next
+        // arrivals, by a warp that is waiting anyway
+        if (!CLUSTER && multi && w.rank == 0 && warp == kWarps - 1)
+        {
+            if (lane < 16)
+                sync[blockIdx.x].words[(tag + 2u) & 3u][lane] = 0ull;
+            __threadfence();
+        }
         bar_sync(3, kAll);
         if (*(volatile int *)&s_stop)
             break;
@@ -665,33 +986,46 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
                     r[k] = make_float3(fmaf(-af, q[k].x, r[k].x), fmaf(-af, q[k].y, r[k].y),
                                        fmaf(-af, q[k].z, r[k].z));
                     z[k] = symv(M[k], r[k]);
-                    if (multi)
+                    if (!CLUSTER && multi)
                         st_row(d.z + w.row0 + li, z[k], tag + 1u);
+                    if (CLUSTER)
+                        for (int j = 0; j < s_npeer; j++)
+                        {
+                            const TeamPeer o = s_peer[j];
+                            const int row = w.row0 + li;
+                            if (row >= o.row0 && row < o.row1)
+                                peer_store(o.z + 16u * unsigned(row), o.bar,
+                                           __float_as_int(z[k].x), __float_as_int(z[k].y),
+                                           __float_as_int(z[k].z), 0);
+                        }
                     pr = fdot(r[k], z[k]);
                     prr = fdot(r[k], r[k]);
                 }
                 pr = warp_sum(pr);
                 prr = warp_sum(prr);
-                if (lane == 0)
-                {
-                    cpart[1][ch] = pr;
-                    cpart[2][ch] = prr;
-                }
+                chunk_add<2>(s_dig[1], lane < 8 ? pr : prr, s_scale[lane < 8 ? 1 : 2]);
             }
         }
         bar_arrive(4, kAll);
         // the halo rows of the new z, while the sums are under way
 #pragma unroll
-        for (int u = 0; u < kHaloAhead; u++)
+        for (int u = 0; u < (CLUSTER ? 0 : kHaloAhead); u++)
         {
             const int i = tid + u * kWorkers;
             if (i < nhalo)
                 hz[u] = poll_row(d.z + w.halo0 + (i < own0 ? i : i + nrow), tag + 1u, sc.limit,
                                  &s_err);
         }
+        if (CLUSTER && nhalo > 0)
+        {
+            if (!mbar_wait(bar_h, hphase, sc.limit))
+                s_err = 1;
+            hphase ^= 1u;
+        }
         bar_sync(5, kAll);
-        if (*(volatile int *)&s_stop)
-            break;
+        // (every worker has seen the phase: the next one may be counted)
+        if (CLUSTER && nhalo > 0 && tid == 0)
+            mbar_expect(bar_h, 16u * unsigned(nhalo));
         bf = *(volatile float *)&s_bf;
     }
 #pragma unroll
@@ -704,13 +1038,21 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
             d.r[row] = f4(r[k]);
         }
     }
+    if (CLUSTER)
+        cluster_sync(); // peers may still be storing here
 }
 
-const void *team_kernel(int chunks_per_warp, bool skew)
+const void *team_kernel(int k, bool skew, bool cluster)
 {
-    if (chunks_per_warp <= 1)
-        return skew ? (const void *)k_pcg_team<1, true> : (const void *)k_pcg_team<1, false>;
-    return skew ? (const void *)k_pcg_team<2, true> : (const void *)k_pcg_team<2, false>;
+    if (cluster)
+        return k <= 1 ? (skew ? (const void *)k_pcg_team<1, true, true>
+                              : (const void *)k_pcg_team<1, false, true>)
+                      : (skew ? (const void *)k_pcg_team<2, true, true>
+                              : (const void *)k_pcg_team<2, false, true>);
+    return k <= 1 ? (skew ? (const void *)k_pcg_team<1, true, false>
+                          : (const void *)k_pcg_team<1, false, false>)
+                  : (skew ? (const void *)k_pcg_team<2, true, false>
+                          : (const void *)k_pcg_team<2, false, false>);
 }
 
 } // namespace cloth
