@@ -130,6 +130,7 @@ struct Batch
     bool persist_1b = false; // single-barrier variant (shared memory, every halo staged)
     bool persist_team = false; // k_pcg_team: the matrix on chip
     int team_rows = 1;         // its rows per thread
+    bool team_half = false;    // k_pcg_half: the stored blocks only
     int team_cluster = 0;      // its teams are clusters of this many blocks (0: not clusters)
     TeamBlock *d_work = nullptr;
     char *d_sync = nullptr;    // behind the work list: arrival counts or team sums
@@ -824,7 +825,7 @@ int make_batch(cloth_ctx *ctx, const std::vector<cloth_s *> &members,
 const void *persistent_kernel(const Batch *b)
 {
     if (b->persist_team)
-        return team_kernel(b->team_rows, b->skew, b->team_cluster > 0);
+        return team_kernel(b->team_rows, b->team_half, b->skew, b->team_cluster > 0);
     if (b->persist_1b)
         return (const void *)k_pcg1_persistent;
     if (b->skew)
@@ -895,31 +896,57 @@ TeamBlock team_block(const Tables &t, int inst, int rank, int r0, int r1)
     return w;
 }
 
-// Adds instance i of b to a k_pcg_team work list in at most `blocks` blocks (K
-// rows a thread, rows in 32-aligned chunks); false when one does not fit its SM.
-bool team_split(const Batch *b, int i, int blocks, int K, bool cluster, size_t cap,
+// An on-chip kernel: k_pcg_team or k_pcg_half (half) with K rows a thread.
+struct TeamKernel
+{
+    int K;
+    bool half;
+};
+
+// Adds instance i of b to an on-chip kernel's work list in at most `blocks`
+// blocks (rows in 32-aligned chunks); false when one does not fit its SM.
+bool team_split(const Batch *b, int i, int blocks, TeamKernel tk, bool cluster, size_t cap,
                 std::vector<TeamBlock> &work, size_t &smem)
 {
     const cloth_s *c = b->members[i];
     const Tables &t = c->tab;
+    const InstDesc &h = c->h;
+    const bool skew = h.Aw != nullptr;
     const size_t first = work.size();
     const int rows =
         ((t.nv + blocks - 1) / blocks + kRedRows - 1) / kRedRows * kRedRows;
-    if (rows > K * kTeamWorkers)
+    if (rows > tk.K * kTeamWorkers || (tk.half && h.width_up > 15))
         return false;
     size_t most = 0;
     for (int r0 = 0; r0 < t.nv; r0 += rows)
     {
         work.push_back(team_block(t, i, int(work.size() - first), r0, std::min(t.nv, r0 + rows)));
-        const TeamBlock &w = work.back();
-        most = std::max(most, team_smem_bytes(w.halo1 - w.halo0, w.row1 - w.row0, c->h.width,
-                                              c->h.Aw != nullptr, team_reg_slots(K, b->skew),
-                                              cluster));
-        if (most > cap || w.halo1 - w.halo0 > 65535)
+        TeamBlock &w = work.back();
+        const int halo = w.halo1 - w.halo0, nr = w.row1 - w.row0;
+        size_t bytes = 0;
+        bool fits = halo <= 65535;
+        if (tk.half)
+        {
+            // as many planes of stored blocks as fit: all, or those from the
+            // first upper one on (the diagonal's serves no lower slot)
+            int planes = h.width_up;
+            while (planes > 0 && half_smem_bytes(halo, nr, planes, h.width_lo + h.width_up, skew,
+                                                 cluster) > cap)
+                planes--;
+            bytes = half_smem_bytes(halo, nr, planes, h.width_lo + h.width_up, skew, cluster);
+            const int u0 = planes == h.width_up ? 0 : 1;
+            w.p_global = u0 | std::min(u0 + planes, h.width_up) << 8;
+            fits = planes >= 2 && halo <= 4096;
+        }
+        else
+            bytes = team_smem_bytes(halo, nr, h.width, skew, team_reg_slots(tk.K, b->skew),
+                                    cluster);
+        if (!fits || bytes > cap)
         {
             work.resize(first);
             return false;
         }
+        most = std::max(most, bytes);
     }
     for (size_t k = first; k < work.size(); k++)
         work[k].nblk = int(work.size() - first);
@@ -929,8 +956,8 @@ bool team_split(const Batch *b, int i, int blocks, int K, bool cluster, size_t c
 
 // Plan of k_pcg_team whose teams are clusters of C blocks (at_once: all of them
 // resident together).
-bool plan_cluster(cloth_ctx *ctx, const Batch *b, int K, int C, std::vector<TeamBlock> &work,
-                  size_t &smem, bool at_once)
+bool plan_cluster(cloth_ctx *ctx, const Batch *b, TeamKernel tk, int C,
+                  std::vector<TeamBlock> &work, size_t &smem, bool at_once)
 {
     const size_t cap = size_t(ctx->max_smem_optin) - 6144;
     const int n = int(b->members.size());
@@ -945,12 +972,12 @@ bool plan_cluster(cloth_ctx *ctx, const Batch *b, int K, int C, std::vector<Team
     });
     for (int i : order)
     {
-        if (!team_split(b, i, C, K, true, cap, work, smem))
+        if (!team_split(b, i, C, tk, true, cap, work, smem))
             return false;
         while (work.size() % size_t(C))
             work.push_back(TeamBlock{-1, 0, 0, 0, 0, 0, 0, 0});
     }
-    const void *f = team_kernel(K, b->skew, true);
+    const void *f = team_kernel(tk.K, tk.half, b->skew, true);
     cudaLaunchConfig_t cfg;
     std::memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3(unsigned(work.size()));
@@ -979,7 +1006,8 @@ bool plan_cluster(cloth_ctx *ctx, const Batch *b, int K, int C, std::vector<Team
 // Plan of k_pcg_team with K rows per thread and teams of any number of blocks,
 // all resident at once: every block's rows, their blocks and p over their
 // columns on its SM.  False when the set does not fit.
-bool plan_team(cloth_ctx *ctx, const Batch *b, int K, std::vector<TeamBlock> &work, size_t &smem)
+bool plan_team(cloth_ctx *ctx, const Batch *b, TeamKernel tk, std::vector<TeamBlock> &work,
+               size_t &smem)
 {
     const int G = std::min(ctx->num_sms, kTeamMaxBlocks);
     const int n = int(b->members.size());
@@ -998,12 +1026,12 @@ bool plan_team(cloth_ctx *ctx, const Batch *b, int K, std::vector<TeamBlock> &wo
             std::max(1ll, (long long)(G - (n - 1)) * nv / std::max(1ll, total));
         const int want =
             std::max(1, std::min<int>(int(share), (nv + kTeamMinRows - 1) / kTeamMinRows));
-        if (!team_split(b, i, want, K, false, cap, work, smem))
+        if (!team_split(b, i, want, tk, false, cap, work, smem))
             return false;
     }
     if (int(work.size()) > G)
         return false;
-    const void *f = team_kernel(K, b->skew, false);
+    const void *f = team_kernel(tk.K, tk.half, b->skew, false);
     int occ = 0;
     if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, int(cap)) !=
             cudaSuccess ||
@@ -1035,22 +1063,33 @@ int plan_persistent(cloth_ctx *ctx, Batch *b)
         int most = 0;
         for (auto *c : b->members)
             most = std::max(most, c->tab.nv);
-        // Clusters where the set's cloths fit them and all run at once.  Up to
-        // 320 rows a block alone is fastest (16^2: 2.3 us per iteration, 2.8
-        // in a cluster of 16; 20^2: 2.7 alone, 2.7 in 8), above it 16 blocks
-        // (32^2: 2.6 us, 2.9 as two blocks), while one row a thread is enough
-        // (64^2: 2.9 us, 3.3 over the whole GPU; 90^2, two rows: 4.8 and 3.4)
-        const int C = most <= kTeamAloneRows ? 1 : kClusterMax;
-        if (plan_cluster(ctx, b, 1, C, work, b->smem_persist, true))
-        {
-            b->team_rows = 1;
+        auto use = [&](TeamKernel k, int C) {
+            b->team_rows = k.K;
+            b->team_half = k.half;
             b->team_cluster = C;
+        };
+        // Clusters where the set's cloths fit them with one row a thread and
+        // all run at once.  Up to 320 rows a block alone is fastest (us per
+        // iteration, 16^2: 2.3, in a cluster of 16 2.8; 20^2: 2.7 and 2.7), above
+        // it 16 blocks (32^2: 2.6, two blocks 2.9; 64^2: 2.9, the whole GPU 3.3;
+        // 80^2: 3.3 and 3.3)
+        const TeamKernel one{1, false};
+        const int C = most <= kTeamAloneRows ? 1 : kClusterMax;
+        if (plan_cluster(ctx, b, one, C, work, b->smem_persist, true))
+        {
+            use(one, C);
             return upload_work(b, work, sizeof(unsigned long long), sizeof(TeamBlock));
         }
-        for (int K = 1; K <= 2; K++)
-            if (plan_team(ctx, b, K, work, b->smem_persist))
+        // Teams over the whole GPU: the whole matrix on chip where it fits (256^2:
+        // 4.7 us with one row a thread, 5.1 with two; 5.3 with the stored blocks
+        // alone), else the stored blocks (300^2: 6.9, the kernel that reads the
+        // matrix from L2 13.0; 512^2: 16.5 and 21.4), with as few rows a thread
+        // as hold the set (362^2: 8.2 with two, 8.6 with three)
+        for (TeamKernel k : {one, TeamKernel{2, false}, TeamKernel{2, true}, TeamKernel{3, true},
+                             TeamKernel{4, true}})
+            if (plan_team(ctx, b, k, work, b->smem_persist))
             {
-                b->team_rows = K;
+                use(k, 0);
                 return upload_work(b, work, sizeof(TeamSync), alignof(TeamSync) * 64);
             }
         b->persist_team = false;

@@ -218,7 +218,8 @@ struct TeamBlock
     int nblk;   // team size
     int row0, row1;
     int halo0, halo1;
-    int p_global; // the team keeps p in global memory (a block of it is not staged)
+    int p_global; // the team keeps p in global memory (a block of it is not staged);
+                  // k_pcg_half: its planes of stored blocks on chip, first | end << 8
 };
 
 // Fixed-point scale: sums are carried as round(v * 2^s) with s chosen from
@@ -274,6 +275,15 @@ __host__ __device__ inline size_t team_smem_bytes(int halo, int rows, int width,
     const size_t rp = size_t((rows + 31) / 32) * 32;
     const size_t planes = width > reg_slots ? width - reg_slots : 0;
     return (size_t(halo) + (cluster ? halo - rows : 0)) * 16 + planes * rp * (skew ? 42 : 26);
+}
+// The same of a k_pcg_half block: planes of stored blocks, and 16-bit words of
+// `words` slots per row.
+__host__ __device__ inline size_t half_smem_bytes(int halo, int rows, int planes, int words,
+                                                  bool skew, bool cluster)
+{
+    const size_t rp = size_t((rows + 31) / 32) * 32;
+    return (size_t(halo) + (cluster ? halo - rows : 0)) * 16 + size_t(planes) * rp * (skew ? 40 : 24) +
+           size_t(words) * rp * 2;
 }
 // A team that is one thread-block cluster: its most blocks, and a block whose
 // halo holds rows [row0, row1) of this one (row i of z goes to z + 16 i in the

@@ -365,6 +365,363 @@ __device__ __forceinline__ float ratio(const Top48 &a, const Top48 &b, float rb,
     return __uint_as_float(r);
 }
 
+// What the warps of a block share; in a cluster also the blocks' sum records
+// (p.q; r.z; r.r), the barriers they and the z rows are counted on, and where a
+// row of z goes: the blocks whose columns touch rows of this one.
+template <bool CLUSTER> struct Shared
+{
+    alignas(16) int4 rec[3][CLUSTER ? kClusterMax : 1];
+    alignas(8) unsigned long long bar[3];
+    TeamPeer peer[CLUSTER ? kClusterMax : 1];
+    int npeer;
+    float af, bf;
+    int stop, err, go;
+};
+
+// Block start: the descriptor and the shared state; false (after the cluster
+// has met twice) when there is nothing to solve.
+template <bool CLUSTER>
+__device__ __forceinline__ bool team_begin(InstDesc *const *descs, const TeamBlock &w, InstDesc &d,
+                                           Shared<CLUSTER> &sh)
+{
+    if (threadIdx.x == 0)
+    {
+        sh.stop = 0;
+        sh.err = 0;
+        sh.go = 0;
+        if (!CLUSTER || w.inst >= 0)
+        {
+            d = *descs[w.inst];
+            sh.go = __ldcg(&d.st->active);
+        }
+        if (CLUSTER)
+        {
+            for (int i = 0; i < 3; i++)
+                asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(sh.bar + i))
+                             : "memory");
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        }
+    }
+    __syncthreads();
+    if (CLUSTER)
+        cluster_sync();
+    if (!sh.go && CLUSTER)
+        cluster_sync();
+    return sh.go != 0;
+}
+
+// One thread of a cluster's block: the blocks that need rows of this one, and
+// the first count of its own halo rows.  z_at: the z buffer of a block whose
+// halo has that many rows, as an offset in its shared memory.
+template <class F>
+__device__ __forceinline__ void find_peers(const TeamBlock *work, const TeamBlock &w,
+                                           Shared<true> &sh, F z_at)
+{
+    const unsigned bar = smem_u32(sh.bar + 2);
+    int n = 0;
+    for (int j = 0; j < w.nblk; j++)
+    {
+        const TeamBlock o = work[blockIdx.x - w.rank + j];
+        if (j == w.rank || o.halo0 >= w.row1 || o.halo1 <= w.row0)
+            continue;
+        // row i of this block is entry i - halo0 of block j's range, and
+        // that less its own rows in front of it in its z buffer
+        const int own = o.row0 < w.row0 ? o.row1 - o.row0 : 0;
+        sh.peer[n++] = TeamPeer{max(o.halo0, w.row0), min(o.halo1, w.row1),
+                                peer_addr(z_at(o.halo1 - o.halo0), j) -
+                                    16u * unsigned(o.halo0 + own),
+                                peer_addr(bar, j)};
+    }
+    sh.npeer = n;
+    const int nhalo = (w.halo1 - w.halo0) - (w.row1 - w.row0);
+    if (nhalo > 0)
+        mbar_expect(bar, 16u * unsigned(nhalo));
+}
+// A row of z to the blocks that need it.
+__device__ __forceinline__ void push_row(const Shared<true> &sh, int row, float3 z)
+{
+    for (int j = 0; j < sh.npeer; j++)
+    {
+        const TeamPeer o = sh.peer[j];
+        if (row >= o.row0 && row < o.row1)
+            peer_store(o.z + 16u * unsigned(row), o.bar, __float_as_int(z.x),
+                       __float_as_int(z.y), __float_as_int(z.z), 0);
+    }
+}
+
+// The control warp of a block: takes the digits the workers have added,
+// exchanges them with the team, forms alpha, beta and the end of the solve, and
+// posts them.
+template <bool CLUSTER>
+__device__ __forceinline__ void control_warp(const InstDesc &d, const TeamBlock &w, TeamSync *sync,
+                                             const SpinCfg &sc, int it0, bool multi,
+                                             Shared<CLUSTER> &sh, int (*dig)[8], int *scale)
+{
+    InstState *st = d.st;
+    const int lane = threadIdx.x & 31;
+    constexpr int kAll = kTeamThreads;
+    unsigned long long(*words)[16] = CLUSTER ? nullptr : sync[blockIdx.x - w.rank].words;
+    const unsigned bar_p = smem_u32(sh.bar), bar_z = smem_u32(sh.bar + 1);
+    // this lane's peer: block lane % 16, sum lane / 16 (r.z, r.r)
+    const int pr_ = lane & (kClusterMax - 1), pq_ = lane / kClusterMax;
+    unsigned to_p = 0, to_z = 0, at_p = 0, at_z = 0;
+    if (CLUSTER && pr_ < w.nblk)
+    {
+        to_p = peer_addr(bar_p, pr_);
+        to_z = peer_addr(bar_z, pr_);
+        at_p = peer_addr(smem_u32(&sh.rec[0][w.rank]), pr_);
+        at_z = peer_addr(smem_u32(&sh.rec[1 + pq_][w.rank]), pr_);
+    }
+    unsigned phase = 0;
+    // the scalars as exact sums: what alpha and beta were formed from too
+    Raw pq = raw(__ldcg(&st->pq)), rho = raw(__ldcg(&st->rho)), rr = raw(__ldcg(&st->rr));
+    Raw rho_b = rho, rho_a = rho, pq_a = pq;
+    const double alpha0 = __ldcg(&st->alpha), beta0 = __ldcg(&st->beta);
+    bool have_a = false, have_b = false;
+    // the convergence threshold on ||r||^2
+    const double bb = __ldcg(&st->bb);
+    double thr = 0.0;
+    if (d.rel_tol2 > 0.0)
+        thr = d.rel_tol2 * bb;
+    if (d.abs_tol2 > 0.0)
+        thr = fmax(thr, d.abs_tol2);
+    const bool tests = d.rel_tol2 > 0.0 || d.abs_tol2 > 0.0;
+    const Top48 thr48 = top48(raw(thr));
+    const long long thr_key = key(thr48) + 2;
+    const int check_every = d.check_every, max_iters = d.max_iters;
+    int to_check = check_every - 1 - (it0 + check_every - 1) % check_every;
+    Top48 rho48 = top48(rho);
+    float rb_rho = recip(rho48);
+    int s_pq = fx_scale(__ldcg(&st->pq)), s_rho = fx_scale(__ldcg(&st->rho)),
+        s_rr = fx_scale(__ldcg(&st->rr));
+    const unsigned long long target = (unsigned long long)w.nblk + sc.extra;
+    int it = it0, stop = 0;
+    if (lane < 3)
+        scale[lane] = lane == 0 ? s_pq : lane == 1 ? s_rho : s_rr;
+    if (lane < 24)
+        dig[lane >> 3][lane & 7] = 0;
+    // the end of the solve is told at the next alpha (the workers' step
+    // towards it changes nothing that is kept)
+    bar_sync(6, kAll); // the workers have filled shared memory
+    for (;;)
+    {
+        unsigned long long *wd = CLUSTER ? nullptr : words[it & 3];
+        // ---- p.q and alpha
+        bar_sync(2, kAll);
+        if (*(volatile int *)&sh.err)
+            stop = 9;
+        float af = 0.f;
+        Top48 pq48 = rho48;
+        if (!stop)
+        {
+            const Digits v = take(dig[0]);
+            bool bad = false;
+            if (!multi)
+                bad = decode(v, s_pq, pq);
+            else if (CLUSTER)
+            {
+                const int4 c = carried(v);
+                if (lane == 0)
+                    mbar_expect(bar_p, 16u * (unsigned(w.nblk) + sc.extra));
+                __syncwarp();
+                if (lane < w.nblk)
+                    peer_store(at_p, to_p, c.x, c.y, c.z, c.w);
+                if (mbar_wait(bar_p, phase, sc.limit))
+                    bad = decode(sh.rec[0], w.nblk, s_pq, pq);
+                else
+                    stop = 9;
+                __syncwarp();
+            }
+            else
+            {
+                if (lane < 4)
+                    word_add(wd, v, lane);
+                Words x;
+                unsigned n = 0;
+                for (;;)
+                {
+                    x.load(wd);
+                    if (x.all_in(target))
+                    {
+                        bad = x.decode(w.nblk, s_pq, pq);
+                        break;
+                    }
+                    if (++n > sc.limit)
+                    {
+                        stop = 9;
+                        break;
+                    }
+                    if (n > 256)
+                        __nanosleep(32);
+                }
+            }
+            if (!stop)
+            {
+                pq48 = top48(pq);
+                bool ok;
+                af = ratio(rho48, pq48, recip(pq48), &ok);
+                if (bad)
+                    stop = 6;
+                else if (pq48.hi == 0u)
+                    stop = 7;
+                else if (!ok)
+                    af = float(value(rho) / value(pq));
+            }
+        }
+        if (lane == 0)
+        {
+            sh.af = af;
+            sh.stop = stop;
+        }
+        __syncwarp();
+        bar_arrive(3, kAll);
+        if (stop)
+            break;
+        rho_a = rho;
+        pq_a = pq;
+        have_a = true;
+        s_pq = scale_of(pq, pq48);
+        if (lane == 0)
+            scale[0] = s_pq;
+        // ---- r.z, r.r and beta
+        bar_sync(4, kAll);
+        if (*(volatile int *)&sh.err)
+            stop = 9;
+        float bf = 0.f;
+        Raw rz = rho;
+        Top48 new48 = rho48;
+        Digits v2;
+        Words x, y;
+        bool bad = false;
+        unsigned n = 0;
+        if (!stop)
+        {
+            const Digits v1 = take(dig[1]);
+            v2 = take(dig[2]);
+            if (!multi)
+                bad = decode(v1, s_rho, rz);
+            else if (CLUSTER)
+            {
+                const int4 c1 = carried(v1), c2 = carried(v2);
+                const int4 c = pq_ ? c2 : c1;
+                if (lane == 0)
+                    mbar_expect(bar_z, 32u * (unsigned(w.nblk) + sc.extra));
+                __syncwarp();
+                if (pr_ < w.nblk)
+                    peer_store(at_z, to_z, c.x, c.y, c.z, c.w);
+                if (mbar_wait(bar_z, phase, sc.limit))
+                    bad = decode(sh.rec[1], w.nblk, s_rho, rz);
+                else
+                    stop = 9;
+                __syncwarp();
+            }
+            else
+            {
+                if (lane < 8)
+                    word_add(wd + 4 + (lane & 4), lane < 4 ? v1 : v2, lane & 3);
+                for (;;)
+                {
+                    x.load(wd + 4);
+                    if (x.all_in(target))
+                    {
+                        bad = x.decode(w.nblk, s_rho, rz);
+                        break;
+                    }
+                    if (++n > sc.limit)
+                    {
+                        stop = 9;
+                        break;
+                    }
+                    if (n > 256)
+                        __nanosleep(32);
+                }
+            }
+            if (!stop)
+            {
+                new48 = top48(rz);
+                bool ok;
+                bf = ratio(new48, rho48, rb_rho, &ok);
+                if (!ok)
+                    bf = rho48.hi == 0u ? 0.f : float(value(rz) / value(rho));
+            }
+        }
+        if (lane == 0)
+            sh.bf = bf;
+        __syncwarp();
+        bar_arrive(5, kAll);
+        // ---- r.r, the convergence test and the next scales, while the
+        // workers form p and A p
+        phase ^= 1u;
+        if (!stop && multi && !CLUSTER)
+            for (;;)
+            {
+                y.load(wd + 8);
+                if (y.all_in(target))
+                    break;
+                if (++n > sc.limit)
+                {
+                    stop = 9;
+                    break;
+                }
+            }
+        if (stop)
+            continue; // a wait gave up: told at the next alpha
+        bad |= !multi    ? decode(v2, s_rr, rr)
+               : CLUSTER ? decode(sh.rec[2], w.nblk, s_rr, rr)
+                         : y.decode(w.nblk, s_rr, rr);
+        it++;
+        rho_b = rho;
+        have_b = true;
+        rho = rz;
+        rho48 = new48;
+        rb_rho = recip(rho48);
+        const Top48 r48 = top48(rr);
+        s_rho = scale_of(rho, rho48);
+        s_rr = scale_of(rr, r48);
+        if (lane == 0)
+        {
+            scale[1] = s_rho;
+            scale[2] = s_rr;
+        }
+        const bool check = to_check == 0 || it >= max_iters;
+        to_check = to_check == 0 ? check_every - 1 : to_check - 1;
+        if (bad)
+            stop = 6;
+        else
+        {
+            if (check && tests &&
+                (r48.hi == 0u || thr48.hi == 0u || key(r48) <= thr_key))
+            {
+                const double v = value(rr);
+                if ((d.rel_tol2 > 0.0 && v <= d.rel_tol2 * bb) ||
+                    (d.abs_tol2 > 0.0 && v <= d.abs_tol2))
+                    stop = 1;
+            }
+            if (!stop && it >= max_iters)
+                stop = 8;
+        }
+    }
+    if (lane == 0)
+    {
+        if (stop == 9)
+            atomicExch(&st->bar_err, 1);
+        if (w.rank == 0)
+        {
+            const double rho_d = value(rho), b_d = value(rho_b);
+            st->iter = it;
+            st->status = stop == 1 ? 0 : stop;
+            st->rho = rho_d;
+            st->rr = value(rr);
+            st->pq = value(pq);
+            st->alpha = have_a ? value(rho_a) / value(pq_a) : alpha0;
+            st->beta = have_b ? (b_d == 0.0 ? 0.0 : rho_d / b_d) : beta0;
+            st->active = 0;
+        }
+    }
+    if (CLUSTER)
+        cluster_sync();
+}
+
 __device__ __forceinline__ float3 pick(bool on, float3 a, float3 b)
 {
     return make_float3(on ? a.x : b.x, on ? a.y : b.y, on ? a.z : b.z);
@@ -392,44 +749,11 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
     __shared__ InstDesc d;
     __shared__ int s_dig[3][8];  // digits of the block's sums: p.q, r.z, r.r
     __shared__ int s_scale[3];   // and their scales
-    __shared__ float s_af, s_bf;
-    __shared__ int s_stop, s_err, s_go;
-    // cluster: the blocks' sum records (p.q; r.z; r.r), the barriers they and
-    // the z rows are counted on, and where a row of z goes: the blocks whose
-    // columns touch rows of this one
-    __shared__ alignas(16) int4 s_rec[CLUSTER ? 3 : 1][kClusterMax];
-    __shared__ alignas(8) unsigned long long s_bar[3];
-    __shared__ TeamPeer s_peer[CLUSTER ? kClusterMax : 1];
-    __shared__ int s_npeer;
+    __shared__ Shared<CLUSTER> sh;
     const TeamBlock w = work[blockIdx.x];
-    if (threadIdx.x == 0)
-    {
-        s_stop = 0;
-        s_err = 0;
-        s_go = 0;
-        if (!CLUSTER || w.inst >= 0)
-        {
-            d = *descs[w.inst];
-            s_go = __ldcg(&d.st->active);
-        }
-        if (CLUSTER)
-        {
-            for (int i = 0; i < 3; i++)
-                asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(s_bar + i))
-                             : "memory");
-            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        }
-    }
-    __syncthreads();
-    if (CLUSTER)
-        cluster_sync();
-    InstState *st = d.st;
-    if (!s_go)
-    {
-        if (CLUSTER)
-            cluster_sync();
+    if (!team_begin(descs, w, d, sh))
         return;
-    }
+    InstState *st = d.st;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nrow = w.row1 - w.row0, nch = (nrow + 31) >> 5, rp = nch << 5;
     const int nh = w.halo1 - w.halo0, W = max(d.width - RW, 0); // slots in shared memory
@@ -449,297 +773,16 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
 
     if (warp == kWarps)
     {
-        // ------------------------------------------------ control warp
-        unsigned long long(*words)[16] = CLUSTER ? nullptr : sync[blockIdx.x - w.rank].words;
-        const unsigned bar_p = smem_u32(s_bar), bar_z = smem_u32(s_bar + 1);
-        // this lane's peer: block lane % 16, sum lane / 16 (r.z, r.r)
-        const int pr_ = lane & (kClusterMax - 1), pq_ = lane / kClusterMax;
-        unsigned to_p = 0, to_z = 0, at_p = 0, at_z = 0;
-        if (CLUSTER && pr_ < w.nblk)
-        {
-            to_p = peer_addr(bar_p, pr_);
-            to_z = peer_addr(bar_z, pr_);
-            at_p = peer_addr(smem_u32(&s_rec[0][w.rank]), pr_);
-            at_z = peer_addr(smem_u32(&s_rec[CLUSTER ? 1 + pq_ : 0][w.rank]), pr_);
-        }
-        unsigned phase = 0;
-        // the scalars as exact sums: what alpha and beta were formed from too
-        Raw pq = raw(__ldcg(&st->pq)), rho = raw(__ldcg(&st->rho)), rr = raw(__ldcg(&st->rr));
-        Raw rho_b = rho, rho_a = rho, pq_a = pq;
-        const double alpha0 = __ldcg(&st->alpha), beta0 = __ldcg(&st->beta);
-        bool have_a = false, have_b = false;
-        // the convergence threshold on ||r||^2
-        const double bb = __ldcg(&st->bb);
-        double thr = 0.0;
-        if (d.rel_tol2 > 0.0)
-            thr = d.rel_tol2 * bb;
-        if (d.abs_tol2 > 0.0)
-            thr = fmax(thr, d.abs_tol2);
-        const bool tests = d.rel_tol2 > 0.0 || d.abs_tol2 > 0.0;
-        const Top48 thr48 = top48(raw(thr));
-        const long long thr_key = key(thr48) + 2;
-        const int check_every = d.check_every, max_iters = d.max_iters;
-        int to_check = check_every - 1 - (it0 + check_every - 1) % check_every;
-        Top48 rho48 = top48(rho);
-        float rb_rho = recip(rho48);
-        int s_pq = fx_scale(__ldcg(&st->pq)), s_rho = fx_scale(__ldcg(&st->rho)),
-            s_rr = fx_scale(__ldcg(&st->rr));
-        const unsigned long long target = (unsigned long long)w.nblk + sc.extra;
-        int it = it0, stop = 0;
-        if (lane == 0)
-        {
-            s_scale[0] = s_pq;
-            s_scale[1] = s_rho;
-            s_scale[2] = s_rr;
-        }
-        if (lane < 24)
-            s_dig[lane >> 3][lane & 7] = 0;
-        // the end of the solve is told at the next alpha (the workers' step
-        // towards it changes nothing that is kept)
-        bar_sync(6, kAll); // the workers have filled shared memory
-        for (;;)
-        {
-            unsigned long long *wd = CLUSTER ? nullptr : words[it & 3];
-            // ---- p.q and alpha
-            bar_sync(2, kAll);
-            if (*(volatile int *)&s_err)
-                stop = 9;
-            float af = 0.f;
-            Top48 pq48 = rho48;
-            if (!stop)
-            {
-                const Digits v = take(s_dig[0]);
-                bool bad = false;
-                if (!multi)
-                    bad = decode(v, s_pq, pq);
-                else if (CLUSTER)
-                {
-                    const int4 c = carried(v);
-                    if (lane == 0)
-                        mbar_expect(bar_p, 16u * (unsigned(w.nblk) + sc.extra));
-                    __syncwarp();
-                    if (lane < w.nblk)
-                        peer_store(at_p, to_p, c.x, c.y, c.z, c.w);
-                    if (mbar_wait(bar_p, phase, sc.limit))
-                        bad = decode(s_rec[0], w.nblk, s_pq, pq);
-                    else
-                        stop = 9;
-                    __syncwarp();
-                }
-                else
-                {
-                    if (lane < 4)
-                        word_add(wd, v, lane);
-                    Words x;
-                    unsigned n = 0;
-                    for (;;)
-                    {
-                        x.load(wd);
-                        if (x.all_in(target))
-                        {
-                            bad = x.decode(w.nblk, s_pq, pq);
-                            break;
-                        }
-                        if (++n > sc.limit)
-                        {
-                            stop = 9;
-                            break;
-                        }
-                        if (n > 256)
-                            __nanosleep(32);
-                    }
-                }
-                if (!stop)
-                {
-                    pq48 = top48(pq);
-                    bool ok;
-                    af = ratio(rho48, pq48, recip(pq48), &ok);
-                    if (bad)
-                        stop = 6;
-                    else if (pq48.hi == 0u)
-                        stop = 7;
-                    else if (!ok)
-                        af = float(value(rho) / value(pq));
-                }
-            }
-            if (lane == 0)
-            {
-                s_af = af;
-                s_stop = stop;
-            }
-            __syncwarp();
-            bar_arrive(3, kAll);
-            if (stop)
-                break;
-            rho_a = rho;
-            pq_a = pq;
-            have_a = true;
-            s_pq = scale_of(pq, pq48);
-            if (lane == 0)
-                s_scale[0] = s_pq;
-            // ---- r.z, r.r and beta
-            bar_sync(4, kAll);
-            if (*(volatile int *)&s_err)
-                stop = 9;
-            float bf = 0.f;
-            Raw rz = rho;
-            Top48 new48 = rho48;
-            Digits v2;
-            Words x, y;
-            bool bad = false;
-            unsigned n = 0;
-            if (!stop)
-            {
-                const Digits v1 = take(s_dig[1]);
-                v2 = take(s_dig[2]);
-                if (!multi)
-                    bad = decode(v1, s_rho, rz);
-                else if (CLUSTER)
-                {
-                    const int4 c1 = carried(v1), c2 = carried(v2);
-                    const int4 c = pq_ ? c2 : c1;
-                    if (lane == 0)
-                        mbar_expect(bar_z, 32u * (unsigned(w.nblk) + sc.extra));
-                    __syncwarp();
-                    if (pr_ < w.nblk)
-                        peer_store(at_z, to_z, c.x, c.y, c.z, c.w);
-                    if (mbar_wait(bar_z, phase, sc.limit))
-                        bad = decode(s_rec[CLUSTER ? 1 : 0], w.nblk, s_rho, rz);
-                    else
-                        stop = 9;
-                    __syncwarp();
-                }
-                else
-                {
-                    if (lane < 8)
-                        word_add(wd + 4 + (lane & 4), lane < 4 ? v1 : v2, lane & 3);
-                    for (;;)
-                    {
-                        x.load(wd + 4);
-                        if (x.all_in(target))
-                        {
-                            bad = x.decode(w.nblk, s_rho, rz);
-                            break;
-                        }
-                        if (++n > sc.limit)
-                        {
-                            stop = 9;
-                            break;
-                        }
-                        if (n > 256)
-                            __nanosleep(32);
-                    }
-                }
-                if (!stop)
-                {
-                    new48 = top48(rz);
-                    bool ok;
-                    bf = ratio(new48, rho48, rb_rho, &ok);
-                    if (!ok)
-                        bf = rho48.hi == 0u ? 0.f : float(value(rz) / value(rho));
-                }
-            }
-            if (lane == 0)
-                s_bf = bf;
-            __syncwarp();
-            bar_arrive(5, kAll);
-            // ---- r.r, the convergence test and the next scales, while the
-            // workers form p and A p
-            phase ^= 1u;
-            if (!stop && multi && !CLUSTER)
-                for (;;)
-                {
-                    y.load(wd + 8);
-                    if (y.all_in(target))
-                        break;
-                    if (++n > sc.limit)
-                    {
-                        stop = 9;
-                        break;
-                    }
-                }
-            if (stop)
-                continue; // a wait gave up: told at the next alpha
-            bad |= !multi    ? decode(v2, s_rr, rr)
-                   : CLUSTER ? decode(s_rec[CLUSTER ? 2 : 0], w.nblk, s_rr, rr)
-                             : y.decode(w.nblk, s_rr, rr);
-            it++;
-            rho_b = rho;
-            have_b = true;
-            rho = rz;
-            rho48 = new48;
-            rb_rho = recip(rho48);
-            const Top48 r48 = top48(rr);
-            s_rho = scale_of(rho, rho48);
-            s_rr = scale_of(rr, r48);
-            if (lane == 0)
-            {
-                s_scale[1] = s_rho;
-                s_scale[2] = s_rr;
-            }
-            const bool check = to_check == 0 || it >= max_iters;
-            to_check = to_check == 0 ? check_every - 1 : to_check - 1;
-            if (bad)
-                stop = 6;
-            else
-            {
-                if (check && tests &&
-                    (r48.hi == 0u || thr48.hi == 0u || key(r48) <= thr_key))
-                {
-                    const double v = value(rr);
-                    if ((d.rel_tol2 > 0.0 && v <= d.rel_tol2 * bb) ||
-                        (d.abs_tol2 > 0.0 && v <= d.abs_tol2))
-                        stop = 1;
-                }
-                if (!stop && it >= max_iters)
-                    stop = 8;
-            }
-        }
-        if (lane == 0)
-        {
-            if (stop == 9)
-                atomicExch(&st->bar_err, 1);
-            if (w.rank == 0)
-            {
-                const double rho_d = value(rho), b_d = value(rho_b);
-                st->iter = it;
-                st->status = stop == 1 ? 0 : stop;
-                st->rho = rho_d;
-                st->rr = value(rr);
-                st->pq = value(pq);
-                st->alpha = have_a ? value(rho_a) / value(pq_a) : alpha0;
-                st->beta = have_b ? (b_d == 0.0 ? 0.0 : rho_d / b_d) : beta0;
-                st->active = 0;
-            }
-        }
-        if (CLUSTER)
-            cluster_sync();
+        control_warp<CLUSTER>(d, w, sync, sc, it0, multi, sh, s_dig, s_scale);
         return;
     }
 
     // ---------------------------------------------------- workers
     const int own0 = w.row0 - w.halo0;
-    const unsigned bar_h = smem_u32(s_bar + 2);
-    if (CLUSTER && tid == 0)
-    {
-        int n = 0;
-        for (int j = 0; j < w.nblk; j++)
-        {
-            const TeamBlock o = work[blockIdx.x - w.rank + j];
-            if (j == w.rank || o.halo0 >= w.row1 || o.halo1 <= w.row0)
-                continue;
-            // row i of this block is entry i - halo0 of block j's range, and
-            // that less its own rows in front of it in its z buffer
-            const int own = o.row0 < w.row0 ? o.row1 - o.row0 : 0;
-            const unsigned z_of_j = smem_u32(sm_dyn) + 16u * unsigned(o.halo1 - o.halo0);
-            s_peer[n++] = TeamPeer{max(o.halo0, w.row0), min(o.halo1, w.row1),
-                                   peer_addr(z_of_j, j) - 16u * unsigned(o.halo0 + own),
-                                   peer_addr(bar_h, j)};
-        }
-        s_npeer = n;
-        if (nhalo > 0)
-            mbar_expect(bar_h, 16u * unsigned(nhalo));
-    }
+    const unsigned bar_h = smem_u32(sh.bar + 2);
+    if constexpr (CLUSTER)
+        if (tid == 0)
+            find_peers(work, w, sh, [](int halo) { return smem_u32(sm_dyn) + 16u * unsigned(halo); });
     unsigned hphase = 0;
     float3 x[K], r[K], z[K], p[K];
     float M[K][6];
@@ -871,7 +914,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
             else if (tag == unsigned(it0))
                 zz = xyz(__ldcg(d.z + w.halo0 + j));
             else
-                zz = poll_row(d.z + w.halo0 + j, tag, sc.limit, &s_err);
+                zz = poll_row(d.z + w.halo0 + j, tag, sc.limit, &sh.err);
             sp[j] = f4(first ? zz : pform(zz, bf, xyz(sp[j])));
         }
 #pragma unroll
@@ -968,9 +1011,9 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
             __threadfence();
         }
         bar_sync(3, kAll);
-        if (*(volatile int *)&s_stop)
+        if (*(volatile int *)&sh.stop)
             break;
-        const float af = *(volatile float *)&s_af;
+        const float af = *(volatile float *)&sh.af;
         // ---- dx += alpha p, r -= alpha q, z = M^-1 r; r.z and r.r per chunk
 #pragma unroll
         for (int k = 0; k < K; k++)
@@ -988,16 +1031,8 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
                     z[k] = symv(M[k], r[k]);
                     if (!CLUSTER && multi)
                         st_row(d.z + w.row0 + li, z[k], tag + 1u);
-                    if (CLUSTER)
-                        for (int j = 0; j < s_npeer; j++)
-                        {
-                            const TeamPeer o = s_peer[j];
-                            const int row = w.row0 + li;
-                            if (row >= o.row0 && row < o.row1)
-                                peer_store(o.z + 16u * unsigned(row), o.bar,
-                                           __float_as_int(z[k].x), __float_as_int(z[k].y),
-                                           __float_as_int(z[k].z), 0);
-                        }
+                    if constexpr (CLUSTER)
+                        push_row(sh, w.row0 + li, z[k]);
                     pr = fdot(r[k], z[k]);
                     prr = fdot(r[k], r[k]);
                 }
@@ -1014,19 +1049,19 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
             const int i = tid + u * kWorkers;
             if (i < nhalo)
                 hz[u] = poll_row(d.z + w.halo0 + (i < own0 ? i : i + nrow), tag + 1u, sc.limit,
-                                 &s_err);
+                                 &sh.err);
         }
         if (CLUSTER && nhalo > 0)
         {
             if (!mbar_wait(bar_h, hphase, sc.limit))
-                s_err = 1;
+                sh.err = 1;
             hphase ^= 1u;
         }
         bar_sync(5, kAll);
         // (every worker has seen the phase: the next one may be counted)
         if (CLUSTER && nhalo > 0 && tid == 0)
             mbar_expect(bar_h, 16u * unsigned(nhalo));
-        bf = *(volatile float *)&s_bf;
+        bf = *(volatile float *)&sh.bf;
     }
 #pragma unroll
     for (int k = 0; k < K; k++)
@@ -1042,8 +1077,380 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
         cluster_sync(); // peers may still be storing here
 }
 
-const void *team_kernel(int k, bool skew, bool cluster)
+// The same solve for blocks with more rows than fit with their whole matrix:
+// only the diagonal and upper blocks are kept, each read by its own row and by
+// the rows whose lower block is its transpose.  Where not even those fit, the
+// planes [u0, u1) of them are on chip (the first upper ones, which serve lower
+// slots too; the work list says which), the others and the lower blocks whose
+// transposed row another block owns come from L2.  A column and the transposed
+// block's plane share one 16-bit word.  K: rows per thread.
+template <int K, bool SKEW, bool CLUSTER>
+__global__ void __launch_bounds__(kTeamThreads, 1)
+    k_pcg_half(InstDesc *const *descs, const TeamBlock *work, TeamSync *sync, SpinCfg sc)
 {
+    constexpr int kAll = kTeamThreads;
+    constexpr int kAhead3 = 3; // halo rows per thread polled before beta is known
+    extern __shared__ float4 sm_dyn[];
+    __shared__ InstDesc d;
+    __shared__ int s_dig[3][8];
+    __shared__ int s_scale[3];
+    __shared__ Shared<CLUSTER> sh;
+    const TeamBlock w = work[blockIdx.x];
+    if (!team_begin(descs, w, d, sh))
+        return;
+    InstState *st = d.st;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int nrow = w.row1 - w.row0, nch = (nrow + 31) >> 5, rp = nch << 5;
+    const int nh = w.halo1 - w.halo0, nhalo = nh - nrow;
+    const bool skew = SKEW && d.Aw;
+    const bool multi = w.nblk > 1 || sc.extra != 0u;
+    const int it0 = __ldcg(&st->iter);
+    const int u0 = w.p_global & 255, u1 = w.p_global >> 8; // planes on chip
+    const int wl = d.width_lo, wu = d.width_up;
+    float4 *sp = sm_dyn;
+    float4 *sz = sp + nh;
+    float4 *sU0 = CLUSTER ? sz + nhalo : sz;
+    float4 *sUw = sU0 + size_t(u1 - u0) * rp;
+    float2 *sU1 = reinterpret_cast<float2 *>(skew ? sUw + size_t(u1 - u0) * rp : sUw);
+    // words of the lower slots (column | plane << 12), then of the upper planes
+    unsigned short *scol = reinterpret_cast<unsigned short *>(sU1 + size_t(u1 - u0) * rp);
+    if (warp == kWarps)
+    {
+        control_warp<CLUSTER>(d, w, sync, sc, it0, multi, sh, s_dig, s_scale);
+        return;
+    }
+    const int own0 = w.row0 - w.halo0;
+    const unsigned bar_h = smem_u32(sh.bar + 2);
+    if constexpr (CLUSTER)
+        if (tid == 0)
+            find_peers(work, w, sh, [](int halo) { return smem_u32(sm_dyn) + 16u * unsigned(halo); });
+    unsigned hphase = 0;
+    float3 x[K], r[K], z[K];
+    int info[K];
+    const float4 *pold = (it0 & 1) ? d.p1 : d.p0;
+#pragma unroll
+    for (int k = 0; k < K; k++)
+    {
+        const int li = (warp + k * kWarps) * 32 + lane, row = w.row0 + li;
+        info[k] = 0;
+        x[k] = r[k] = z[k] = make_float3(0.f, 0.f, 0.f);
+        if (li < nrow)
+        {
+            info[k] = d.rowinfo[row];
+            x[k] = xyz(d.dx[row]);
+            r[k] = xyz(d.r[row]);
+            z[k] = xyz(d.z[row]);
+        }
+    }
+    if (it0 > 0) // a solve handed over in its middle
+        for (int i = tid; i < nh; i += kWorkers)
+            sp[i] = __ldcg(pold + w.halo0 + i);
+#pragma unroll 4
+    for (int u = warp; u < (wl + wu) * nch; u += kWarps)
+    {
+        const int s = u / nch, li = (u - s * nch) * 32 + lane, row = w.row0 + li;
+        const int inf = li < nrow ? d.rowinfo[row] : 0, ds = (inf >> 8) & 255;
+        const bool upper = s >= wl;
+        const int uu = s - wl; // upper plane
+        unsigned short word = 0;
+        if (upper ? uu < (inf & 255) - ds : s < ds)
+        {
+            if (upper)
+            {
+                const uint32_t oa = up_idx(uu, row, wu);
+                word = (unsigned short)(d.colu[oa] - w.halo0);
+                if (uu >= u0 && uu < u1)
+                {
+                    const size_t o = size_t(uu - u0) * rp + li;
+                    sU0[o] = d.A0[oa];
+                    sU1[o] = d.A1[oa];
+                    if (SKEW && skew)
+                        sUw[o] = d.Aw[oa];
+                }
+            }
+            else
+            {
+                const uint32_t ref = d.lref[lo_idx(s, row, wl)];
+                word = (unsigned short)((lref_col(ref) - w.halo0) | int(ref >> 24) << 12);
+            }
+        }
+        scol[size_t(s) * rp + li] = word;
+    }
+    // halo rows of z of the first iteration (written before this launch)
+    float3 hz[kAhead3];
+    if (CLUSTER)
+        for (int i = tid; i < nhalo; i += kWorkers)
+            sz[i] = __ldcg(d.z + w.halo0 + (i < own0 ? i : i + nrow));
+    else
+#pragma unroll
+        for (int u = 0; u < kAhead3; u++)
+        {
+            const int i = tid + u * kWorkers;
+            hz[u] = make_float3(0.f, 0.f, 0.f);
+            if (i < nhalo)
+                hz[u] = xyz(__ldcg(d.z + w.halo0 + (i < own0 ? i : i + nrow)));
+        }
+    float bf = float(__ldcg(&st->beta));
+    bar_sync(6, kAll);
+    for (unsigned tag = unsigned(it0);; tag++)
+    {
+        // ---- p = z + beta p_old over the halo and the own rows
+        const bool first = bf == 0.f;
+        for (int i = tid, u = 0; i < nhalo; i += kWorkers, u++)
+        {
+            const int j = i < own0 ? i : i + nrow;
+            float3 zz;
+            if (CLUSTER)
+                zz = xyz(sz[i]);
+            else if (u < kAhead3)
+                zz = u == 0 ? hz[0] : u == 1 ? hz[1] : hz[2];
+            else if (tag == unsigned(it0))
+                zz = xyz(__ldcg(d.z + w.halo0 + j));
+            else
+                zz = poll_row(d.z + w.halo0 + j, tag, sc.limit, &sh.err);
+            sp[j] = f4(first ? zz : pform(zz, bf, xyz(sp[j])));
+        }
+#pragma unroll
+        for (int k = 0; k < K; k++)
+        {
+            const int li = (warp + k * kWarps) * 32 + lane;
+            if (li < nrow)
+                sp[own0 + li] = f4(first ? z[k] : pform(z[k], bf, xyz(sp[own0 + li])));
+        }
+        bar_sync(1, kWorkers);
+        // ---- q = A p; p.q per 32-row chunk
+        float3 q[K];
+#pragma unroll
+        for (int k = 0; k < K; k++)
+        {
+            const int ch = warp + k * kWarps, li = ch * 32 + lane, row = w.row0 + li;
+            q[k] = make_float3(0.f, 0.f, 0.f);
+            if (ch < nch)
+            {
+                const int ds = (info[k] >> 8) & 255, ne = (info[k] & 255) - ds;
+                const int top_l = __reduce_max_sync(kFull, ds),
+                          top_u = __reduce_max_sync(kFull, ne);
+                const unsigned short *cc = scol + li;
+                auto add = [&](bool on, float4 a0, float2 a1, float4 aw, float3 pc, bool lower) {
+                    const float A[6] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y};
+                    float3 t = q[k] + symv(A, pc);
+                    if (SKEW && skew)
+                    {
+                        const float3 cw = skewv(aw, pc);
+                        t = lower ? t - cw : t + cw;
+                    }
+                    q[k] = pick(on, t, q[k]);
+                };
+                const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+                // upper planes that are not on chip: the first three in flight
+                // from here
+                constexpr int kPre = 3;
+                float4 f0[kPre], fw[kPre];
+                float2 f1[kPre];
+#pragma unroll
+                for (int i = 0; i < kPre; i++)
+                {
+                    const int u = i == 0 ? 0 : u1 + i - 1;
+                    f0[i] = fw[i] = zero4;
+                    f1[i] = make_float2(0.f, 0.f);
+                    if ((i > 0 || u0 > 0) && u < ne)
+                    {
+                        const uint32_t oa = up_idx(u, row, wu);
+                        f0[i] = __ldg(d.A0 + oa);
+                        f1[i] = __ldg(d.A1 + oa);
+                        if (SKEW && skew)
+                            fw[i] = __ldg(d.Aw + oa);
+                    }
+                }
+                // lower slots, kLow at a time, their blocks first
+                constexpr int kLow = 3;
+                for (int s0 = 0; s0 < top_l; s0 += kLow)
+                {
+                    float4 a0[kLow], aw[kLow], pc[kLow];
+                    float2 a1[kLow];
+#pragma unroll
+                    for (int i = 0; i < kLow; i++)
+                    {
+                        const unsigned wd = cc[min(s0 + i, top_l - 1) * rp];
+                        const int c = int(wd & 4095u), u = int(wd >> 12), lr = c - own0;
+                        a0[i] = aw[i] = zero4;
+                        a1[i] = make_float2(0.f, 0.f);
+                        pc[i] = sp[c];
+                        if (unsigned(lr) < unsigned(nrow) && unsigned(u - u0) < unsigned(u1 - u0))
+                        {
+                            const int o = (u - u0) * rp + lr;
+                            a0[i] = sU0[o];
+                            a1[i] = sU1[o];
+                            if (SKEW && skew)
+                                aw[i] = sUw[o];
+                        }
+                        else if (s0 + i < ds)
+                        {
+                            const uint32_t oa = up_idx(u, c + w.halo0, wu);
+                            a0[i] = __ldg(d.A0 + oa);
+                            a1[i] = __ldg(d.A1 + oa);
+                            if (SKEW && skew)
+                                aw[i] = __ldg(d.Aw + oa);
+                        }
+                    }
+#pragma unroll
+                    for (int i = 0; i < kLow; i++)
+                        add(s0 + i < ds, a0[i], a1[i], aw[i], xyz(pc[i]), true);
+                }
+                // upper slots in order
+                const unsigned short *cu = cc + wl * rp;
+                if (u0 > 0)
+                    add(ne > 0, f0[0], f1[0], fw[0], xyz(sp[cu[0]]), false);
+                const int top_r = min(top_u, u1);
+                constexpr int kUp = 3;
+                for (int b = u0; b < top_r; b += kUp)
+                {
+                    float4 a0[kUp], aw[kUp], pc[kUp];
+                    float2 a1[kUp];
+#pragma unroll
+                    for (int i = 0; i < kUp; i++)
+                    {
+                        const int u = min(b + i, top_r - 1), o = (u - u0) * rp + li;
+                        pc[i] = sp[cu[u * rp]];
+                        a0[i] = sU0[o];
+                        a1[i] = sU1[o];
+                        aw[i] = zero4;
+                        if (SKEW && skew)
+                            aw[i] = sUw[o];
+                    }
+#pragma unroll
+                    for (int i = 0; i < kUp; i++)
+                        add(b + i < min(ne, u1), a0[i], a1[i], aw[i], xyz(pc[i]), false);
+                }
+#pragma unroll
+                for (int i = 1; i < kPre; i++)
+                    if (u1 + i - 1 < top_u)
+                        add(u1 + i - 1 < ne, f0[i], f1[i], fw[i], xyz(sp[cu[(u1 + i - 1) * rp]]),
+                            false);
+                for (int u = u1 + kPre - 1; u < top_u; u++)
+                {
+                    float4 a0 = zero4, aw = zero4;
+                    float2 a1 = make_float2(0.f, 0.f);
+                    if (u < ne)
+                    {
+                        const uint32_t oa = up_idx(u, row, wu);
+                        a0 = __ldg(d.A0 + oa);
+                        a1 = __ldg(d.A1 + oa);
+                        if (SKEW && skew)
+                            aw = __ldg(d.Aw + oa);
+                    }
+                    add(u < ne, a0, a1, aw, xyz(sp[cu[u * rp]]), false);
+                }
+                const float3 pv = xyz(sp[own0 + min(li, nrow - 1)]);
+                chunk_add<1>(s_dig[0], warp_sum(li < nrow ? fdot(pv, q[k]) : 0.f), s_scale[0]);
+            }
+        }
+        bar_arrive(2, kAll);
+        if (!CLUSTER && multi && w.rank == 0 && warp == kWarps - 1)
+        {
+            // the sum words of iteration it + 2 (see k_pcg_team)
+            if (lane < 16)
+                sync[blockIdx.x].words[(tag + 2u) & 3u][lane] = 0ull;
+            __threadfence();
+        }
+        // the inverse diagonal blocks, in flight while alpha is awaited
+        float4 m0[K];
+        float2 m1[K];
+#pragma unroll
+        for (int k = 0; k < K; k++)
+        {
+            const int li = (warp + k * kWarps) * 32 + lane;
+            m0[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+            m1[k] = make_float2(0.f, 0.f);
+            if (li < nrow)
+            {
+                m0[k] = __ldg(d.M0 + w.row0 + li);
+                m1[k] = __ldg(d.M1 + w.row0 + li);
+            }
+        }
+        bar_sync(3, kAll);
+        if (*(volatile int *)&sh.stop)
+            break;
+        const float af = *(volatile float *)&sh.af;
+        // ---- dx += alpha p, r -= alpha q, z = M^-1 r; r.z and r.r per chunk
+#pragma unroll
+        for (int k = 0; k < K; k++)
+        {
+            const int ch = warp + k * kWarps, li = ch * 32 + lane;
+            if (ch < nch)
+            {
+                float pr = 0.f, prr = 0.f;
+                if (li < nrow)
+                {
+                    const float3 p = xyz(sp[own0 + li]);
+                    x[k] = make_float3(fmaf(af, p.x, x[k].x), fmaf(af, p.y, x[k].y),
+                                       fmaf(af, p.z, x[k].z));
+                    r[k] = make_float3(fmaf(-af, q[k].x, r[k].x), fmaf(-af, q[k].y, r[k].y),
+                                       fmaf(-af, q[k].z, r[k].z));
+                    const float M[6] = {m0[k].x, m0[k].y, m0[k].z, m0[k].w, m1[k].x, m1[k].y};
+                    z[k] = symv(M, r[k]);
+                    if constexpr (CLUSTER)
+                        push_row(sh, w.row0 + li, z[k]);
+                    else if (multi)
+                        st_row(d.z + w.row0 + li, z[k], tag + 1u);
+                    pr = fdot(r[k], z[k]);
+                    prr = fdot(r[k], r[k]);
+                }
+                pr = warp_sum(pr);
+                prr = warp_sum(prr);
+                chunk_add<2>(s_dig[1], lane < 8 ? pr : prr, s_scale[lane < 8 ? 1 : 2]);
+            }
+        }
+        bar_arrive(4, kAll);
+        // the halo rows of the new z, while the sums are under way
+        if (CLUSTER)
+        {
+            if (nhalo > 0 && !mbar_wait(bar_h, hphase, sc.limit))
+                sh.err = 1;
+            hphase ^= 1u;
+        }
+        else
+#pragma unroll
+            for (int u = 0; u < kAhead3; u++)
+            {
+                const int i = tid + u * kWorkers;
+                if (i < nhalo)
+                    hz[u] = poll_row(d.z + w.halo0 + (i < own0 ? i : i + nrow), tag + 1u,
+                                     sc.limit, &sh.err);
+            }
+        bar_sync(5, kAll);
+        if (CLUSTER && nhalo > 0 && tid == 0)
+            mbar_expect(bar_h, 16u * unsigned(nhalo));
+        bf = *(volatile float *)&sh.bf;
+    }
+#pragma unroll
+    for (int k = 0; k < K; k++)
+    {
+        const int li = (warp + k * kWarps) * 32 + lane, row = w.row0 + li;
+        if (li < nrow)
+        {
+            d.dx[row] = f4(x[k]);
+            d.r[row] = f4(r[k]);
+        }
+    }
+    if (CLUSTER)
+        cluster_sync();
+}
+
+template <int K> const void *half_kernel(bool skew, bool cluster)
+{
+    return cluster ? (skew ? (const void *)k_pcg_half<K, true, true>
+                           : (const void *)k_pcg_half<K, false, true>)
+                   : (skew ? (const void *)k_pcg_half<K, true, false>
+                           : (const void *)k_pcg_half<K, false, false>);
+}
+
+const void *team_kernel(int k, bool half, bool skew, bool cluster)
+{
+    if (half)
+        return k <= 2   ? half_kernel<2>(skew, cluster)
+               : k == 3 ? half_kernel<3>(skew, cluster)
+                        : half_kernel<4>(skew, cluster);
     if (cluster)
         return k <= 1 ? (skew ? (const void *)k_pcg_team<1, true, true>
                               : (const void *)k_pcg_team<1, false, true>)

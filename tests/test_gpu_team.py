@@ -23,16 +23,21 @@ def _conf(h, w, model):
 # one row short of, at and past a 32-row chunk; the most rows of one row per
 # thread in a single block (512) and the fewest of two; the largest single
 # block and the smallest team; a short last block; a set whose teams hold two
-# rows per thread; uneven teams in one launch
+# rows per thread; uneven teams in one launch; sets of cloths too large for the
+# whole matrix on chip: every stored block on chip, and a part of them (with
+# rows whose transposed blocks another block owns), two, three and four rows a
+# thread
 @pytest.mark.parametrize("model", ["quadratic", "dihedral"])
 @pytest.mark.parametrize("shapes", [[(2, 2)], [(3, 7)], [(4, 8)],
                                     [(3, 11)], [(16, 32)], [(19, 27)], [(20, 32)], [(21, 31)],
                                     [(65, 64)], [(128, 129)],
                                     [(150, 150), (149, 150), (150, 149), (140, 150)],
-                                    [(5, 5), (90, 31), (2, 40), (64, 64)]])
+                                    [(5, 5), (90, 31), (2, 40), (64, 64)], [(270, 300)],
+                                    [(300, 320), (5, 5)], [(400, 401)], [(470, 480)]])
 def test_team_kernel_matches_graph_loop(ctx, shapes, model):
     from acousticsim_gb300 import BaraffClothGpu, params
-    p = params(max_iters=4000, rel_tol=1e-6)
+    big = sum(h * w for h, w in shapes) > 60000  # a few iterations show it
+    p = params(max_iters=60 if big else 4000, rel_tol=1e-6)
     out = {}
     for solver in ("persistent", "graph_loop"):
         ctx.set_solver(solver)
@@ -45,7 +50,8 @@ def test_team_kernel_matches_graph_loop(ctx, shapes, model):
         iters = []
         for _ in range(2):  # the second step starts from the first one's dx
             st = ctx.batch_step(cloths, 0.0, p)
-            assert all(s["status"] == "OK" and s["solver"] == solver for s in st), st
+            assert all(s["status"] in (("OK", "MAXITER") if big else ("OK",)) and
+                       s["solver"] == solver for s in st), st
             iters.append([s["iters"] for s in st])
         out[solver] = iters, [c.GetPos() for c in cloths], [c.get_dx() for c in cloths]
         for c in cloths:
