@@ -896,7 +896,8 @@ TeamBlock team_block(const Tables &t, int inst, int rank, int r0, int r1)
     return w;
 }
 
-// An on-chip kernel: k_pcg_team or k_pcg_half (half) with K rows a thread.
+// An on-chip kernel: k_pcg_team or k_pcg_half (half) with K rows a thread (0:
+// one, without blocks in registers).
 struct TeamKernel
 {
     int K;
@@ -915,7 +916,7 @@ bool team_split(const Batch *b, int i, int blocks, TeamKernel tk, bool cluster, 
     const size_t first = work.size();
     const int rows =
         ((t.nv + blocks - 1) / blocks + kRedRows - 1) / kRedRows * kRedRows;
-    if (rows > tk.K * kTeamWorkers || (tk.half && h.width_up > 15))
+    if (rows > std::max(tk.K, 1) * kTeamWorkers || (tk.half && h.width_up > 15))
         return false;
     size_t most = 0;
     for (int r0 = 0; r0 < t.nv; r0 += rows)
@@ -1073,20 +1074,20 @@ int plan_persistent(cloth_ctx *ctx, Batch *b)
         // iteration, 16^2: 2.3, in a cluster of 16 2.8; 20^2: 2.7 and 2.7), above
         // it 16 blocks (32^2: 2.6, two blocks 2.9; 64^2: 2.9, the whole GPU 3.3;
         // 80^2: 3.3 and 3.3)
-        const TeamKernel one{1, false};
         const int C = most <= kTeamAloneRows ? 1 : kClusterMax;
+        const TeamKernel one{b->skew ? 0 : 1, false};
         if (plan_cluster(ctx, b, one, C, work, b->smem_persist, true))
         {
             use(one, C);
             return upload_work(b, work, sizeof(unsigned long long), sizeof(TeamBlock));
         }
         // Teams over the whole GPU: the whole matrix on chip where it fits (256^2:
-        // 4.7 us with one row a thread, 5.1 with two; 5.3 with the stored blocks
-        // alone), else the stored blocks (300^2: 6.9, the kernel that reads the
-        // matrix from L2 13.0; 512^2: 16.5 and 21.4), with as few rows a thread
-        // as hold the set (362^2: 8.2 with two, 8.6 with three)
-        for (TeamKernel k : {one, TeamKernel{2, false}, TeamKernel{2, true}, TeamKernel{3, true},
-                             TeamKernel{4, true}})
+        // 4.2 us with one row a thread), else the stored blocks (300^2: 6.8, the
+        // kernel that reads the matrix from L2 13.0; 512^2: 15.8 and 21.4), with
+        // as few rows a thread as hold the set (362^2: 7.8 with two, 8.6 with
+        // three)
+        for (TeamKernel k : {one, TeamKernel{1, false}, TeamKernel{2, false}, TeamKernel{2, true},
+                             TeamKernel{3, true}, TeamKernel{4, true}})
             if (plan_team(ctx, b, k, work, b->smem_persist))
             {
                 use(k, 0);

@@ -261,20 +261,27 @@ struct TeamSync
 {
     unsigned long long words[4][16];
 };
-// Slots of a row whose blocks k_pcg_team holds in registers (K rows a thread).
+// Slots of a row whose blocks k_pcg_team holds in registers: with k = 1 rows a
+// thread; none with 2, nor with k = 0, one row a thread as well (with skew parts,
+// whose kernel has fewer registers to spare, the faster one where it fits:
+// 128^2 3.8 us per iteration, 4.0 with four; without them eight are faster:
+// 64^2 2.7 us, 2.8 with none).
 __host__ __device__ constexpr int team_reg_slots(int k, bool skew_kernel)
 {
-    return k > 1 ? 0 : skew_kernel ? 4 : 8;
+    return k != 1 ? 0 : skew_kernel ? 4 : 8;
 }
-// Dynamic shared memory of a k_pcg_team block: p over its halo; blocks (skew
+// One slot of 32 rows in shared memory: blocks, offsets of p, skew parts.
+__host__ __device__ constexpr int team_slot_bytes(bool skew) { return 32 * (skew ? 44 : 28); }
+// Dynamic shared memory of a k_pcg_team block: p over its halo; the inverse
+// diagonal blocks; blocks (skew
 // parts) and local column indices of the rows' other slots; in a cluster, z
 // over the halo rows of other blocks.
 __host__ __device__ inline size_t team_smem_bytes(int halo, int rows, int width, bool skew,
                                                   int reg_slots, bool cluster)
 {
-    const size_t rp = size_t((rows + 31) / 32) * 32;
-    const size_t planes = width > reg_slots ? width - reg_slots : 0;
-    return (size_t(halo) + (cluster ? halo - rows : 0)) * 16 + planes * rp * (skew ? 42 : 26);
+    const size_t slots = width > reg_slots ? width - reg_slots : 0;
+    return (size_t(halo) + (cluster ? halo - rows : 0)) * 16 +
+           size_t((rows + 1) & ~1) * 24 + size_t((rows + 31) / 32) * slots * team_slot_bytes(skew);
 }
 // The same of a k_pcg_half block: planes of stored blocks, and 16-bit words of
 // `words` slots per row.

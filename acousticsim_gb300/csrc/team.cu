@@ -23,11 +23,14 @@
 // The arithmetic is that of the other PCG drivers, bit for bit.
 //
 // Measured (one GB300, us per PCG iteration over a whole step, before: the
-// kernel that reads the matrix from L2 and forms the scalars in FP64): 20x20
-// 11.8 -> 3.8, 64x64 12.2 -> 3.2, 97x61 11.8 -> 3.7, 193x255 12.4 -> 4.4,
-// 128x128 with dihedral bending 14.1 -> 4.9.
+// kernel that reads the matrix from L2 and forms the scalars in FP64): 16x16
+// 13.1 -> 2.2, 64x64 12.2 -> 2.6, 97x61 11.8 -> 3.3, 193x255 12.4 -> 4.0,
+// 256x256 12.7 -> 4.2, 512x512 21.5 -> 15.8, 128x128 with dihedral bending
+// 14.1 -> 3.8.
 #include "internal.h"
 #include "pcg_math.cuh"
+
+#include <type_traits>
 
 namespace cloth {
 
@@ -36,7 +39,7 @@ namespace {
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kWorkers = kTeamWorkers;
 constexpr int kWarps = kWorkers / 32;
-constexpr int kHaloAhead = 2; // halo rows per thread polled before beta is known
+constexpr int kHaloAhead = 3; // halo rows per thread polled before beta is known
 
 // ---- named barriers: 1 the workers, 2-6 workers with the control warp
 __device__ __forceinline__ void bar_sync(int id, int n)
@@ -171,31 +174,78 @@ __device__ __forceinline__ double value(const Raw &r)
     return fx_value((unsigned long long)r.hi << 16 | r.lo >> 32, r.lo & 0xffffffffull, r.s);
 }
 
-// Adds 32-row chunks' FP32 sums to the block's digits: lanes 8 q .. 8 q + 4 add
-// quantity q's (v and its scale s are theirs), dig[8 q .. 8 q + 3] being its
-// digits and dig[8 q + 4] the count of sums out of range.  NQ quantities.
-template <int NQ> __device__ __forceinline__ void chunk_add(int *dig, float v, int s)
+// Adds 32-row chunks' FP32 sums to the block's digits, one sum per group of 8
+// lanes (v, its scale s and its quantity's digits dig[0 .. 3] are theirs; dig[4]
+// counts sums out of range).
+__device__ __forceinline__ void chunk_add(int *dig, float v, int s, bool on)
 {
     const unsigned bits = __float_as_uint(v);
-    const int e = int((bits >> 23) & 0xffu), lane = threadIdx.x & 31, j = lane & 7;
-    unsigned m = e ? (bits & 0x7fffffu) | 0x800000u : 0u; // (subnormal: below any scale in use)
-    int sh = e - 150 + s;                                 // |v| = m 2^sh units
-    const bool bad = e == 255 || (e != 0 && sh >= 72);
-    if (sh < 0)
+    const int e = int((bits >> 23) & 0xffu), j = threadIdx.x & 7;
+    unsigned m = (bits & 0x7fffffu) | 0x800000u;
+    int sh = e - 150 + s; // |v| = m 2^sh units
+    bool bad = false;
+    if (__any_sync(kFull, unsigned(sh) >= 72u || unsigned(e - 1) >= 254u))
     {
-        m = sh > -25 ? (m + (1u << (-sh - 1))) >> -sh : 0u;
-        sh = 0;
+        // zero or subnormal (below any scale in use), Inf / NaN, out of range,
+        // or digits below the unit
+        if (e == 0)
+            m = 0u;
+        bad = e == 255 || (e != 0 && sh >= 72);
+        if (sh < 0)
+        {
+            m = sh > -25 ? (m + (1u << (-sh - 1))) >> -sh : 0u;
+            sh = 0;
+        }
+        sh = min(sh, 71);
     }
     const int k = (sh * 43) >> 10, off = sh - 24 * k; // sh / 24, sh % 24
-    int x = j == k ? int((m << off) & 0xffffffu) : j == k + 1 ? int(m >> (24 - off)) : 0;
-    if (bits & 0x80000000u)
-        x = -x;
+    int x = j == k ? int((m << off) & 0xffffffu) : int(m >> (24 - off));
+    const int sign = int(bits) >> 31;
+    x = (x ^ sign) - sign;
+    bool add = on && unsigned(j - k) < 2u;
     if (bad)
-        x = j == 4 ? 1 : 0;
-    else if (j > 3)
-        x = 0;
-    if (x != 0 && lane < 8 * NQ)
-        atomicAdd(dig + lane, x);
+    {
+        x = 1;
+        add = on && j == 4;
+    }
+    if (add)
+        atomicAdd(dig + j, x);
+}
+// The sums of a warp's K chunks (the same in every lane; zero where it has
+// none): p.q.
+template <int K>
+__device__ __forceinline__ void chunks_add(int (*dig)[8], const int *scale, const float (&pq)[K])
+{
+    const int g = (threadIdx.x & 31) >> 3;
+    float v = pq[0];
+#pragma unroll
+    for (int k = 1; k < K; k++)
+        v = g == k ? pq[k] : v;
+    chunk_add(dig[0], v, scale[0], g < K);
+}
+// Both r.z and r.r of a warp's K chunks: the first half-warp holds the first
+// one's sums, the second the other's (warp_sum2).
+template <int K>
+__device__ __forceinline__ void chunks_add2(int (*dig)[8], const int *scale, const float (&v2)[K])
+{
+    const int g = (threadIdx.x & 31) >> 3, q = 1 + (g >> 1);
+    const int s = scale[q];
+    // two chunks at a time, one per group of a half-warp
+#pragma unroll
+    for (int k = 0; k < K; k += 2)
+        chunk_add(dig[q], (g & 1) && k + 1 < K ? v2[k + 1 < K ? k + 1 : k] : v2[k], s,
+                  !(g & 1) || k + 1 < K);
+}
+// warp_sum of a in the first half-warp and of b in the second: the same pairs
+// are added at every step, so the sums are warp_sum's bit for bit.
+__device__ __forceinline__ float warp_sum2(float a, float b)
+{
+    const bool hi = threadIdx.x & 16;
+    float v = (hi ? b : a) + __shfl_xor_sync(kFull, hi ? a : b, 16);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1)
+        v += __shfl_xor_sync(kFull, v, o);
+    return v;
 }
 
 // V from its digits; true when it is out of the 96-bit range.
@@ -303,6 +353,18 @@ __device__ __forceinline__ Top48 top48(const Raw &v)
 {
     Top48 r;
     unsigned long long hi = (unsigned long long)v.hi, lo = v.lo;
+    // the usual range (a sum's last value has 2^70 units): 32-bit shifts
+    if (unsigned(hi >> 32) == 0u && unsigned(hi) != 0u)
+    {
+        const unsigned h = unsigned(hi), m = unsigned(lo >> 16), l = unsigned(lo) << 16;
+        const int c = __clz(int(h));
+        const unsigned w0 = __funnelshift_l(m, h, c), w1 = __funnelshift_l(l, m, c);
+        r.neg = false;
+        r.hi = w0 >> 8;
+        r.lo = (w0 & 0xffu) << 16 | w1 >> 16;
+        r.e = 48 + 32 - c - 24 - v.s;
+        return r;
+    }
     r.neg = v.hi < 0;
     if (r.neg)
     {
@@ -345,11 +407,19 @@ __device__ __forceinline__ int scale_of(const Raw &v, const Top48 &t)
 // within 2^-38 of a midpoint: one time in ~10,000), or the result is not in
 // the normal range, *ok = false and the caller divides in FP64.  rb: about
 // 1 / b.hi.
-__device__ __forceinline__ float recip(const Top48 &b) { return __fdividef(1.f, float(b.hi)); }
+// (hi as a float by its bits; lo to 23 of them)
+__device__ __forceinline__ float hi_f(const Top48 &t)
+{
+    return __uint_as_float(0x4b000000u | (t.hi & 0x7fffffu));
+}
+__device__ __forceinline__ float lo_f(const Top48 &t)
+{
+    return (__uint_as_float(0x4b000000u | t.lo >> 1) - 0x1p23f) * 0x1p-23f;
+}
+__device__ __forceinline__ float recip(const Top48 &b) { return __fdividef(1.f, hi_f(b)); }
 __device__ __forceinline__ float ratio(const Top48 &a, const Top48 &b, float rb, bool *ok)
 {
-    const float ah = float(a.hi), al = float(a.lo) * 0x1p-24f;
-    const float bh = float(b.hi), bl = float(b.lo) * 0x1p-24f;
+    const float ah = hi_f(a), al = lo_f(a), bh = hi_f(b), bl = lo_f(b);
     const float q1 = ah * rb;
     const float rem = fmaf(-q1, bl, fmaf(-q1, bh, ah) + al);
     const float q2 = rem * rb;
@@ -732,19 +802,19 @@ __device__ __forceinline__ float3 pick(bool on, float3 a, float3 b)
 // K: chunks of 32 rows per warp (a block owns at most K * kTeamWorkers rows).
 // SKEW: the launch set holds a dihedral-bending instance; skew block parts
 // are kept and applied where an instance has them.
-// Of each row the first kRegSlots blocks are in registers where a thread has
-// one row, the others in shared memory: its bandwidth (11 wavefronts per slot
-// and warp, 5 of them for p and the column) bounds the SpMV of a full block.
+// The first RW blocks of a row are in registers (where a thread has one row),
+// the others in shared memory: its bandwidth (11 wavefronts per slot and warp,
+// 5 of them for p and the column) bounds the SpMV of a full block.
 // CLUSTER: every team is one thread-block cluster (the launch's cluster size,
 // idle blocks included) and exchanges sums and z rows through its blocks'
 // shared memory: ~400 cycles a sum instead of ~1,500.  Teams are independent,
 // so a launch may have more of them than fit on the GPU at once.
-template <int K, bool SKEW, bool CLUSTER>
+template <int K, int RW, bool SKEW, bool CLUSTER>
 __global__ void __launch_bounds__(kTeamThreads, 1)
     k_pcg_team(InstDesc *const *descs, const TeamBlock *work, TeamSync *sync, SpinCfg sc)
 {
     constexpr int kAll = kTeamThreads;
-    constexpr int RW = team_reg_slots(K, SKEW);
+    constexpr int RC = RW > 0 ? 5 : 0; // slots past the RW whose offsets of p are in registers
     extern __shared__ float4 sm_dyn[];
     __shared__ InstDesc d;
     __shared__ int s_dig[3][8];  // digits of the block's sums: p.q, r.z, r.r
@@ -755,7 +825,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
         return;
     InstState *st = d.st;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nrow = w.row1 - w.row0, nch = (nrow + 31) >> 5, rp = nch << 5;
+    const int nrow = w.row1 - w.row0, nch = (nrow + 31) >> 5;
     const int nh = w.halo1 - w.halo0, W = max(d.width - RW, 0); // slots in shared memory
     const bool skew = SKEW && d.Aw;
     // the test hook's extra arrivals make a team of one wait too
@@ -766,10 +836,14 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
     const int nhalo = nh - nrow;
     float4 *sp = sm_dyn;
     float4 *sz = sp + nh;
-    float4 *sA0 = CLUSTER ? sz + nhalo : sz;
-    float4 *sAw = sA0 + size_t(W) * rp;
-    float2 *sA1 = reinterpret_cast<float2 *>(skew ? sAw + size_t(W) * rp : sAw);
-    unsigned short *scol = reinterpret_cast<unsigned short *>(sA1 + size_t(W) * rp);
+    // chunk by chunk and slot by slot a record of 32 rows: blocks (16 and 8
+    // bytes), byte offsets of p (and skew parts), so that a walk over the slots
+    // has constant strides
+    constexpr int kRec = team_slot_bytes(false);
+    const int rec = team_slot_bytes(skew);
+    float4 *sM0 = CLUSTER ? sz + nhalo : sz; // inverse diagonal blocks
+    float2 *sM1 = reinterpret_cast<float2 *>(sM0 + nrow);
+    char *sA = reinterpret_cast<char *>(sM1 + ((nrow + 1) & ~1));
 
     if (warp == kWarps)
     {
@@ -785,7 +859,6 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
             find_peers(work, w, sh, [](int halo) { return smem_u32(sm_dyn) + 16u * unsigned(halo); });
     unsigned hphase = 0;
     float3 x[K], r[K], z[K], p[K];
-    float M[K][6];
     int len[K];
     float bf = float(__ldcg(&st->beta));
     {
@@ -802,7 +875,8 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
                 x[k] = xyz(d.dx[row]);
                 r[k] = xyz(d.r[row]);
                 z[k] = xyz(d.z[row]);
-                load_sym(d.M0, d.M1, row, M[k]);
+                sM0[li] = d.M0[row];
+                sM1[li] = d.M1[row];
                 if (it0 > 0)
                     p[k] = xyz(__ldcg(pold + row));
             }
@@ -828,7 +902,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
         return d.colu[oa] - w.halo0;
     };
     float rA[RW + 1][6], rw[RW + 1][3];
-    unsigned rc[RW + 1];
+    unsigned rc[RW + RC + 1];
     if (RW > 0)
     {
         const int li = warp * 32 + lane, row = w.row0 + li;
@@ -836,7 +910,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
 #pragma unroll
         for (int s = 0; s < RW; s++)
         {
-            rc[s] = 0u;
+            rc[s] = li < nrow ? unsigned(own0 + li) * 16u : 0u;
 #pragma unroll
             for (int i = 0; i < 6; i++)
                 rA[s][i] = 0.f;
@@ -855,6 +929,14 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
                 }
             }
         }
+#pragma unroll
+        for (int s = RW; s < RW + RC; s++)
+        {
+            uint32_t oa;
+            rc[s] = li < nrow ? unsigned(own0 + li) * 16u : 0u;
+            if (s < (info & 255))
+                rc[s] = unsigned(block_of(s, row, info, oa)) * 16u;
+        }
     }
     const int ds0 = RW > 0 && warp * 32 + lane < nrow
                         ? (d.rowinfo[w.row0 + warp * 32 + lane] >> 8) & 255
@@ -863,25 +945,31 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
 #pragma unroll 2
         for (int u = warp; u < W * nch; u += kWarps)
         {
-            const int s = u / nch, li = (u - s * nch) * 32 + lane, row = w.row0 + li;
+            const int c = u / W, s = u - c * W, li = c * 32 + lane, row = w.row0 + li;
             const int info = li < nrow ? d.rowinfo[row] : 0, slot = s + RW;
-            const size_t o = size_t(s) * rp + li;
-            if (slot >= (info & 255))
+            char *at = sA + size_t(u) * rec;
+            float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f), aw = a0;
+            float2 a1 = make_float2(0.f, 0.f);
+            // past a row's last slot: a zero block at the row's own column
+            int col = li < nrow ? own0 + li : 0;
+            if (slot < (info & 255))
             {
-                scol[o] = 0; // read where another row of the warp has the slot
-                continue;
+                uint32_t oa;
+                col = block_of(slot, row, info, oa);
+                a0 = d.A0[oa];
+                a1 = d.A1[oa];
+                if (SKEW && skew)
+                {
+                    aw = d.Aw[oa];
+                    // the transposed block's skew part changes sign
+                    aw.w = slot < ((info >> 8) & 255) ? -1.f : 1.f;
+                }
             }
-            uint32_t oa;
-            const int c = block_of(slot, row, info, oa);
-            sA0[o] = d.A0[oa];
-            sA1[o] = d.A1[oa];
+            reinterpret_cast<float4 *>(at)[lane] = a0;
+            reinterpret_cast<float2 *>(at + 512)[lane] = a1;
+            reinterpret_cast<unsigned *>(at + 768)[lane] = unsigned(col) * 16u;
             if (SKEW && skew)
-            {
-                float4 aw = d.Aw[oa];
-                aw.w = slot < ((info >> 8) & 255) ? -1.f : 1.f; // the transposed block's skew part changes sign
-                sAw[o] = aw;
-            }
-            scol[o] = (unsigned short)c;
+                reinterpret_cast<float4 *>(at + kRec)[lane] = aw;
         }
     }
     // halo rows of z of the first iteration (written before this launch)
@@ -910,7 +998,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
             if (CLUSTER)
                 zz = xyz(sz[i]);
             else if (u < kHaloAhead)
-                zz = u == 0 ? hz[0] : hz[1];
+                zz = u == 0 ? hz[0] : u == 1 ? hz[1] : hz[2];
             else if (tag == unsigned(it0))
                 zz = xyz(__ldcg(d.z + w.halo0 + j));
             else
@@ -930,75 +1018,93 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
         bar_sync(1, kWorkers);
         // ---- q = A p; p.q per 32-row chunk
         float3 q[K];
+        float part[K];
 #pragma unroll
         for (int k = 0; k < K; k++)
         {
             const int ch = warp + k * kWarps, li = ch * 32 + lane;
             q[k] = make_float3(0.f, 0.f, 0.f);
+            part[k] = 0.f;
             if (ch < nch)
             {
-                const float4 *a0 = sA0 + li;
-                const float2 *a1 = sA1 + li;
-                const unsigned short *cc = scol + li;
-                // kAhead slots at a time, loads first and products selected, not
-                // branched around (a branch per slot made the walk three times
-                // as long); a row's planes past its last slot hold column 0
-                constexpr int kAhead = 4;
-                const int n = len[k];
+                // kAhead slots at a time, loads first; past a row's last slot
+                // the blocks are zero (a branch per slot made the walk three
+                // times as long)
+                constexpr int kAhead = K > 1 || SKEW ? 4 : 8;
+                auto p_at = [&](unsigned off) {
+                    return *reinterpret_cast<const float4 *>(reinterpret_cast<const char *>(sp) +
+                                                             off);
+                };
 #pragma unroll
                 for (int s0 = 0; s0 < RW; s0 += kAhead)
                 {
                     float4 pc[kAhead];
 #pragma unroll
                     for (int i = 0; i < kAhead; i++)
-                        pc[i] = *reinterpret_cast<const float4 *>(
-                            reinterpret_cast<const char *>(sp) + rc[s0 + i]);
+                        if (s0 + i < RW)
+                            pc[i] = p_at(rc[s0 + i]);
 #pragma unroll
                     for (int i = 0; i < kAhead; i++)
                     {
                         const int s = s0 + i;
-                        float3 t = q[k] + symv(rA[s], xyz(pc[i]));
+                        if (s >= RW)
+                            continue;
+                        q[k] = q[k] + symv(rA[s], xyz(pc[i]));
                         if (SKEW && skew)
                         {
                             const float3 cw = skewv(
                                 make_float4(rw[s][0], rw[s][1], rw[s][2], 0.f), xyz(pc[i]));
-                            t = s < ds0 ? t - cw : t + cw;
+                            q[k] = s < ds0 ? q[k] - cw : q[k] + cw;
                         }
-                        q[k] = pick(s < n, t, q[k]);
                     }
                 }
-                const int top = __reduce_max_sync(kFull, n - RW);
-                for (int s0 = 0; s0 < top; s0 += kAhead)
-                {
-                    float4 u[kAhead];
-                    float2 v[kAhead];
-                    float4 pc[kAhead];
-                    int o[kAhead];
+                // N slots of this lane's row from at on; their offsets of p in
+                // registers where the first of them is rc's
+                auto walk = [&](const char *at, auto count, auto known) {
+                    constexpr int N = decltype(count)::value, C = decltype(known)::value;
+                    float4 u[N], pc[N];
+                    float2 v[N];
 #pragma unroll
-                    for (int i = 0; i < kAhead; i++)
+                    for (int i = 0; i < N; i++)
                     {
-                        o[i] = min(s0 + i, top - 1) * rp;
-                        pc[i] = sp[cc[o[i]]];
-                        u[i] = a0[o[i]];
-                        v[i] = a1[o[i]];
+                        const char *a = at + i * (SKEW ? rec : kRec);
+                        pc[i] = p_at(C >= 0 ? rc[C >= 0 ? C + i : 0]
+                                            : reinterpret_cast<const unsigned *>(a + 768)[lane]);
+                        u[i] = reinterpret_cast<const float4 *>(a)[lane];
+                        v[i] = reinterpret_cast<const float2 *>(a + 512)[lane];
                     }
 #pragma unroll
-                    for (int i = 0; i < kAhead; i++)
+                    for (int i = 0; i < N; i++)
                     {
                         const float A[6] = {u[i].x, u[i].y, u[i].z, u[i].w, v[i].x, v[i].y};
-                        float3 t = q[k] + symv(A, xyz(pc[i]));
+                        q[k] = q[k] + symv(A, xyz(pc[i]));
                         if (SKEW && skew)
                         {
-                            const float4 aw = sAw[o[i] + li];
+                            const float4 aw =
+                                reinterpret_cast<const float4 *>(at + i * rec + kRec)[lane];
                             const float3 cw = skewv(aw, xyz(pc[i]));
-                            t = aw.w < 0.f ? t - cw : t + cw;
+                            q[k] = aw.w < 0.f ? q[k] - cw : q[k] + cw;
                         }
-                        q[k] = pick(s0 + i < n - RW, t, q[k]);
                     }
+                };
+                const int top = __reduce_max_sync(kFull, len[k] - RW);
+                const char *at = sA + ch * W * rec;
+                using std::integral_constant;
+                int s0 = 0;
+                if (RC > 0 && top >= RC)
+                {
+                    walk(at, integral_constant<int, RC ? RC : 1>(), integral_constant<int, RW>());
+                    s0 = RC;
+                    at += RC * rec;
                 }
-                chunk_add<1>(s_dig[0], warp_sum(li < nrow ? fdot(p[k], q[k]) : 0.f), s_scale[0]);
+                for (; s0 + kAhead <= top; s0 += kAhead, at += kAhead * rec)
+                    walk(at, integral_constant<int, kAhead>(), integral_constant<int, -1>());
+                for (; s0 < top; s0++, at += rec)
+                    walk(at, integral_constant<int, 1>(), integral_constant<int, -1>());
+                part[k] = warp_sum(li < nrow ? fdot(p[k], q[k]) : 0.f);
             }
         }
+        chunks_add<K>(s_dig, s_scale, part);
         bar_arrive(2, kAll);
         // the sum words of iteration it + 2 were last polled in iteration
         // it - 2, which every block of the team has left (its r.z words of
@@ -1010,25 +1116,35 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
                 sync[blockIdx.x].words[(tag + 2u) & 3u][lane] = 0ull;
             __threadfence();
         }
+        float4 m0[K]; // (in flight while alpha is awaited)
+        float2 m1[K];
+#pragma unroll
+        for (int k = 0; k < K; k++)
+        {
+            const int li = min((warp + k * kWarps) * 32 + lane, nrow - 1);
+            m0[k] = sM0[li];
+            m1[k] = sM1[li];
+        }
         bar_sync(3, kAll);
         if (*(volatile int *)&sh.stop)
             break;
         const float af = *(volatile float *)&sh.af;
-        // ---- dx += alpha p, r -= alpha q, z = M^-1 r; r.z and r.r per chunk
+        // ---- r -= alpha q, z = M^-1 r; r.z and r.r per chunk (dx += alpha p
+        // once they are on their way)
 #pragma unroll
         for (int k = 0; k < K; k++)
         {
             const int ch = warp + k * kWarps, li = ch * 32 + lane;
+            part[k] = 0.f;
             if (ch < nch)
             {
                 float pr = 0.f, prr = 0.f;
                 if (li < nrow)
                 {
-                    x[k] = make_float3(fmaf(af, p[k].x, x[k].x), fmaf(af, p[k].y, x[k].y),
-                                       fmaf(af, p[k].z, x[k].z));
                     r[k] = make_float3(fmaf(-af, q[k].x, r[k].x), fmaf(-af, q[k].y, r[k].y),
                                        fmaf(-af, q[k].z, r[k].z));
-                    z[k] = symv(M[k], r[k]);
+                    const float M[6] = {m0[k].x, m0[k].y, m0[k].z, m0[k].w, m1[k].x, m1[k].y};
+                    z[k] = symv(M, r[k]);
                     if (!CLUSTER && multi)
                         st_row(d.z + w.row0 + li, z[k], tag + 1u);
                     if constexpr (CLUSTER)
@@ -1036,12 +1152,15 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
                     pr = fdot(r[k], z[k]);
                     prr = fdot(r[k], r[k]);
                 }
-                pr = warp_sum(pr);
-                prr = warp_sum(prr);
-                chunk_add<2>(s_dig[1], lane < 8 ? pr : prr, s_scale[lane < 8 ? 1 : 2]);
+                part[k] = warp_sum2(pr, prr);
             }
         }
+        chunks_add2<K>(s_dig, s_scale, part);
         bar_arrive(4, kAll);
+#pragma unroll
+        for (int k = 0; k < K; k++)
+            x[k] = make_float3(fmaf(af, p[k].x, x[k].x), fmaf(af, p[k].y, x[k].y),
+                               fmaf(af, p[k].z, x[k].z));
         // the halo rows of the new z, while the sums are under way
 #pragma unroll
         for (int u = 0; u < (CLUSTER ? 0 : kHaloAhead); u++)
@@ -1089,7 +1208,6 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
     k_pcg_half(InstDesc *const *descs, const TeamBlock *work, TeamSync *sync, SpinCfg sc)
 {
     constexpr int kAll = kTeamThreads;
-    constexpr int kAhead3 = 3; // halo rows per thread polled before beta is known
     extern __shared__ float4 sm_dyn[];
     __shared__ InstDesc d;
     __shared__ int s_dig[3][8];
@@ -1109,11 +1227,14 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
     const int wl = d.width_lo, wu = d.width_up;
     float4 *sp = sm_dyn;
     float4 *sz = sp + nh;
-    float4 *sU0 = CLUSTER ? sz + nhalo : sz;
-    float4 *sUw = sU0 + size_t(u1 - u0) * rp;
-    float2 *sU1 = reinterpret_cast<float2 *>(skew ? sUw + size_t(u1 - u0) * rp : sUw);
-    // words of the lower slots (column | plane << 12), then of the upper planes
-    unsigned short *scol = reinterpret_cast<unsigned short *>(sU1 + size_t(u1 - u0) * rp);
+    // plane by plane the rows' stored blocks (24 bytes; with skew parts 40):
+    // read 8 bytes at a time, conflict-free at any row
+    const int kb = SKEW && skew ? 40 : 24;
+    char *sU = reinterpret_cast<char *>(CLUSTER ? sz + nhalo : sz);
+    // chunk by chunk and slot by slot 32 words: the lower slots' (column | plane
+    // << 12), then the upper planes' columns
+    unsigned short *scol =
+        reinterpret_cast<unsigned short *>(sU + size_t(u1 - u0) * rp * kb);
     if (warp == kWarps)
     {
         control_warp<CLUSTER>(d, w, sync, sc, it0, multi, sh, s_dig, s_scale);
@@ -1145,45 +1266,80 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
     if (it0 > 0) // a solve handed over in its middle
         for (int i = tid; i < nh; i += kWorkers)
             sp[i] = __ldcg(pold + w.halo0 + i);
-#pragma unroll 4
+    unsigned far = 0u; // chunks of this warp with a lower slot whose block is not on chip
+#pragma unroll 2
     for (int u = warp; u < (wl + wu) * nch; u += kWarps)
     {
-        const int s = u / nch, li = (u - s * nch) * 32 + lane, row = w.row0 + li;
+        const int c = u / (wl + wu), s = u - c * (wl + wu), li = c * 32 + lane,
+                  row = w.row0 + li;
         const int inf = li < nrow ? d.rowinfo[row] : 0, ds = (inf >> 8) & 255;
-        const bool upper = s >= wl;
         const int uu = s - wl; // upper plane
-        unsigned short word = 0;
-        if (upper ? uu < (inf & 255) - ds : s < ds)
+        // past a row's last slot: its own column and a block on chip (not used),
+        // or a zero block
+        unsigned word = unsigned(own0 + min(li, nrow - 1)) | (s < wl ? unsigned(u0) << 12 : 0u);
+        if (s < wl)
         {
-            if (upper)
-            {
-                const uint32_t oa = up_idx(uu, row, wu);
-                word = (unsigned short)(d.colu[oa] - w.halo0);
-                if (uu >= u0 && uu < u1)
-                {
-                    const size_t o = size_t(uu - u0) * rp + li;
-                    sU0[o] = d.A0[oa];
-                    sU1[o] = d.A1[oa];
-                    if (SKEW && skew)
-                        sUw[o] = d.Aw[oa];
-                }
-            }
-            else
+            if (s < ds)
             {
                 const uint32_t ref = d.lref[lo_idx(s, row, wl)];
-                word = (unsigned short)((lref_col(ref) - w.halo0) | int(ref >> 24) << 12);
+                word = unsigned(lref_col(ref) - w.halo0) | (ref >> 24) << 12;
             }
         }
-        scol[size_t(s) * rp + li] = word;
+        else
+        {
+            float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f), aw = a0;
+            float2 a1 = make_float2(0.f, 0.f);
+            const bool here = uu >= u0 && uu < u1;
+            if (uu < (inf & 255) - ds)
+            {
+                const uint32_t oa = up_idx(uu, row, wu);
+                word = unsigned(d.colu[oa] - w.halo0);
+                if (here)
+                {
+                    a0 = d.A0[oa];
+                    a1 = d.A1[oa];
+                    if (SKEW && skew)
+                        aw = d.Aw[oa];
+                }
+            }
+            if (here)
+            {
+                float2 *o = reinterpret_cast<float2 *>(sU + (size_t(uu - u0) * rp + li) * kb);
+                o[0] = make_float2(a0.x, a0.y);
+                o[1] = make_float2(a0.z, a0.w);
+                o[2] = a1;
+                if (SKEW && skew)
+                {
+                    o[3] = make_float2(aw.x, aw.y);
+                    o[4] = make_float2(aw.z, 0.f);
+                }
+            }
+        }
+        scol[size_t(u) * 32 + lane] = (unsigned short)word;
+    }
+    bar_sync(1, kWorkers);
+#pragma unroll
+    for (int k = 0; k < K; k++)
+    {
+        const int ch = warp + k * kWarps;
+        bool any = false;
+        if (ch < nch)
+            for (int s = 0; s < ((info[k] >> 8) & 255); s++)
+            {
+                const unsigned wd = scol[(size_t(ch) * (wl + wu) + s) * 32 + lane];
+                any |= unsigned(int(wd & 4095u) - own0) >= unsigned(nrow) ||
+                       (wd >> 12) - unsigned(u0) >= unsigned(u1 - u0);
+            }
+        far |= __any_sync(kFull, any) ? 1u << k : 0u;
     }
     // halo rows of z of the first iteration (written before this launch)
-    float3 hz[kAhead3];
+    float3 hz[kHaloAhead];
     if (CLUSTER)
         for (int i = tid; i < nhalo; i += kWorkers)
             sz[i] = __ldcg(d.z + w.halo0 + (i < own0 ? i : i + nrow));
     else
 #pragma unroll
-        for (int u = 0; u < kAhead3; u++)
+        for (int u = 0; u < kHaloAhead; u++)
         {
             const int i = tid + u * kWorkers;
             hz[u] = make_float3(0.f, 0.f, 0.f);
@@ -1202,7 +1358,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
             float3 zz;
             if (CLUSTER)
                 zz = xyz(sz[i]);
-            else if (u < kAhead3)
+            else if (u < kHaloAhead)
                 zz = u == 0 ? hz[0] : u == 1 ? hz[1] : hz[2];
             else if (tag == unsigned(it0))
                 zz = xyz(__ldcg(d.z + w.halo0 + j));
@@ -1220,131 +1376,147 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
         bar_sync(1, kWorkers);
         // ---- q = A p; p.q per 32-row chunk
         float3 q[K];
+        float part[K];
 #pragma unroll
         for (int k = 0; k < K; k++)
         {
             const int ch = warp + k * kWarps, li = ch * 32 + lane, row = w.row0 + li;
             q[k] = make_float3(0.f, 0.f, 0.f);
-            if (ch < nch)
+            part[k] = 0.f;
+            if (ch >= nch)
+                continue;
+            const int ds = (info[k] >> 8) & 255, ne = (info[k] & 255) - ds;
+            const int top_l = __reduce_max_sync(kFull, ds), top_u = __reduce_max_sync(kFull, ne);
+            struct Block
             {
-                const int ds = (info[k] >> 8) & 255, ne = (info[k] & 255) - ds;
-                const int top_l = __reduce_max_sync(kFull, ds),
-                          top_u = __reduce_max_sync(kFull, ne);
-                const unsigned short *cc = scol + li;
-                auto add = [&](bool on, float4 a0, float2 a1, float4 aw, float3 pc, bool lower) {
-                    const float A[6] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y};
-                    float3 t = q[k] + symv(A, pc);
-                    if (SKEW && skew)
-                    {
-                        const float3 cw = skewv(aw, pc);
-                        t = lower ? t - cw : t + cw;
-                    }
-                    q[k] = pick(on, t, q[k]);
-                };
-                const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
-                // upper planes that are not on chip: the first three in flight
-                // from here
-                constexpr int kPre = 3;
-                float4 f0[kPre], fw[kPre];
-                float2 f1[kPre];
-#pragma unroll
-                for (int i = 0; i < kPre; i++)
+                float A[6];
+                float4 w;
+            };
+            auto add = [&](const Block &b, float4 pc, bool lower, bool on) {
+                float3 t = q[k] + symv(b.A, xyz(pc));
+                if (SKEW && skew)
                 {
-                    const int u = i == 0 ? 0 : u1 + i - 1;
-                    f0[i] = fw[i] = zero4;
-                    f1[i] = make_float2(0.f, 0.f);
-                    if ((i > 0 || u0 > 0) && u < ne)
-                    {
-                        const uint32_t oa = up_idx(u, row, wu);
-                        f0[i] = __ldg(d.A0 + oa);
-                        f1[i] = __ldg(d.A1 + oa);
-                        if (SKEW && skew)
-                            fw[i] = __ldg(d.Aw + oa);
-                    }
+                    const float3 cw = skewv(b.w, xyz(pc));
+                    t = lower ? t - cw : t + cw;
                 }
-                // lower slots, kLow at a time, their blocks first
-                constexpr int kLow = 3;
+                q[k] = pick(on, t, q[k]);
+            };
+            auto on_chip = [&](const char *at) {
+                const float2 *o = reinterpret_cast<const float2 *>(at);
+                const float2 e0 = o[0], e1 = o[1], e2 = o[2];
+                Block b{{e0.x, e0.y, e1.x, e1.y, e2.x, e2.y}, {0.f, 0.f, 0.f, 0.f}};
+                if (SKEW && skew)
+                {
+                    const float2 e3 = o[3], e4 = o[4];
+                    b.w = make_float4(e3.x, e3.y, e4.x, 0.f);
+                }
+                return b;
+            };
+            auto from_l2 = [&](bool on, int u, int r) {
+                Block b{{0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+                if (on)
+                {
+                    const uint32_t oa = up_idx(u, r, wu);
+                    const float4 a0 = __ldg(d.A0 + oa);
+                    const float2 a1 = __ldg(d.A1 + oa);
+                    b.A[0] = a0.x;
+                    b.A[1] = a0.y;
+                    b.A[2] = a0.z;
+                    b.A[3] = a0.w;
+                    b.A[4] = a1.x;
+                    b.A[5] = a1.y;
+                    if (SKEW && skew)
+                        b.w = __ldg(d.Aw + oa);
+                }
+                return b;
+            };
+            // upper planes that are not on chip: the first three in flight from here
+            Block f[3];
+#pragma unroll
+            for (int i = 0; i < 3; i++)
+            {
+                const int u = i == 0 ? 0 : u1 + i - 1;
+                f[i] = from_l2((i > 0 || u0 > 0) && u < ne, u, row);
+            }
+            // lower slots, kLow at a time, loads first
+            const unsigned short *cc = scol + size_t(ch) * (wl + wu) * 32 + lane;
+            constexpr int kLow = 3;
+            const char *sUl = sU - (own0 + u0 * rp) * kb; // block of row own0 + r, plane u
+            if (!(far >> k & 1u))
                 for (int s0 = 0; s0 < top_l; s0 += kLow)
                 {
-                    float4 a0[kLow], aw[kLow], pc[kLow];
-                    float2 a1[kLow];
+                    Block b[kLow];
+                    float4 pc[kLow];
 #pragma unroll
                     for (int i = 0; i < kLow; i++)
                     {
-                        const unsigned wd = cc[min(s0 + i, top_l - 1) * rp];
-                        const int c = int(wd & 4095u), u = int(wd >> 12), lr = c - own0;
-                        a0[i] = aw[i] = zero4;
-                        a1[i] = make_float2(0.f, 0.f);
+                        const unsigned wd = cc[min(s0 + i, top_l - 1) * 32];
+                        pc[i] = sp[wd & 4095u];
+                        b[i] = on_chip(sUl + int((wd >> 12) * unsigned(rp) + (wd & 4095u)) * kb);
+                    }
+#pragma unroll
+                    for (int i = 0; i < kLow; i++)
+                        add(b[i], pc[i], true, s0 + i < ds);
+                }
+            else
+                for (int s0 = 0; s0 < top_l; s0 += kLow)
+                {
+                    Block b[kLow];
+                    float4 pc[kLow];
+#pragma unroll
+                    for (int i = 0; i < kLow; i++)
+                    {
+                        const unsigned wd = cc[min(s0 + i, top_l - 1) * 32];
+                        const int c = int(wd & 4095u), u = int(wd >> 12);
                         pc[i] = sp[c];
-                        if (unsigned(lr) < unsigned(nrow) && unsigned(u - u0) < unsigned(u1 - u0))
-                        {
-                            const int o = (u - u0) * rp + lr;
-                            a0[i] = sU0[o];
-                            a1[i] = sU1[o];
-                            if (SKEW && skew)
-                                aw[i] = sUw[o];
-                        }
-                        else if (s0 + i < ds)
-                        {
-                            const uint32_t oa = up_idx(u, c + w.halo0, wu);
-                            a0[i] = __ldg(d.A0 + oa);
-                            a1[i] = __ldg(d.A1 + oa);
-                            if (SKEW && skew)
-                                aw[i] = __ldg(d.Aw + oa);
-                        }
+                        if (unsigned(c - own0) < unsigned(nrow) &&
+                            unsigned(u - u0) < unsigned(u1 - u0))
+                            b[i] = on_chip(sUl + (u * rp + c) * kb);
+                        else
+                            b[i] = from_l2(s0 + i < ds, u, c + w.halo0);
                     }
 #pragma unroll
                     for (int i = 0; i < kLow; i++)
-                        add(s0 + i < ds, a0[i], a1[i], aw[i], xyz(pc[i]), true);
+                        add(b[i], pc[i], true, s0 + i < ds);
                 }
-                // upper slots in order
-                const unsigned short *cu = cc + wl * rp;
-                if (u0 > 0)
-                    add(ne > 0, f0[0], f1[0], fw[0], xyz(sp[cu[0]]), false);
-                const int top_r = min(top_u, u1);
-                constexpr int kUp = 3;
-                for (int b = u0; b < top_r; b += kUp)
+            // upper slots in order (past a row's last one the blocks are zero)
+            const unsigned short *cu = cc + wl * 32;
+            if (u0 > 0)
+                add(f[0], sp[cu[0]], false, true);
+            const int top_r = min(top_u, u1);
+            const char *at = sU + li * kb;
+            const unsigned short *cr = cu + u0 * 32;
+            auto walk = [&](auto count) {
+                constexpr int N = decltype(count)::value;
+                Block b[N];
+                float4 pc[N];
+#pragma unroll
+                for (int i = 0; i < N; i++)
                 {
-                    float4 a0[kUp], aw[kUp], pc[kUp];
-                    float2 a1[kUp];
-#pragma unroll
-                    for (int i = 0; i < kUp; i++)
-                    {
-                        const int u = min(b + i, top_r - 1), o = (u - u0) * rp + li;
-                        pc[i] = sp[cu[u * rp]];
-                        a0[i] = sU0[o];
-                        a1[i] = sU1[o];
-                        aw[i] = zero4;
-                        if (SKEW && skew)
-                            aw[i] = sUw[o];
-                    }
-#pragma unroll
-                    for (int i = 0; i < kUp; i++)
-                        add(b + i < min(ne, u1), a0[i], a1[i], aw[i], xyz(pc[i]), false);
+                    pc[i] = sp[cr[i * 32]];
+                    b[i] = on_chip(at + i * rp * kb);
                 }
 #pragma unroll
-                for (int i = 1; i < kPre; i++)
-                    if (u1 + i - 1 < top_u)
-                        add(u1 + i - 1 < ne, f0[i], f1[i], fw[i], xyz(sp[cu[(u1 + i - 1) * rp]]),
-                            false);
-                for (int u = u1 + kPre - 1; u < top_u; u++)
-                {
-                    float4 a0 = zero4, aw = zero4;
-                    float2 a1 = make_float2(0.f, 0.f);
-                    if (u < ne)
-                    {
-                        const uint32_t oa = up_idx(u, row, wu);
-                        a0 = __ldg(d.A0 + oa);
-                        a1 = __ldg(d.A1 + oa);
-                        if (SKEW && skew)
-                            aw = __ldg(d.Aw + oa);
-                    }
-                    add(u < ne, a0, a1, aw, xyz(sp[cu[u * rp]]), false);
-                }
-                const float3 pv = xyz(sp[own0 + min(li, nrow - 1)]);
-                chunk_add<1>(s_dig[0], warp_sum(li < nrow ? fdot(pv, q[k]) : 0.f), s_scale[0]);
-            }
+                for (int i = 0; i < N; i++)
+                    add(b[i], pc[i], false, true);
+                at += N * rp * kb;
+                cr += N * 32;
+            };
+            int u = u0;
+            for (; u + 3 <= top_r; u += 3)
+                walk(std::integral_constant<int, 3>());
+            for (; u < top_r; u++)
+                walk(std::integral_constant<int, 1>());
+#pragma unroll
+            for (int i = 1; i < 3; i++)
+                if (u1 + i - 1 < top_u)
+                    add(f[i], sp[cu[(u1 + i - 1) * 32]], false, true);
+            for (u = u1 + 2; u < top_u; u++)
+                add(from_l2(u < ne, u, row), sp[cu[u * 32]], false, true);
+            const float3 pv = xyz(sp[own0 + min(li, nrow - 1)]);
+            part[k] = warp_sum(li < nrow ? fdot(pv, q[k]) : 0.f);
         }
+        chunks_add<K>(s_dig, s_scale, part);
         bar_arrive(2, kAll);
         if (!CLUSTER && multi && w.rank == 0 && warp == kWarps - 1)
         {
@@ -1372,19 +1544,18 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
         if (*(volatile int *)&sh.stop)
             break;
         const float af = *(volatile float *)&sh.af;
-        // ---- dx += alpha p, r -= alpha q, z = M^-1 r; r.z and r.r per chunk
+        // ---- r -= alpha q, z = M^-1 r; r.z and r.r per chunk (dx += alpha p
+        // once they are on their way)
 #pragma unroll
         for (int k = 0; k < K; k++)
         {
             const int ch = warp + k * kWarps, li = ch * 32 + lane;
+            part[k] = 0.f;
             if (ch < nch)
             {
                 float pr = 0.f, prr = 0.f;
                 if (li < nrow)
                 {
-                    const float3 p = xyz(sp[own0 + li]);
-                    x[k] = make_float3(fmaf(af, p.x, x[k].x), fmaf(af, p.y, x[k].y),
-                                       fmaf(af, p.z, x[k].z));
                     r[k] = make_float3(fmaf(-af, q[k].x, r[k].x), fmaf(-af, q[k].y, r[k].y),
                                        fmaf(-af, q[k].z, r[k].z));
                     const float M[6] = {m0[k].x, m0[k].y, m0[k].z, m0[k].w, m1[k].x, m1[k].y};
@@ -1396,12 +1567,22 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
                     pr = fdot(r[k], z[k]);
                     prr = fdot(r[k], r[k]);
                 }
-                pr = warp_sum(pr);
-                prr = warp_sum(prr);
-                chunk_add<2>(s_dig[1], lane < 8 ? pr : prr, s_scale[lane < 8 ? 1 : 2]);
+                part[k] = warp_sum2(pr, prr);
             }
         }
+        chunks_add2<K>(s_dig, s_scale, part);
         bar_arrive(4, kAll);
+#pragma unroll
+        for (int k = 0; k < K; k++)
+        {
+            const int li = (warp + k * kWarps) * 32 + lane;
+            if (li < nrow)
+            {
+                const float3 p = xyz(sp[own0 + li]);
+                x[k] = make_float3(fmaf(af, p.x, x[k].x), fmaf(af, p.y, x[k].y),
+                                   fmaf(af, p.z, x[k].z));
+            }
+        }
         // the halo rows of the new z, while the sums are under way
         if (CLUSTER)
         {
@@ -1411,7 +1592,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
         }
         else
 #pragma unroll
-            for (int u = 0; u < kAhead3; u++)
+            for (int u = 0; u < kHaloAhead; u++)
             {
                 const int i = tid + u * kWorkers;
                 if (i < nhalo)
@@ -1445,21 +1626,24 @@ template <int K> const void *half_kernel(bool skew, bool cluster)
                            : (const void *)k_pcg_half<K, false, false>);
 }
 
+template <int K> const void *row_kernel(bool skew, bool cluster)
+{
+    constexpr int T = K < 1 ? 1 : K;
+    return cluster ? (skew ? (const void *)k_pcg_team<T, team_reg_slots(K, true), true, true>
+                           : (const void *)k_pcg_team<T, team_reg_slots(K, false), false, true>)
+                   : (skew ? (const void *)k_pcg_team<T, team_reg_slots(K, true), true, false>
+                           : (const void *)k_pcg_team<T, team_reg_slots(K, false), false, false>);
+}
+
 const void *team_kernel(int k, bool half, bool skew, bool cluster)
 {
     if (half)
         return k <= 2   ? half_kernel<2>(skew, cluster)
                : k == 3 ? half_kernel<3>(skew, cluster)
                         : half_kernel<4>(skew, cluster);
-    if (cluster)
-        return k <= 1 ? (skew ? (const void *)k_pcg_team<1, true, true>
-                              : (const void *)k_pcg_team<1, false, true>)
-                      : (skew ? (const void *)k_pcg_team<2, true, true>
-                              : (const void *)k_pcg_team<2, false, true>);
-    return k <= 1 ? (skew ? (const void *)k_pcg_team<1, true, false>
-                          : (const void *)k_pcg_team<1, false, false>)
-                  : (skew ? (const void *)k_pcg_team<2, true, false>
-                          : (const void *)k_pcg_team<2, false, false>);
+    return k == 0   ? row_kernel<0>(skew, cluster)
+           : k == 1 ? row_kernel<1>(skew, cluster)
+                    : row_kernel<2>(skew, cluster);
 }
 
 } // namespace cloth
