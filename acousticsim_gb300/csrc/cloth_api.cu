@@ -2,6 +2,7 @@
 // step driver (one CUDA graph per launch set, PCG as a device-side while loop),
 // batches and exports.  Declarations and reference mapping: include/cloth_gb300.h.
 #include <map>
+#include <tuple>
 #include "internal.h"
 
 #include <algorithm>
@@ -55,6 +56,20 @@ cloth_s::~cloth_s()
 
 namespace cloth {
 namespace detail {
+
+// One launch of a persistent PCG kernel: its work list, and behind it what is
+// zeroed before every launch (arrival counts or team sums).
+struct PersistLaunch
+{
+    const void *func = nullptr;
+    bool on_chip = false; // k_pcg_team or k_pcg_half (their arguments)
+    int cluster = 0;      // teams are clusters of this many blocks (0: all blocks resident)
+    int grid = 0, block = 0;
+    size_t smem = 0;
+    TeamBlock *d_work = nullptr;
+    char *d_sync = nullptr;
+    size_t sync_bytes = 0;
+};
 
 struct Batch
 {
@@ -128,16 +143,8 @@ struct Batch
     bool persist_ok = false;
     bool persist_sm = false; // own-row state in shared memory
     bool persist_1b = false; // single-barrier variant (shared memory, every halo staged)
-    bool persist_team = false; // k_pcg_team: the matrix on chip
-    int team_rows = 1;         // its rows per thread
-    bool team_half = false;    // k_pcg_half: the stored blocks only
-    int team_cluster = 0;      // its teams are clusters of this many blocks (0: not clusters)
-    TeamBlock *d_work = nullptr;
-    char *d_sync = nullptr;    // behind the work list: arrival counts or team sums
-    size_t sync_bytes = 0;
-    int grid_persist = 0, block_persist = kPBlock;
+    std::vector<PersistLaunch> launches; // side by side, each over its own members
     int halo_cap = 0, rows_cap = 0;
-    size_t smem_persist = 0;
     SpinCfg spin = {kSpinLimitDefault, 0u}; // the context's setting when the set was built
     // graph loop: the active count at which the loop stops and the persistent
     // kernel finishes the rest (0: the loop runs to the end), and the launch
@@ -156,8 +163,8 @@ struct Batch
             cudaFree(mem);
         if (h_pinned)
             cudaFreeHost(h_pinned);
-        if (d_work)
-            cudaFree(d_work);
+        for (auto &l : launches)
+            cudaFree(l.d_work);
     }
 };
 
@@ -821,11 +828,9 @@ int make_batch(cloth_ctx *ctx, const std::vector<cloth_s *> &members,
     return CLOTH_OK;
 }
 
-// The persistent kernel a plan launches.
+// The two-barrier or single-barrier persistent kernel a plan launches.
 const void *persistent_kernel(const Batch *b)
 {
-    if (b->persist_team)
-        return team_kernel(b->team_rows, b->team_half, b->skew, b->team_cluster > 0);
     if (b->persist_1b)
         return (const void *)k_pcg1_persistent;
     if (b->skew)
@@ -834,28 +839,28 @@ const void *persistent_kernel(const Batch *b)
     return b->persist_sm ? (const void *)k_pcg_persistent_sm : (const void *)k_pcg_persistent_gm;
 }
 
-// The persistent kernels' arguments (k_pcg_team takes fewer).
+// The persistent kernels' arguments (the on-chip ones take fewer).
 struct PersistArgs
 {
-    void *team[4], *two[5];
-    explicit PersistArgs(Batch *b)
-        : team{&b->d_descs, &b->d_work, &b->d_sync, &b->spin},
-          two{&b->d_descs, &b->d_work, &b->halo_cap, &b->rows_cap, &b->spin}
+    void *chip[4], *two[5];
+    PersistArgs(Batch *b, PersistLaunch &l)
+        : chip{&b->d_descs, &l.d_work, &l.d_sync, &b->spin},
+          two{&b->d_descs, &l.d_work, &b->halo_cap, &b->rows_cap, &b->spin}
     {
     }
-    void **of(const Batch *b) { return b->persist_team ? team : two; }
+    void **of(const PersistLaunch &l) { return l.on_chip ? chip : two; }
 };
 
 // How a persistent launch keeps its teams together: all blocks resident, or
 // every team a cluster.
-cudaLaunchAttribute persist_attribute(const Batch *b)
+cudaLaunchAttribute persist_attribute(const PersistLaunch &l)
 {
     cudaLaunchAttribute at;
     std::memset(&at, 0, sizeof(at));
-    if (b->persist_team && b->team_cluster > 0)
+    if (l.cluster > 0)
     {
         at.id = cudaLaunchAttributeClusterDimension;
-        at.val.clusterDim.x = unsigned(b->team_cluster);
+        at.val.clusterDim.x = unsigned(l.cluster);
         at.val.clusterDim.y = at.val.clusterDim.z = 1;
     }
     else
@@ -866,18 +871,19 @@ cudaLaunchAttribute persist_attribute(const Batch *b)
     return at;
 }
 
-// The work list of a persistent launch, and behind it per_block bytes for
-// every block, zeroed before each launch.
-int upload_work(Batch *b, const std::vector<TeamBlock> &work, size_t per_block, size_t align)
+// Adds a launch over a work list, with per_block bytes zeroed for every block.
+int add_launch(Batch *b, PersistLaunch l, const std::vector<TeamBlock> &work, size_t per_block,
+               size_t align)
 {
     const size_t at = align_up(work.size() * sizeof(TeamBlock), align);
-    b->sync_bytes = work.size() * per_block;
-    CK(cudaMalloc(&b->d_work, at + b->sync_bytes));
-    b->d_sync = reinterpret_cast<char *>(b->d_work) + at;
-    CK(cudaMemcpy(b->d_work, work.data(), work.size() * sizeof(TeamBlock),
-                  cudaMemcpyHostToDevice));
-    b->grid_persist = int(work.size());
+    l.sync_bytes = work.size() * per_block;
+    CK(cudaMalloc(&l.d_work, at + l.sync_bytes));
+    l.d_sync = reinterpret_cast<char *>(l.d_work) + at;
+    l.grid = int(work.size());
+    b->launches.push_back(l);
     b->persist_ok = true;
+    CK(cudaMemcpy(l.d_work, work.data(), work.size() * sizeof(TeamBlock),
+                  cudaMemcpyHostToDevice));
     return CLOTH_OK;
 }
 
@@ -930,13 +936,23 @@ bool team_split(const Batch *b, int i, int blocks, TeamKernel tk, bool cluster, 
         {
             // as many planes of stored blocks as fit: all, or those from the
             // first upper one on (the diagonal's serves no lower slot)
-            int planes = h.width_up;
-            while (planes > 0 && half_smem_bytes(halo, nr, planes, h.width_lo + h.width_up, skew,
-                                                 cluster) > cap)
+            const int words = h.width_lo + h.width_up;
+            auto need = [&](int planes, int ext) {
+                return half_smem_bytes(halo, nr, ext, planes, words, skew, cluster);
+            };
+            int planes = h.width_up, ext = 0;
+            while (planes > 0 && need(planes, 0) > cap)
                 planes--;
-            bytes = half_smem_bytes(halo, nr, planes, h.width_lo + h.width_up, skew, cluster);
             const int u0 = planes == h.width_up ? 0 : 1;
-            w.p_global = u0 | std::min(u0 + planes, h.width_up) << 8;
+            planes = std::min(planes, h.width_up - u0);
+            // and, in what is left, the rows in front (an even number: planes
+            // stay 16-byte aligned)
+            if (planes > 0 && need(planes, 0) <= cap)
+                ext = int(std::min<size_t>(size_t(w.row0 - w.halo0),
+                                           (cap - need(planes, 0)) / (size_t(planes) * (skew ? 40 : 24)))) &
+                      ~1;
+            bytes = need(planes, ext);
+            w.p_global = u0 | (u0 + planes) << 4 | ext << 8;
             fits = planes >= 2 && halo <= 4096;
         }
         else
@@ -955,23 +971,30 @@ bool team_split(const Batch *b, int i, int blocks, TeamKernel tk, bool cluster, 
     return true;
 }
 
-// Plan of k_pcg_team whose teams are clusters of C blocks (at_once: all of them
-// resident together).
-bool plan_cluster(cloth_ctx *ctx, const Batch *b, TeamKernel tk, int C,
-                  std::vector<TeamBlock> &work, size_t &smem, bool at_once)
+// Most dynamic shared memory of a block of a cluster.
+size_t cluster_smem_cap(const cloth_ctx *ctx) { return size_t(ctx->max_smem_optin) - 6144; }
+
+// Plan of an on-chip kernel over some members, its teams clusters of C blocks
+// (at_once: all of them resident together).
+bool plan_cluster(cloth_ctx *ctx, const Batch *b, std::vector<int> which, TeamKernel tk, int C,
+                  bool at_once, std::vector<TeamBlock> &work, PersistLaunch &l)
 {
-    const size_t cap = size_t(ctx->max_smem_optin) - 6144;
-    const int n = int(b->members.size());
-    smem = 0;
+    const size_t cap = cluster_smem_cap(ctx);
+    const int n = int(which.size());
+    size_t smem = 0;
     work.clear();
-    // the largest first: clusters start in this order as SMs come free
-    std::vector<int> order(n);
-    for (int i = 0; i < n; i++)
-        order[i] = i;
-    std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
-        return b->members[x]->tab.nv > b->members[y]->tab.nv;
-    });
-    for (int i : order)
+    // clusters start in this order as SMs come free: the ones that should run
+    // longest first (PCG iterations grow with the waves a step sends over the
+    // cloth's vertices, a side's worth at sqrt(stiffness / density))
+    auto cost = [&](int i) {
+        const cloth_s *c = b->members[i];
+        const double k = std::max({c->mat.stretch_k[0], c->mat.stretch_k[1], 0.f});
+        const double rho = std::max(1e-12, double(c->mat.density));
+        return double(c->tab.nv) * std::sqrt(double(c->tab.nv) * k / rho);
+    };
+    std::stable_sort(which.begin(), which.end(),
+                     [&](int x, int y) { return cost(x) > cost(y); });
+    for (int i : which)
     {
         if (!team_split(b, i, C, tk, true, cap, work, smem))
             return false;
@@ -979,6 +1002,12 @@ bool plan_cluster(cloth_ctx *ctx, const Batch *b, TeamKernel tk, int C,
             work.push_back(TeamBlock{-1, 0, 0, 0, 0, 0, 0, 0});
     }
     const void *f = team_kernel(tk.K, tk.half, b->skew, true);
+    l = PersistLaunch();
+    l.func = f;
+    l.on_chip = true;
+    l.cluster = C;
+    l.block = kTeamThreads;
+    l.smem = smem;
     cudaLaunchConfig_t cfg;
     std::memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3(unsigned(work.size()));
@@ -1008,8 +1037,9 @@ bool plan_cluster(cloth_ctx *ctx, const Batch *b, TeamKernel tk, int C,
 // all resident at once: every block's rows, their blocks and p over their
 // columns on its SM.  False when the set does not fit.
 bool plan_team(cloth_ctx *ctx, const Batch *b, TeamKernel tk, std::vector<TeamBlock> &work,
-               size_t &smem)
+               PersistLaunch &l)
 {
+    size_t smem = 0;
     const int G = std::min(ctx->num_sms, kTeamMaxBlocks);
     const int n = int(b->members.size());
     if (n > G)
@@ -1018,7 +1048,6 @@ bool plan_team(cloth_ctx *ctx, const Batch *b, TeamKernel tk, std::vector<TeamBl
     long long total = 0;
     for (auto *c : b->members)
         total += c->tab.nv;
-    smem = 0;
     work.clear();
     for (int i = 0; i < n; i++)
     {
@@ -1043,6 +1072,92 @@ bool plan_team(cloth_ctx *ctx, const Batch *b, TeamKernel tk, std::vector<TeamBl
         cudaGetLastError();
         return false;
     }
+    l = PersistLaunch();
+    l.func = f;
+    l.on_chip = true;
+    l.block = kTeamThreads;
+    l.smem = smem;
+    return true;
+}
+
+// Plan of a set as one launch per size of cluster, side by side: every cloth
+// gets the smallest cluster that holds it with one row a thread (16 blocks: 7,680
+// rows), or 16 blocks with its stored blocks alone (~16,000 rows), and clusters
+// start, the largest cloths first, as SMs come free.  While the set leaves SMs
+// idle the clusters are doubled.  False when a cloth fits no cluster.
+bool plan_queue(cloth_ctx *ctx, Batch *b, int *rc)
+{
+    struct Choice
+    {
+        TeamKernel k;
+        int C;
+    };
+    const TeamKernel one{b->skew ? 0 : 1, false};
+    const size_t cap = cluster_smem_cap(ctx);
+    const int n = int(b->members.size());
+    std::vector<Choice> choice(n);
+    std::vector<TeamBlock> work;
+    long long blocks = 0;
+    for (int i = 0; i < n; i++)
+    {
+        bool fits = false;
+        size_t smem = 0;
+        for (int C = 1; C <= kClusterMax && !fits; C *= 2)
+            for (TeamKernel k : {one, TeamKernel{1, false}})
+            {
+                work.clear();
+                if ((fits = team_split(b, i, C, k, true, cap, work, smem)))
+                {
+                    choice[i] = Choice{k, C};
+                    break;
+                }
+            }
+        for (TeamKernel k : {TeamKernel{2, false}, TeamKernel{2, true}, TeamKernel{3, true},
+                             TeamKernel{4, true}})
+        {
+            if (fits)
+                break;
+            work.clear();
+            if ((fits = team_split(b, i, kClusterMax, k, true, cap, work, smem)))
+                choice[i] = Choice{k, kClusterMax};
+        }
+        if (!fits)
+            return false;
+        blocks += choice[i].C;
+    }
+    while (blocks * 2 <= ctx->num_sms * 3 / 4)
+    {
+        blocks = 0;
+        bool grew = false;
+        for (int i = 0; i < n; i++)
+        {
+            Choice &c = choice[i];
+            if (c.C < kClusterMax && b->members[i]->tab.nv > 64 * c.C)
+            {
+                c.C *= 2;
+                grew = true;
+            }
+            blocks += c.C;
+        }
+        if (!grew)
+            break;
+    }
+    // one launch per kernel and cluster size, the largest first
+    std::map<std::tuple<int, int, int>, std::vector<int>> groups;
+    for (int i = 0; i < n; i++)
+        groups[std::make_tuple(-choice[i].C, -int(choice[i].k.half), -choice[i].k.K)].push_back(i);
+    std::vector<std::pair<PersistLaunch, std::vector<TeamBlock>>> plans;
+    for (auto &g : groups)
+    {
+        PersistLaunch l;
+        const Choice &c = choice[g.second[0]];
+        if (!plan_cluster(ctx, b, g.second, c.k, c.C, false, work, l))
+            return false;
+        plans.emplace_back(l, work);
+    }
+    for (auto &p : plans)
+        if (*rc == CLOTH_OK)
+            *rc = add_launch(b, p.first, p.second, sizeof(unsigned long long), sizeof(TeamBlock));
     return true;
 }
 
@@ -1059,28 +1174,26 @@ int plan_persistent(cloth_ctx *ctx, Batch *b)
     std::vector<TeamBlock> work;
     if (ctx->solver != CLOTH_SOLVER_PERSISTENT_1B)
     {
-        b->persist_team = true;
-        b->block_persist = kTeamThreads;
         int most = 0;
+        std::vector<int> all;
         for (auto *c : b->members)
+        {
             most = std::max(most, c->tab.nv);
-        auto use = [&](TeamKernel k, int C) {
-            b->team_rows = k.K;
-            b->team_half = k.half;
-            b->team_cluster = C;
-        };
-        // Clusters where the set's cloths fit them with one row a thread and
-        // all run at once.  Up to 320 rows a block alone is fastest (us per
-        // iteration, 16^2: 2.3, in a cluster of 16 2.8; 20^2: 2.7 and 2.7), above
-        // it 16 blocks (32^2: 2.6, two blocks 2.9; 64^2: 2.9, the whole GPU 3.3;
-        // 80^2: 3.3 and 3.3)
+            all.push_back(int(all.size()));
+        }
+        PersistLaunch l;
+        // Clusters of one size where the set's cloths fit them with one row a
+        // thread and all run at once.  Up to 320 rows a block alone is fastest
+        // (us per iteration, 16^2: 2.2, in a cluster of 16 2.8), above it 16
+        // blocks (32^2: 2.6, two blocks 2.9; 64^2: 2.7, the whole GPU 3.3;
+        // 80^2: 3.0 and 3.3)
         const int C = most <= kTeamAloneRows ? 1 : kClusterMax;
         const TeamKernel one{b->skew ? 0 : 1, false};
-        if (plan_cluster(ctx, b, one, C, work, b->smem_persist, true))
-        {
-            use(one, C);
-            return upload_work(b, work, sizeof(unsigned long long), sizeof(TeamBlock));
-        }
+        if (plan_cluster(ctx, b, all, one, C, true, work, l))
+            return add_launch(b, l, work, sizeof(unsigned long long), sizeof(TeamBlock));
+        int rc = CLOTH_OK;
+        if (most <= kClusterMax * kTeamWorkers && plan_queue(ctx, b, &rc))
+            return rc;
         // Teams over the whole GPU: the whole matrix on chip where it fits (256^2:
         // 4.2 us with one row a thread), else the stored blocks (300^2: 6.8, the
         // kernel that reads the matrix from L2 13.0; 512^2: 15.8 and 21.4), with
@@ -1088,12 +1201,10 @@ int plan_persistent(cloth_ctx *ctx, Batch *b)
         // three)
         for (TeamKernel k : {one, TeamKernel{1, false}, TeamKernel{2, false}, TeamKernel{2, true},
                              TeamKernel{3, true}, TeamKernel{4, true}})
-            if (plan_team(ctx, b, k, work, b->smem_persist))
-            {
-                use(k, 0);
-                return upload_work(b, work, sizeof(TeamSync), alignof(TeamSync) * 64);
-            }
-        b->persist_team = false;
+            if (plan_team(ctx, b, k, work, l))
+                return add_launch(b, l, work, sizeof(TeamSync), alignof(TeamSync) * 64);
+        if (plan_queue(ctx, b, &rc))
+            return rc;
     }
     work.clear();
     const size_t smem_cap_bytes =
@@ -1224,7 +1335,8 @@ int plan_persistent(cloth_ctx *ctx, Batch *b)
     const size_t sm_bytes = size_t(max_entries) * sizeof(float4) +
                             size_t(max_rows) * (kPersistMShared ? 72 : 48) + part_bytes;
     b->persist_sm = sm_bytes <= smem_cap_bytes;
-    b->smem_persist =
+    PersistLaunch l;
+    l.smem =
         b->persist_sm ? sm_bytes : size_t(max_entries) * sizeof(float4) + part_bytes;
     // the single-barrier variant keeps dx, p and M^-1 per own row (56 bytes)
     // next to u over the halo: it fits wherever the two-barrier one does
@@ -1238,7 +1350,7 @@ int plan_persistent(cloth_ctx *ctx, Batch *b)
         cudaFuncSetAttribute(k_pcg_persistent_gm_skew, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              int(smem_cap_bytes)) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ2, persistent_kernel(b), kPBlock,
-                                                      b->smem_persist) != cudaSuccess ||
+                                                      l.smem) != cudaSuccess ||
         occ2 * ctx->num_sms < int(work.size()))
     {
         cudaGetLastError();
@@ -1246,8 +1358,9 @@ int plan_persistent(cloth_ctx *ctx, Batch *b)
     }
     // one arrival count per block slot (the team barrier of the two-barrier
     // kernels) behind the work list
-    b->block_persist = kPBlock;
-    return upload_work(b, work, sizeof(unsigned long long), sizeof(TeamBlock));
+    l.func = persistent_kernel(b);
+    l.block = kPBlock;
+    return add_launch(b, l, work, sizeof(unsigned long long), sizeof(TeamBlock));
 }
 
 int add_kernel(cudaGraph_t g, cudaGraphNode_t *node, const cudaGraphNode_t *deps,
@@ -1290,12 +1403,16 @@ int build_graph(Batch *b, bool full, cudaGraphExec_t *exec)
     void *a_upd[] = {&b->d_descs, &b->d_rt, &b->d_ctl, &one, &hnd, &no_left};
     void *a_adv[] = {&b->d_descs, &b->d_rt, &b->d_ctl, &all_rows};
     (void)zero;
+    std::vector<cudaGraphNode_t> ends; // the persistent launches
     auto chain = [&](void *f, int grid, void **args) {
         if (rc != CLOTH_OK)
             return;
-        rc = add_kernel(g, &n, last ? &last : nullptr, last ? 1 : 0, f, grid,
+        const bool join = !ends.empty();
+        rc = add_kernel(g, &n, join ? ends.data() : last ? &last : nullptr,
+                        join ? ends.size() : last ? 1 : 0, f, grid,
                         f == (void *)k_cond ? 1 : kTile, args);
         last = n;
+        ends.clear();
     };
     if (!b->persist_ok &&
         cudaGraphConditionalHandleCreate(&hnd, g, 1, cudaGraphCondAssignDefault) !=
@@ -1323,43 +1440,47 @@ int build_graph(Batch *b, bool full, cudaGraphExec_t *exec)
     if (b->persist_ok)
     {
         b->spin = b->ctx->spin;
-        PersistArgs a_per(b);
-        if (rc == CLOTH_OK)
+        // the launches side by side behind the assembly, each after its zeroed
+        // counts; what follows waits for all of them
+        const cudaGraphNode_t root = last;
+        for (auto &l : b->launches)
         {
-            // the team barriers' arrival counts (or team sums) start at zero
+            if (rc != CLOTH_OK)
+                break;
+            PersistArgs args(b, l);
             cudaMemsetParams mp;
             std::memset(&mp, 0, sizeof(mp));
-            mp.dst = b->d_sync;
+            mp.dst = l.d_sync;
             mp.value = 0;
             mp.elementSize = 4;
-            mp.width = b->sync_bytes / 4;
+            mp.width = l.sync_bytes / 4;
             mp.height = 1;
-            if (cudaGraphAddMemsetNode(&n, g, last ? &last : nullptr, last ? 1 : 0, &mp) !=
+            cudaGraphNode_t m = nullptr;
+            if (cudaGraphAddMemsetNode(&m, g, root ? &root : nullptr, root ? 1 : 0, &mp) !=
                 cudaSuccess)
+            {
                 rc = fail(CLOTH_ERR_CUDA, "cudaGraphAddMemsetNode failed");
-            else
-                last = n;
-        }
-        if (rc == CLOTH_OK)
-        {
+                break;
+            }
             cudaKernelNodeParams p;
             std::memset(&p, 0, sizeof(p));
-            p.func = const_cast<void *>(persistent_kernel(b));
-            p.gridDim = dim3(b->grid_persist);
-            p.blockDim = dim3(b->block_persist);
-            p.sharedMemBytes = unsigned(b->smem_persist);
-            p.kernelParams = a_per.of(b);
-            if (cudaGraphAddKernelNode(&n, g, last ? &last : nullptr, last ? 1 : 0, &p) !=
-                cudaSuccess)
+            p.func = const_cast<void *>(l.func);
+            p.gridDim = dim3(l.grid);
+            p.blockDim = dim3(l.block);
+            p.sharedMemBytes = unsigned(l.smem);
+            p.kernelParams = args.of(l);
+            if (cudaGraphAddKernelNode(&n, g, &m, 1, &p) != cudaSuccess)
                 rc = fail(CLOTH_ERR_CUDA, "cudaGraphAddKernelNode(persistent) failed");
             else
             {
-                const cudaLaunchAttribute at = persist_attribute(b);
+                const cudaLaunchAttribute at = persist_attribute(l);
                 if (cudaGraphKernelNodeSetAttribute(n, at.id, &at.val) != cudaSuccess)
                     rc = fail(CLOTH_ERR_CUDA, "launch attribute on graph node failed");
-                last = n;
+                ends.push_back(n);
             }
         }
+        if (rc == CLOTH_OK)
+            last = ends.back();
     }
     else
         chain((void *)k_cond, 1, a_cond);
@@ -1447,18 +1568,21 @@ int launch_persistent(Batch *b)
     cloth_ctx *ctx = b->ctx;
     PhaseTimer t(ctx, PH_SPMV);
     b->spin = ctx->spin;
-    PersistArgs args(b);
-    CK(cudaMemsetAsync(b->d_sync, 0, b->sync_bytes, ctx->stream));
-    cudaLaunchAttribute at = persist_attribute(b);
-    cudaLaunchConfig_t cfg;
-    std::memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3(b->grid_persist);
-    cfg.blockDim = dim3(b->block_persist);
-    cfg.dynamicSmemBytes = b->smem_persist;
-    cfg.stream = ctx->stream;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    CK(cudaLaunchKernelExC(&cfg, persistent_kernel(b), args.of(b)));
+    for (auto &l : b->launches)
+    {
+        PersistArgs args(b, l);
+        CK(cudaMemsetAsync(l.d_sync, 0, l.sync_bytes, ctx->stream));
+        cudaLaunchAttribute at = persist_attribute(l);
+        cudaLaunchConfig_t cfg;
+        std::memset(&cfg, 0, sizeof(cfg));
+        cfg.gridDim = dim3(l.grid);
+        cfg.blockDim = dim3(l.block);
+        cfg.dynamicSmemBytes = l.smem;
+        cfg.stream = ctx->stream;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        CK(cudaLaunchKernelExC(&cfg, l.func, args.of(l)));
+    }
     return CLOTH_OK;
 }
 

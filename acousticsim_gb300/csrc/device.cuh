@@ -219,7 +219,8 @@ struct TeamBlock
     int row0, row1;
     int halo0, halo1;
     int p_global; // the team keeps p in global memory (a block of it is not staged);
-                  // k_pcg_half: its planes of stored blocks on chip, first | end << 8
+                  // k_pcg_half: its planes of stored blocks on chip and the
+                  // rows in front of its own with them, first | end << 4 | rows << 8
 };
 
 // Fixed-point scale: sums are carried as round(v * 2^s) with s chosen from
@@ -283,14 +284,16 @@ __host__ __device__ inline size_t team_smem_bytes(int halo, int rows, int width,
     return (size_t(halo) + (cluster ? halo - rows : 0)) * 16 +
            size_t((rows + 1) & ~1) * 24 + size_t((rows + 31) / 32) * slots * team_slot_bytes(skew);
 }
-// The same of a k_pcg_half block: planes of stored blocks, and 16-bit words of
-// `words` slots per row.
-__host__ __device__ inline size_t half_smem_bytes(int halo, int rows, int planes, int words,
-                                                  bool skew, bool cluster)
+// 16-byte units of p over a halo in 12 bytes an entry.
+__host__ __device__ constexpr int half_p_quads(int halo) { return (3 * halo + 3) / 4; }
+// The same of a k_pcg_half block: planes of stored blocks of its rows and of
+// `ext` rows in front of them, and 16-bit words of `words` slots per row.
+__host__ __device__ inline size_t half_smem_bytes(int halo, int rows, int ext, int planes,
+                                                  int words, bool skew, bool cluster)
 {
     const size_t rp = size_t((rows + 31) / 32) * 32;
-    return (size_t(halo) + (cluster ? halo - rows : 0)) * 16 + size_t(planes) * rp * (skew ? 40 : 24) +
-           size_t(words) * rp * 2;
+    return size_t(half_p_quads(halo) + (cluster ? halo - rows : 0)) * 16 +
+           size_t(planes) * (rp + ext) * (skew ? 40 : 24) + size_t(words) * rp * 2;
 }
 // A team that is one thread-block cluster: its most blocks, and a block whose
 // halo holds rows [row0, row1) of this one (row i of z goes to z + 16 i in the

@@ -1200,8 +1200,9 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
 // only the diagonal and upper blocks are kept, each read by its own row and by
 // the rows whose lower block is its transpose.  Where not even those fit, the
 // planes [u0, u1) of them are on chip (the first upper ones, which serve lower
-// slots too; the work list says which), the others and the lower blocks whose
-// transposed row another block owns come from L2.  A column and the transposed
+// slots too; the work list says which) and the others come from L2, as do the
+// lower blocks whose transposed row another block owns, but for the last rows
+// in front of this block's that fit as well.  A column and the transposed
 // block's plane share one 16-bit word.  K: rows per thread.
 template <int K, bool SKEW, bool CLUSTER>
 __global__ void __launch_bounds__(kTeamThreads, 1)
@@ -1223,10 +1224,23 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
     const bool skew = SKEW && d.Aw;
     const bool multi = w.nblk > 1 || sc.extra != 0u;
     const int it0 = __ldcg(&st->iter);
-    const int u0 = w.p_global & 255, u1 = w.p_global >> 8; // planes on chip
+    // on chip: planes [u0, u1), of this block's rows and of the last `ext` rows
+    // in front of them (other blocks' rows that lower slots refer to)
+    const int u0 = w.p_global & 15, u1 = w.p_global >> 4 & 15, ext = w.p_global >> 8;
+    const int re = rp + ext; // rows of a plane
     const int wl = d.width_lo, wu = d.width_up;
-    float4 *sp = sm_dyn;
-    float4 *sz = sp + nh;
+    // p over the halo in 12 bytes an entry (x and y, then z)
+    float2 *spx = reinterpret_cast<float2 *>(sm_dyn);
+    float *spz = reinterpret_cast<float *>(spx + nh);
+    auto p_get = [&](int j) {
+        const float2 v = spx[j];
+        return make_float3(v.x, v.y, spz[j]);
+    };
+    auto p_set = [&](int j, float3 v) {
+        spx[j] = make_float2(v.x, v.y);
+        spz[j] = v.z;
+    };
+    float4 *sz = sm_dyn + half_p_quads(nh);
     // plane by plane the rows' stored blocks (24 bytes; with skew parts 40):
     // read 8 bytes at a time, conflict-free at any row
     const int kb = SKEW && skew ? 40 : 24;
@@ -1234,17 +1248,20 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
     // chunk by chunk and slot by slot 32 words: the lower slots' (column | plane
     // << 12), then the upper planes' columns
     unsigned short *scol =
-        reinterpret_cast<unsigned short *>(sU + size_t(u1 - u0) * rp * kb);
+        reinterpret_cast<unsigned short *>(sU + size_t(u1 - u0) * re * kb);
     if (warp == kWarps)
     {
         control_warp<CLUSTER>(d, w, sync, sc, it0, multi, sh, s_dig, s_scale);
         return;
     }
     const int own0 = w.row0 - w.halo0;
+    // A warp's k-th chunk: the first kWarps chunks in turn, then from the last warp
+    // on (the first chunks have the lower slots that other blocks own)
+    auto chunk = [&](int k) { return k * kWarps + (k == 0 ? warp : kWarps - 1 - warp); };
     const unsigned bar_h = smem_u32(sh.bar + 2);
     if constexpr (CLUSTER)
         if (tid == 0)
-            find_peers(work, w, sh, [](int halo) { return smem_u32(sm_dyn) + 16u * unsigned(halo); });
+            find_peers(work, w, sh, [](int halo) { return smem_u32(sm_dyn) + 16u * unsigned(half_p_quads(halo)); });
     unsigned hphase = 0;
     float3 x[K], r[K], z[K];
     int info[K];
@@ -1252,7 +1269,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
 #pragma unroll
     for (int k = 0; k < K; k++)
     {
-        const int li = (warp + k * kWarps) * 32 + lane, row = w.row0 + li;
+        const int li = chunk(k) * 32 + lane, row = w.row0 + li;
         info[k] = 0;
         x[k] = r[k] = z[k] = make_float3(0.f, 0.f, 0.f);
         if (li < nrow)
@@ -1265,7 +1282,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
     }
     if (it0 > 0) // a solve handed over in its middle
         for (int i = tid; i < nh; i += kWorkers)
-            sp[i] = __ldcg(pold + w.halo0 + i);
+            p_set(i, xyz(__ldcg(pold + w.halo0 + i)));
     unsigned far = 0u; // chunks of this warp with a lower slot whose block is not on chip
 #pragma unroll 2
     for (int u = warp; u < (wl + wu) * nch; u += kWarps)
@@ -1304,7 +1321,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
             }
             if (here)
             {
-                float2 *o = reinterpret_cast<float2 *>(sU + (size_t(uu - u0) * rp + li) * kb);
+                float2 *o = reinterpret_cast<float2 *>(sU + (size_t(uu - u0) * re + ext + li) * kb);
                 o[0] = make_float2(a0.x, a0.y);
                 o[1] = make_float2(a0.z, a0.w);
                 o[2] = a1;
@@ -1317,17 +1334,37 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
         }
         scol[size_t(u) * 32 + lane] = (unsigned short)word;
     }
+    for (int i = tid; i < ext; i += kWorkers)
+    {
+        const int row = w.row0 - ext + i, inf = d.rowinfo[row],
+                  ne = (inf & 255) - ((inf >> 8) & 255);
+        for (int uu = u0; uu < min(u1, ne); uu++)
+        {
+            const uint32_t oa = up_idx(uu, row, wu);
+            const float4 a0 = d.A0[oa];
+            float2 *o = reinterpret_cast<float2 *>(sU + (size_t(uu - u0) * re + i) * kb);
+            o[0] = make_float2(a0.x, a0.y);
+            o[1] = make_float2(a0.z, a0.w);
+            o[2] = d.A1[oa];
+            if (SKEW && skew)
+            {
+                const float4 aw = d.Aw[oa];
+                o[3] = make_float2(aw.x, aw.y);
+                o[4] = make_float2(aw.z, 0.f);
+            }
+        }
+    }
     bar_sync(1, kWorkers);
 #pragma unroll
     for (int k = 0; k < K; k++)
     {
-        const int ch = warp + k * kWarps;
+        const int ch = chunk(k);
         bool any = false;
         if (ch < nch)
             for (int s = 0; s < ((info[k] >> 8) & 255); s++)
             {
                 const unsigned wd = scol[(size_t(ch) * (wl + wu) + s) * 32 + lane];
-                any |= unsigned(int(wd & 4095u) - own0) >= unsigned(nrow) ||
+                any |= int(wd & 4095u) < own0 - ext ||
                        (wd >> 12) - unsigned(u0) >= unsigned(u1 - u0);
             }
         far |= __any_sync(kFull, any) ? 1u << k : 0u;
@@ -1364,14 +1401,14 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
                 zz = xyz(__ldcg(d.z + w.halo0 + j));
             else
                 zz = poll_row(d.z + w.halo0 + j, tag, sc.limit, &sh.err);
-            sp[j] = f4(first ? zz : pform(zz, bf, xyz(sp[j])));
+            p_set(j, first ? zz : pform(zz, bf, p_get(j)));
         }
 #pragma unroll
         for (int k = 0; k < K; k++)
         {
-            const int li = (warp + k * kWarps) * 32 + lane;
+            const int li = chunk(k) * 32 + lane;
             if (li < nrow)
-                sp[own0 + li] = f4(first ? z[k] : pform(z[k], bf, xyz(sp[own0 + li])));
+                p_set(own0 + li, first ? z[k] : pform(z[k], bf, p_get(own0 + li)));
         }
         bar_sync(1, kWorkers);
         // ---- q = A p; p.q per 32-row chunk
@@ -1380,7 +1417,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
 #pragma unroll
         for (int k = 0; k < K; k++)
         {
-            const int ch = warp + k * kWarps, li = ch * 32 + lane, row = w.row0 + li;
+            const int ch = chunk(k), li = ch * 32 + lane, row = w.row0 + li;
             q[k] = make_float3(0.f, 0.f, 0.f);
             part[k] = 0.f;
             if (ch >= nch)
@@ -1392,11 +1429,11 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
                 float A[6];
                 float4 w;
             };
-            auto add = [&](const Block &b, float4 pc, bool lower, bool on) {
-                float3 t = q[k] + symv(b.A, xyz(pc));
+            auto add = [&](const Block &b, float3 pc, bool lower, bool on) {
+                float3 t = q[k] + symv(b.A, pc);
                 if (SKEW && skew)
                 {
-                    const float3 cw = skewv(b.w, xyz(pc));
+                    const float3 cw = skewv(b.w, pc);
                     t = lower ? t - cw : t + cw;
                 }
                 q[k] = pick(on, t, q[k]);
@@ -1431,9 +1468,10 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
                 return b;
             };
             // upper planes that are not on chip: the first three in flight from here
-            Block f[3];
+            constexpr int kPre = 2;
+            Block f[kPre];
 #pragma unroll
-            for (int i = 0; i < 3; i++)
+            for (int i = 0; i < kPre; i++)
             {
                 const int u = i == 0 ? 0 : u1 + i - 1;
                 f[i] = from_l2((i > 0 || u0 > 0) && u < ne, u, row);
@@ -1441,18 +1479,18 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
             // lower slots, kLow at a time, loads first
             const unsigned short *cc = scol + size_t(ch) * (wl + wu) * 32 + lane;
             constexpr int kLow = 3;
-            const char *sUl = sU - (own0 + u0 * rp) * kb; // block of row own0 + r, plane u
+            const char *sUl = sU - (own0 - ext + u0 * re) * kb; // entry c, plane u at (u re + c) kb
             if (!(far >> k & 1u))
                 for (int s0 = 0; s0 < top_l; s0 += kLow)
                 {
                     Block b[kLow];
-                    float4 pc[kLow];
+                    float3 pc[kLow];
 #pragma unroll
                     for (int i = 0; i < kLow; i++)
                     {
                         const unsigned wd = cc[min(s0 + i, top_l - 1) * 32];
-                        pc[i] = sp[wd & 4095u];
-                        b[i] = on_chip(sUl + int((wd >> 12) * unsigned(rp) + (wd & 4095u)) * kb);
+                        pc[i] = p_get(wd & 4095u);
+                        b[i] = on_chip(sUl + int((wd >> 12) * unsigned(re) + (wd & 4095u)) * kb);
                     }
 #pragma unroll
                     for (int i = 0; i < kLow; i++)
@@ -1462,16 +1500,15 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
                 for (int s0 = 0; s0 < top_l; s0 += kLow)
                 {
                     Block b[kLow];
-                    float4 pc[kLow];
+                    float3 pc[kLow];
 #pragma unroll
                     for (int i = 0; i < kLow; i++)
                     {
                         const unsigned wd = cc[min(s0 + i, top_l - 1) * 32];
                         const int c = int(wd & 4095u), u = int(wd >> 12);
-                        pc[i] = sp[c];
-                        if (unsigned(c - own0) < unsigned(nrow) &&
-                            unsigned(u - u0) < unsigned(u1 - u0))
-                            b[i] = on_chip(sUl + (u * rp + c) * kb);
+                        pc[i] = p_get(c);
+                        if (c >= own0 - ext && unsigned(u - u0) < unsigned(u1 - u0))
+                            b[i] = on_chip(sUl + (u * re + c) * kb);
                         else
                             b[i] = from_l2(s0 + i < ds, u, c + w.halo0);
                     }
@@ -1482,24 +1519,24 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
             // upper slots in order (past a row's last one the blocks are zero)
             const unsigned short *cu = cc + wl * 32;
             if (u0 > 0)
-                add(f[0], sp[cu[0]], false, true);
+                add(f[0], p_get(cu[0]), false, true);
             const int top_r = min(top_u, u1);
-            const char *at = sU + li * kb;
+            const char *at = sU + (ext + li) * kb;
             const unsigned short *cr = cu + u0 * 32;
             auto walk = [&](auto count) {
                 constexpr int N = decltype(count)::value;
                 Block b[N];
-                float4 pc[N];
+                float3 pc[N];
 #pragma unroll
                 for (int i = 0; i < N; i++)
                 {
-                    pc[i] = sp[cr[i * 32]];
-                    b[i] = on_chip(at + i * rp * kb);
+                    pc[i] = p_get(cr[i * 32]);
+                    b[i] = on_chip(at + i * re * kb);
                 }
 #pragma unroll
                 for (int i = 0; i < N; i++)
                     add(b[i], pc[i], false, true);
-                at += N * rp * kb;
+                at += N * re * kb;
                 cr += N * 32;
             };
             int u = u0;
@@ -1508,12 +1545,12 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
             for (; u < top_r; u++)
                 walk(std::integral_constant<int, 1>());
 #pragma unroll
-            for (int i = 1; i < 3; i++)
+            for (int i = 1; i < kPre; i++)
                 if (u1 + i - 1 < top_u)
-                    add(f[i], sp[cu[(u1 + i - 1) * 32]], false, true);
-            for (u = u1 + 2; u < top_u; u++)
-                add(from_l2(u < ne, u, row), sp[cu[u * 32]], false, true);
-            const float3 pv = xyz(sp[own0 + min(li, nrow - 1)]);
+                    add(f[i], p_get(cu[(u1 + i - 1) * 32]), false, true);
+            for (u = u1 + kPre - 1; u < top_u; u++)
+                add(from_l2(u < ne, u, row), p_get(cu[u * 32]), false, true);
+            const float3 pv = p_get(own0 + min(li, nrow - 1));
             part[k] = warp_sum(li < nrow ? fdot(pv, q[k]) : 0.f);
         }
         chunks_add<K>(s_dig, s_scale, part);
@@ -1531,7 +1568,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
 #pragma unroll
         for (int k = 0; k < K; k++)
         {
-            const int li = (warp + k * kWarps) * 32 + lane;
+            const int li = chunk(k) * 32 + lane;
             m0[k] = make_float4(0.f, 0.f, 0.f, 0.f);
             m1[k] = make_float2(0.f, 0.f);
             if (li < nrow)
@@ -1549,7 +1586,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
 #pragma unroll
         for (int k = 0; k < K; k++)
         {
-            const int ch = warp + k * kWarps, li = ch * 32 + lane;
+            const int ch = chunk(k), li = ch * 32 + lane;
             part[k] = 0.f;
             if (ch < nch)
             {
@@ -1575,10 +1612,10 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
 #pragma unroll
         for (int k = 0; k < K; k++)
         {
-            const int li = (warp + k * kWarps) * 32 + lane;
+            const int li = chunk(k) * 32 + lane;
             if (li < nrow)
             {
-                const float3 p = xyz(sp[own0 + li]);
+                const float3 p = p_get(own0 + li);
                 x[k] = make_float3(fmaf(af, p.x, x[k].x), fmaf(af, p.y, x[k].y),
                                    fmaf(af, p.z, x[k].z));
             }
@@ -1607,7 +1644,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
 #pragma unroll
     for (int k = 0; k < K; k++)
     {
-        const int li = (warp + k * kWarps) * 32 + lane, row = w.row0 + li;
+        const int li = chunk(k) * 32 + lane, row = w.row0 + li;
         if (li < nrow)
         {
             d.dx[row] = f4(x[k]);

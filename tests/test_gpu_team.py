@@ -27,16 +27,22 @@ def _conf(h, w, model):
 # whole matrix on chip: every stored block on chip, and a part of them (with
 # rows whose transposed blocks another block owns), two, three and four rows a
 # thread
+# more cloths than SMs, of every size of cluster, the largest with their stored
+# blocks alone
+MANY = [(3 + k % 5, 4 + k % 3) for k in range(160)] + [(22, 23), (30, 33), (44, 45), (62, 61),
+                                                       (87, 88), (100, 100), (125, 128)]
+
+
 @pytest.mark.parametrize("model", ["quadratic", "dihedral"])
 @pytest.mark.parametrize("shapes", [[(2, 2)], [(3, 7)], [(4, 8)],
                                     [(3, 11)], [(16, 32)], [(19, 27)], [(20, 32)], [(21, 31)],
                                     [(65, 64)], [(128, 129)],
                                     [(150, 150), (149, 150), (150, 149), (140, 150)],
                                     [(5, 5), (90, 31), (2, 40), (64, 64)], [(270, 300)],
-                                    [(300, 320), (5, 5)], [(400, 401)], [(470, 480)]])
+                                    [(300, 320), (5, 5)], [(400, 401)], [(470, 480)], MANY])
 def test_team_kernel_matches_graph_loop(ctx, shapes, model):
     from acousticsim_gb300 import BaraffClothGpu, params
-    big = sum(h * w for h, w in shapes) > 60000  # a few iterations show it
+    big = sum(h * w for h, w in shapes) > 40000  # a few iterations show it
     p = params(max_iters=60 if big else 4000, rel_tol=1e-6)
     out = {}
     for solver in ("persistent", "graph_loop"):
