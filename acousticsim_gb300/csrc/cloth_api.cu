@@ -910,15 +910,15 @@ struct TeamKernel
     bool half;
 };
 
-// Adds instance i of b to an on-chip kernel's work list in at most `blocks`
+// Adds cloth c as instance i to an on-chip kernel's work list in at most `blocks`
 // blocks (rows in 32-aligned chunks); false when one does not fit its SM.
-bool team_split(const Batch *b, int i, int blocks, TeamKernel tk, bool cluster, size_t cap,
-                std::vector<TeamBlock> &work, size_t &smem)
+// skew_kernel: the kernel that applies skew block parts.
+bool team_split(const cloth_s *c, int i, bool skew_kernel, int blocks, TeamKernel tk,
+                bool cluster, size_t cap, std::vector<TeamBlock> &work, size_t &smem)
 {
-    const cloth_s *c = b->members[i];
     const Tables &t = c->tab;
     const InstDesc &h = c->h;
-    const bool skew = h.Aw != nullptr;
+    const bool skew = c->mat.bending_model == CLOTH_BENDING_DIHEDRAL;
     const size_t first = work.size();
     const int rows =
         ((t.nv + blocks - 1) / blocks + kRedRows - 1) / kRedRows * kRedRows;
@@ -956,7 +956,7 @@ bool team_split(const Batch *b, int i, int blocks, TeamKernel tk, bool cluster, 
             fits = planes >= 2 && halo <= 4096;
         }
         else
-            bytes = team_smem_bytes(halo, nr, h.width, skew, team_reg_slots(tk.K, b->skew),
+            bytes = team_smem_bytes(halo, nr, h.width, skew, team_reg_slots(tk.K, skew_kernel),
                                     cluster);
         if (!fits || bytes > cap)
         {
@@ -996,7 +996,7 @@ bool plan_cluster(cloth_ctx *ctx, const Batch *b, std::vector<int> which, TeamKe
                      [&](int x, int y) { return cost(x) > cost(y); });
     for (int i : which)
     {
-        if (!team_split(b, i, C, tk, true, cap, work, smem))
+        if (!team_split(b->members[i], i, b->skew, C, tk, true, cap, work, smem))
             return false;
         while (work.size() % size_t(C))
             work.push_back(TeamBlock{-1, 0, 0, 0, 0, 0, 0, 0});
@@ -1056,7 +1056,7 @@ bool plan_team(cloth_ctx *ctx, const Batch *b, TeamKernel tk, std::vector<TeamBl
             std::max(1ll, (long long)(G - (n - 1)) * nv / std::max(1ll, total));
         const int want =
             std::max(1, std::min<int>(int(share), (nv + kTeamMinRows - 1) / kTeamMinRows));
-        if (!team_split(b, i, want, tk, false, cap, work, smem))
+        if (!team_split(b->members[i], i, b->skew, want, tk, false, cap, work, smem))
             return false;
     }
     if (int(work.size()) > G)
@@ -1080,48 +1080,51 @@ bool plan_team(cloth_ctx *ctx, const Batch *b, TeamKernel tk, std::vector<TeamBl
     return true;
 }
 
-// Plan of a set as one launch per size of cluster, side by side: every cloth
-// gets the smallest cluster that holds it with one row a thread (16 blocks: 7,680
-// rows), or 16 blocks with its stored blocks alone (~16,000 rows), and clusters
-// start, the largest cloths first, as SMs come free.  While the set leaves SMs
-// idle the clusters are doubled.  False when a cloth fits no cluster.
+// A cloth's kernel and cluster in a set of many: the smallest cluster that holds
+// it with one row a thread (16 blocks: 7,680 rows), or 16 blocks with its stored
+// blocks alone (~16,000 rows).  C = 0: none.
+struct ClusterChoice
+{
+    TeamKernel k;
+    int C;
+};
+ClusterChoice cluster_choice(const cloth_ctx *ctx, const cloth_s *c, bool skew_kernel)
+{
+    const TeamKernel one{skew_kernel ? 0 : 1, false};
+    const size_t cap = cluster_smem_cap(ctx);
+    std::vector<TeamBlock> work;
+    size_t smem = 0;
+    for (int C = 1; C <= kClusterMax; C *= 2)
+        for (TeamKernel k : {one, TeamKernel{1, false}})
+        {
+            work.clear();
+            if (team_split(c, 0, skew_kernel, C, k, true, cap, work, smem))
+                return ClusterChoice{k, C};
+        }
+    for (TeamKernel k :
+         {TeamKernel{2, false}, TeamKernel{2, true}, TeamKernel{3, true}, TeamKernel{4, true}})
+    {
+        work.clear();
+        if (team_split(c, 0, skew_kernel, kClusterMax, k, true, cap, work, smem))
+            return ClusterChoice{k, kClusterMax};
+    }
+    return ClusterChoice{one, 0};
+}
+
+// Plan of a set as one launch per size of cluster, side by side, each cloth with
+// cluster_choice's; clusters start, the longest solves first, as SMs come free.
+// While the set leaves SMs idle the clusters are doubled.  False when a cloth fits
+// no cluster.
 bool plan_queue(cloth_ctx *ctx, Batch *b, int *rc)
 {
-    struct Choice
-    {
-        TeamKernel k;
-        int C;
-    };
-    const TeamKernel one{b->skew ? 0 : 1, false};
-    const size_t cap = cluster_smem_cap(ctx);
     const int n = int(b->members.size());
-    std::vector<Choice> choice(n);
+    std::vector<ClusterChoice> choice(n);
     std::vector<TeamBlock> work;
     long long blocks = 0;
     for (int i = 0; i < n; i++)
     {
-        bool fits = false;
-        size_t smem = 0;
-        for (int C = 1; C <= kClusterMax && !fits; C *= 2)
-            for (TeamKernel k : {one, TeamKernel{1, false}})
-            {
-                work.clear();
-                if ((fits = team_split(b, i, C, k, true, cap, work, smem)))
-                {
-                    choice[i] = Choice{k, C};
-                    break;
-                }
-            }
-        for (TeamKernel k : {TeamKernel{2, false}, TeamKernel{2, true}, TeamKernel{3, true},
-                             TeamKernel{4, true}})
-        {
-            if (fits)
-                break;
-            work.clear();
-            if ((fits = team_split(b, i, kClusterMax, k, true, cap, work, smem)))
-                choice[i] = Choice{k, kClusterMax};
-        }
-        if (!fits)
+        choice[i] = cluster_choice(ctx, b->members[i], b->skew);
+        if (choice[i].C == 0)
             return false;
         blocks += choice[i].C;
     }
@@ -1131,7 +1134,7 @@ bool plan_queue(cloth_ctx *ctx, Batch *b, int *rc)
         bool grew = false;
         for (int i = 0; i < n; i++)
         {
-            Choice &c = choice[i];
+            ClusterChoice &c = choice[i];
             if (c.C < kClusterMax && b->members[i]->tab.nv > 64 * c.C)
             {
                 c.C *= 2;
@@ -1150,7 +1153,7 @@ bool plan_queue(cloth_ctx *ctx, Batch *b, int *rc)
     for (auto &g : groups)
     {
         PersistLaunch l;
-        const Choice &c = choice[g.second[0]];
+        const ClusterChoice &c = choice[g.second[0]];
         if (!plan_cluster(ctx, b, g.second, c.k, c.C, false, work, l))
             return false;
         plans.emplace_back(l, work);
@@ -2060,6 +2063,30 @@ Batch *self_batch(cloth_s *c, int *rc)
 }
 
 } // namespace
+
+bool cloth::detail::cluster_plan(cloth_ctx *ctx, const cloth_s *c, ClusterPlan &out)
+{
+    const bool skew = c->mat.bending_model == CLOTH_BENDING_DIHEDRAL;
+    const ClusterChoice ch = cluster_choice(ctx, c, skew);
+    out = ClusterPlan();
+    if (ch.C == 0 ||
+        !team_split(c, 0, skew, ch.C, ch.k, true, cluster_smem_cap(ctx), out.blocks, out.smem))
+        return false;
+    while (out.blocks.size() % size_t(ch.C))
+        out.blocks.push_back(TeamBlock{-1, 0, 0, 0, 0, 0, 0, 0});
+    out.func = team_kernel(ch.k.K, ch.k.half, skew, true);
+    out.cluster = ch.C;
+    out.block = kTeamThreads;
+    if (cudaFuncSetAttribute(out.func, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             int(cluster_smem_cap(ctx))) != cudaSuccess ||
+        cudaFuncSetAttribute(out.func, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
+            cudaSuccess)
+    {
+        cudaGetLastError();
+        return false;
+    }
+    return true;
+}
 
 int cloth::detail::inner_solve(cloth_s *c, const double *rhs64, const cloth_solve_params *p,
                                cloth_solve_stats *stats)

@@ -243,10 +243,13 @@ constexpr unsigned kSpinLimitDefault = 1u << 25; // bounded barrier wait (~secon
 // CLOTH_ERR_TIMEOUT).  `extra` arrivals are added to every barrier's target:
 // 0 in normal use; a test sets it to make the waits run out (arrivals that no
 // block makes), which exercises the timeout path without any device fault.
+// `iters` (on-chip kernels): a launch leaves an instance's solve after that many
+// iterations, still active and ready to be resumed (0: at its end).
 struct SpinCfg
 {
     unsigned limit;
     unsigned extra;
+    unsigned iters = 0u;
 };
 
 // k_pcg_team: worker threads (one row each, or two) and the control warp - 16

@@ -222,6 +222,18 @@ unsigned bulk_stage_bytes(const std::vector<cloth_s *> &cloths, bool skew, bool 
 unsigned bulk_smem(const GraphLoopVariant &v, unsigned stage_bytes);
 int bulk_occupancy(const GraphLoopVariant &v, unsigned stage_bytes, int max_smem);
 
+// How one cloth is solved by a single cluster: the on-chip kernel, its cluster
+// size, shared memory and work list (inst 0), padded to the cluster's blocks.
+struct ClusterPlan
+{
+    const void *func = nullptr;
+    int cluster = 0, block = 0;
+    size_t smem = 0;
+    std::vector<TeamBlock> blocks;
+};
+// The smallest cluster that holds the cloth; false when none does.
+bool cluster_plan(cloth_ctx *ctx, const cloth_s *c, ClusterPlan &out);
+
 // Points the scratch fields of h at base (null: clears them).
 void bind_scratch(const cloth_s *c, InstDesc &h, char *base);
 // Own scratch of a cloth: allocate (and bind, upload the descriptor) / free.

@@ -39,6 +39,7 @@ namespace {
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kWorkers = kTeamWorkers;
 constexpr int kWarps = kWorkers / 32;
+constexpr int kLeave = 10;    // stop code: iterations used up, the solve goes on later
 constexpr int kHaloAhead = 3; // halo rows per thread polled before beta is known
 
 // ---- named barriers: 1 the workers, 2-6 workers with the control warp
@@ -769,6 +770,8 @@ __device__ __forceinline__ void control_warp(const InstDesc &d, const TeamBlock 
             }
             if (!stop && it >= max_iters)
                 stop = 8;
+            if (!stop && sc.iters != 0u && unsigned(it - it0) >= sc.iters)
+                stop = kLeave;
         }
     }
     if (lane == 0)
@@ -779,13 +782,16 @@ __device__ __forceinline__ void control_warp(const InstDesc &d, const TeamBlock 
         {
             const double rho_d = value(rho), b_d = value(rho_b);
             st->iter = it;
-            st->status = stop == 1 ? 0 : stop;
+            st->status = stop == 1 || stop == kLeave ? 0 : stop;
             st->rho = rho_d;
             st->rr = value(rr);
             st->pq = value(pq);
             st->alpha = have_a ? value(rho_a) / value(pq_a) : alpha0;
             st->beta = have_b ? (b_d == 0.0 ? 0.0 : rho_d / b_d) : beta0;
-            st->active = 0;
+            if (stop == kLeave)
+                st->beta = 0.0; // z holds the next p
+            else
+                st->active = 0;
         }
     }
     if (CLUSTER)
@@ -1190,6 +1196,9 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
         {
             d.dx[row] = f4(x[k]);
             d.r[row] = f4(r[k]);
+            // a solve that goes on later starts from its next p, formed above
+            if (*(volatile int *)&sh.stop == kLeave)
+                d.z[row] = f4(p[k]);
         }
     }
     if (CLUSTER)
@@ -1649,6 +1658,8 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
         {
             d.dx[row] = f4(x[k]);
             d.r[row] = f4(r[k]);
+            if (*(volatile int *)&sh.stop == kLeave)
+                d.z[row] = f4(p_get(own0 + li));
         }
     }
     if (CLUSTER)
