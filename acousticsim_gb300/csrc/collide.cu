@@ -37,7 +37,10 @@ namespace {
 
 constexpr int kColBlock = 256;
 constexpr int kLocalCand = 128;  // candidates one point or edge may gather
-constexpr int kRepBlock = 1024;
+constexpr int kRepBlock = 512;     // repulsion: four lanes a contact
+constexpr int kRepStaged = 1100;   // contacts whose records fit in its shared memory,
+constexpr int kRepFields = 65536;  // and their counts (2 bits each)
+constexpr int kRepList = 1024;     // work list entries there
 
 struct BodyView
 {
@@ -90,7 +93,7 @@ struct cloth_collide_s
     PtContact *pt = nullptr;
     EeContact *ee = nullptr;
     int *inc_off = nullptr, *inc_cur = nullptr, *inc = nullptr;
-    int *rptr = nullptr, *cstate = nullptr, *wa = nullptr, *wb = nullptr;
+    int *cstate = nullptr, *wa = nullptr, *wb = nullptr;
     int *tile_sum = nullptr;
     int4 *cverts = nullptr;   // cloth vertices of every contact (and their count)
     int4 *clpos = nullptr, *csucc = nullptr; // place in, and successor on, each vertex's list
@@ -1081,8 +1084,7 @@ __global__ void k_col_links(int nv, const CollideCounts *cnt, int cap_pt, int ca
     (void)cap_pt;
 }
 
-__global__ void k_col_dxr(int nv, const float4 *dx, double *dxr, int *rptr, int ncs,
-                          int *cstate)
+__global__ void k_col_dxr(int nv, const float4 *dx, double *dxr)
 {
     const int stride = gridDim.x * blockDim.x;
     for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += stride)
@@ -1091,177 +1093,271 @@ __global__ void k_col_dxr(int nv, const float4 *dx, double *dxr, int *rptr, int 
         dxr[3 * size_t(v)] = d.x;
         dxr[3 * size_t(v) + 1] = d.y;
         dxr[3 * size_t(v) + 2] = d.z;
-        rptr[v] = 0;
     }
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ncs; i += stride)
-        cstate[i] = 0;
 }
 
-// One contact's impulse on dxr (BaraffCloth.cpp:636-925), v: its cloth vertices.
-__device__ void repulse_one(const CollideCounts &c, const PtContact *pt, const EeContact *ee,
-                            int i, const int *v, const double *mass, double *dxr, double dt,
-                            double K)
+// What a contact's impulse (BaraffCloth.cpp:636-925) takes that does not depend
+// on dxr.  Its relative velocity is (w0 x0 + w1 x1 + w2 x2) / dt over its cloth
+// vertices v, and vertex j's change post * (((a_j It) / ms) n): the reference's
+// expressions for both kinds of contacts, factor by factor in their order (a
+// weight or a factor of 1 leaves a product as it is).
+struct alignas(16) Impulse
 {
-    const double v_thre = 0.01, scale = double(0.1f);
+    int4 v;                // cloth vertices and their count
+    int4 succ;             // the next contact on each one's list, -1: none
+    double n[3], w[3], a[3];
+    double post, ms, rms;  // rms = 1 / ms
+    double den, rden;      // 2 I / den is the impulse; rden = 1 / den
+    double thr, ir0;       // velocity below which it repels, bound of that impulse
+};
+__device__ __forceinline__ Impulse impulse_of(const CollideCounts &c, const PtContact *pt,
+                                              const EeContact *ee, int i, const int4 *cverts,
+                                              const int4 *csucc, const double *mass, double dt,
+                                              double K)
+{
+    const double scale = double(0.1f);
+    const int4 cv = cverts[i];
+    Impulse r;
+    r.v = cv;
+    r.succ = csucc[i];
+    double d;
     if (i < c.n_ee)
     {
         const EeContact &e = ee[i];
         const float a = e.s, b = e.t, a1 = 1 - a;
-        const int v0 = v[0], v1 = v[1];
-        double vrel[3];
         for (int k = 0; k < 3; k++)
-            vrel[k] = (double(a1) * dxr[3 * size_t(v0) + k] + double(a) * dxr[3 * size_t(v1) + k]) /
-                      dt;
-        const double ms = mass[v0] + mass[v1];
-        const double vn = vrel[0] * e.n[0] + vrel[1] * e.n[1] + vrel[2] * e.n[2];
-        const double Ic = vn > v_thre ? 0 : ms * fabs(vn) / 2;
-        const double d = 3e-3 - double(e.depth);
-        double Ir = 0;
-        if (!(vn > double(0.1f) * d / dt))
-        {
-            const double Ir0 = dt * K * d, Ir1 = ms * (double(0.1f) * d / dt - vn);
-            Ir = Ir0 < Ir1 ? Ir0 : Ir1;
-        }
-        const double I = Ic + Ir;
+            r.n[k] = e.n[k];
+        r.w[0] = double(a1);
+        r.w[1] = double(a);
+        r.w[2] = 0.0;
+        r.ms = mass[cv.x] + mass[cv.y];
+        d = 3e-3 - double(e.depth);
+        r.thr = double(0.1f) * d / dt;
         const float den = 1 + a * a + (1 - a) * (1 - a) + b * b + (1 - b) * (1 - b);
-        const double It = 2 * I / double(den);
-        for (int k = 0; k < 3; k++)
-        {
-            dxr[3 * size_t(v0) + k] += scale * dt * double(a1) * It / ms * e.n[k];
-            dxr[3 * size_t(v1) + k] += scale * dt * double(a) * It / ms * e.n[k];
-        }
-        return;
-    }
-    const PtContact &p = pt[i - c.n_ee];
-    double vrel[3], ms;
-    const double bw[3] = {p.bary[0], p.bary[1], p.bary[2]};
-    if (p.cloth_point)
-    {
-        for (int k = 0; k < 3; k++)
-            vrel[k] = dxr[3 * size_t(v[0]) + k] / dt;
-        ms = mass[v[0]];
-    }
-    else
-    {
-        for (int k = 0; k < 3; k++)
-            vrel[k] = (dxr[3 * size_t(v[0]) + k] * bw[0] + dxr[3 * size_t(v[1]) + k] * bw[1] +
-                       dxr[3 * size_t(v[2]) + k] * bw[2]) /
-                      dt;
-        ms = mass[v[0]] + mass[v[1]] + mass[v[2]];
-    }
-    const double vn = vrel[0] * p.n[0] + vrel[1] * p.n[1] + vrel[2] * p.n[2];
-    const double Ic = vn > v_thre ? 0 : ms * fabs(vn) / 2;
-    const double d = 3e-3 - double(p.depth);
-    double Ir = 0;
-    if (!(vn > 0.1 * d / dt))
-    {
-        const double Ir0 = dt * K * d, Ir1 = ms * (0.1 * d / dt - vn);
-        Ir = Ir0 < Ir1 ? Ir0 : Ir1;
-    }
-    const double I = Ic + Ir;
-    const double It = 2 * I / (1 + (bw[0] * bw[0] + bw[1] * bw[1] + bw[2] * bw[2]));
-    if (p.cloth_point)
-        for (int k = 0; k < 3; k++)
-            dxr[3 * size_t(v[0]) + k] += scale * (dt * It / ms * p.n[k]);
-    else
+        r.den = double(den);
         for (int j = 0; j < 3; j++)
-            for (int k = 0; k < 3; k++)
-                dxr[3 * size_t(v[j]) + k] += scale * (dt * bw[j] * It / ms * p.n[k]);
+            r.a[j] = scale * dt * r.w[j];
+        r.post = 1.0;
+    }
+    else
+    {
+        const PtContact &p = pt[i - c.n_ee];
+        const double bw[3] = {p.bary[0], p.bary[1], p.bary[2]};
+        for (int k = 0; k < 3; k++)
+            r.n[k] = p.n[k];
+        d = 3e-3 - double(p.depth);
+        r.thr = 0.1 * d / dt;
+        r.den = 1 + (bw[0] * bw[0] + bw[1] * bw[1] + bw[2] * bw[2]);
+        r.post = scale;
+        r.ms = mass[cv.x];
+        for (int j = 0; j < 3; j++)
+        {
+            r.w[j] = p.cloth_point ? (j == 0 ? 1.0 : 0.0) : bw[j];
+            r.a[j] = dt * r.w[j];
+        }
+        if (!p.cloth_point)
+            r.ms = r.ms + mass[cv.y] + mass[cv.z];
+    }
+    r.ir0 = dt * K * d;
+    r.rms = 1.0 / r.ms;
+    r.rden = 1.0 / r.den;
+    return r;
 }
 
+// a / b, correctly rounded, given y = 1 / b correctly rounded: the remainder of a
+// quotient, exact in one fused multiply-add, times y corrects it; the correction of
+// a quotient within a unit in the last place rounds correctly (Markstein 1990), and
+// a first one brings a * y there.  Outside its conditions (a tiny, huge or not
+// finite operand or quotient) the division itself, except that a zero over a plain
+// divisor is a zero of the product's sign.
+__device__ __forceinline__ double quotient(double a, double b, double y)
+{
+    const double q0 = a * y;
+    double q = fma(fma(-q0, b, a), y, q0);
+    q = fma(fma(-q, b, a), y, q);
+    auto plain = [](double v) {
+        return unsigned(((__double2hiint(v) >> 20) & 0x7ff) - 200) < 1600u;
+    };
+    if (!(plain(q) && plain(a)) || !(plain(b) && plain(y)))
+    {
+        const bool zero = (__double_as_longlong(a) << 1) == 0;
+        q = zero && plain(b) && plain(y) ? q0 : a / b;
+    }
+    return q;
+}
 
+constexpr unsigned kRepSmem = kRepStaged * sizeof(Impulse) + kRepFields / 4;
+
+// Every contact's Impulse (as many as there is room for), so that the divisions,
+// gathers and conversions that need no dxr are out of the repulsion's serial chain.
+__global__ void k_col_rep_prep(const CollideCounts *cnt, int cap_pt, int cap_ee,
+                               const PtContact *pt, const EeContact *ee, const int4 *cverts,
+                               const int4 *csucc, const double *mass, double dt, double K,
+                               Impulse *rec, int cap_rec)
+{
+    CollideCounts c = *cnt;
+    c.n_pt = min(c.n_pt, cap_pt);
+    c.n_ee = min(c.n_ee, cap_ee);
+    const int n = min(c.n_pt + c.n_ee, cap_rec);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        rec[i] = impulse_of(c, pt, ee, i, cverts, csucc, mass, dt, K);
+}
 
 // Repulsion (BaraffCloth.cpp:626-926) in rounds: a contact runs when it heads
 // the list of every vertex it touches (every earlier contact there has run),
 // so the contacts of one round share no vertex and the result is that of the
-// sequential loop.  The first round's contacts come from a scan of all; after
-// that only the new heads of the vertices a round touched can become ready,
-// so each round visits just those (work lists wa / wb, a queued flag per
-// contact).
+// sequential loop.  Each contact counts the lists that it does not head yet; one
+// that runs counts its successors down, and the last count puts a contact on the
+// next round's work list (wa / wb in turn, their first kRepList entries in shared
+// memory).  The counts are 2-bit fields in shared memory while there is room for
+// every contact, else words (cstate).
+//
+// A round is one serial chain for a handful of contacts, bound by the FP64 pipe: a
+// warp's FP64 instruction takes it the same time for one lane as for 32.  So four
+// lanes take a contact (lane k the component k of its velocity and changes, and
+// the quotient of vertex k), the divisions by what a contact has from the start are
+// multiplications by its reciprocal with exact corrections, both kinds of contacts
+// run the same instructions, and a round has one barrier.  REP_FIGURES
 __global__ void __launch_bounds__(kRepBlock) k_col_repulse(
     const CollideCounts *cnt_in, int cap_pt, int cap_ee, const PtContact *pt, const EeContact *ee,
-    const int4 *cverts, const int4 *clpos, const int4 *csucc, const double *mass, int *rptr,
-    int *queued, int *wa, int *wb, double *dxr, double dt, double K, CollideCounts *cw)
+    const int4 *cverts, const int4 *clpos, const int4 *csucc, const double *mass, int *cstate,
+    int *wa, int *wb, double *dxr, double dt, double K, const Impulse *rec, int cap_rec,
+    CollideCounts *cw)
 {
-    __shared__ int s_na, s_nb, s_done;
+    extern __shared__ __align__(16) unsigned char s_mem[];
+    Impulse *s_rec = reinterpret_cast<Impulse *>(s_mem);
+    unsigned *s_field = reinterpret_cast<unsigned *>(s_mem + kRepStaged * sizeof(Impulse));
+    __shared__ int s_list[2][kRepList];
+    __shared__ int s_n[3];
     CollideCounts c = *cnt_in;
     c.n_pt = min(c.n_pt, cap_pt);
     c.n_ee = min(c.n_ee, cap_ee);
     const int n = c.n_pt + c.n_ee;
-    // contact i heads all its lists when every vertex has run exactly the
-    // contacts before it there
-    auto ready = [&](int i) {
-        const int4 cv = cverts[i], lp = clpos[i];
-        bool r = rptr[cv.x] == lp.x;
-        if (cv.w > 1)
-            r = r && rptr[cv.y] == lp.y;
-        if (cv.w > 2)
-            r = r && rptr[cv.z] == lp.z;
-        return r;
-    };
-    if (threadIdx.x == 0)
+    const double rdt = 1.0 / dt;
+    const int lane = threadIdx.x & 31, part = lane & 3, comp = min(part, 2);
+    const bool fields = n <= kRepFields;
+    const int staged = min(n, min(cap_rec, kRepStaged));
+    if (fields)
+        for (int i = threadIdx.x; i < (n + 15) / 16; i += blockDim.x)
+            s_field[i] = 0u;
+    if (threadIdx.x < 3)
+        s_n[threadIdx.x] = 0;
     {
-        s_na = 0;
-        s_nb = 0;
-        s_done = 0;
+        const int4 *src = reinterpret_cast<const int4 *>(rec);
+        int4 *dst = reinterpret_cast<int4 *>(s_rec);
+        for (int i = threadIdx.x; i < staged * int(sizeof(Impulse) / 16); i += blockDim.x)
+            dst[i] = src[i];
     }
     __syncthreads();
+    auto push = [&](int b, int to, int i) {
+        const int k = atomicAdd(&s_n[to], 1);
+        if (k < kRepList)
+            s_list[b][k] = i;
+        else if (k < n)
+            (b ? wb : wa)[k] = i;
+    };
     for (int i = threadIdx.x; i < n; i += blockDim.x)
-        if (ready(i))
-        {
-            queued[i] = 1;
-            wa[atomicAdd(&s_na, 1)] = i;
-        }
-    __syncthreads();
-    int rounds = 0;
-    int *cur = wa, *nxt = wb;
-    while (s_na > 0 && rounds <= n)
     {
-        const int na = s_na;
-        // run this round's contacts (vertex-disjoint), then move their
-        // vertices past them
-        for (int k = threadIdx.x; k < na; k += blockDim.x)
-        {
-            const int i = cur[k];
-            const int4 cv = cverts[i];
-            const int v[3] = {cv.x, cv.y, cv.z};
-            repulse_one(c, pt, ee, i, v, mass, dxr, dt, K);
-            for (int q = 0; q < cv.w; q++)
-                rptr[v[q]]++;
-        }
+        const int4 lp = clpos[i];
+        const int m = cverts[i].w;
+        const int wait = (lp.x != 0) + (m > 1 && lp.y != 0) + (m > 2 && lp.z != 0);
+        if (fields)
+            atomicOr(&s_field[i >> 4], unsigned(wait) << (2 * (i & 15)));
+        else
+            cstate[i] = wait;
+        if (wait == 0)
+            push(0, 0, i);
+    }
+    __syncthreads();
+    int rounds = 0, done = 0;
+    for (;;)
+    {
+        const int now = rounds % 3, to = (rounds + 1) % 3, b = rounds & 1;
+        const int na = min(s_n[now], n);
+        if (na == 0 || done >= n)
+            break;
         if (threadIdx.x == 0)
+            s_n[(rounds + 2) % 3] = 0;
+        for (int k0 = (threadIdx.x >> 5) * 8; k0 < na; k0 += kRepBlock / 4)
         {
-            s_done += na;
-            s_nb = 0;
-        }
-        __syncthreads();
-        // their successors that now head all their lists
-        for (int k = threadIdx.x; k < na; k += blockDim.x)
-        {
-            const int i = cur[k];
-            const int4 sc = csucc[i];
-            const int m = cverts[i].w;
-            const int su[3] = {sc.x, sc.y, sc.z};
-            for (int q = 0; q < m; q++)
+            const int k = min(k0 + (lane >> 2), na - 1);
+            const bool live = k0 + (lane >> 2) < na;
+            const int i = k < kRepList ? s_list[b][k] : (b ? wb : wa)[k];
+            Impulse made;
+            const Impulse *m = s_rec + i;
+            if (i >= staged)
             {
-                const int h = su[q];
-                if (h >= 0 && ready(h) && atomicExch(&queued[h], 1) == 0)
-                    nxt[atomicAdd(&s_nb, 1)] = h;
+                m = rec + i;
+                if (i >= cap_rec)
+                {
+                    made = impulse_of(c, pt, ee, i, cverts, csucc, mass, dt, K);
+                    m = &made;
+                }
+            }
+            const int4 v = m->v;
+            const bool two = v.w > 1, three = v.w > 2;
+            const double *px = dxr + 3 * size_t(v.x) + comp;
+            const double *py = dxr + 3 * size_t(two ? v.y : v.x) + comp;
+            const double *pz = dxr + 3 * size_t(three ? v.z : v.x) + comp;
+            const double x0 = *px, x1 = *py, x2 = *pz;
+            // the next contacts' counts: they run after the barrier
+            if (live && part < v.w)
+            {
+                const int4 sc = m->succ;
+                const int h = part == 0 ? sc.x : part == 1 ? sc.y : sc.z;
+                if (unsigned(h) < unsigned(n))
+                {
+                    const int sh = 2 * (h & 15);
+                    const int left = fields
+                                         ? int(atomicSub(&s_field[h >> 4], 1u << sh) >> sh & 3u)
+                                         : atomicSub(&cstate[h], 1);
+                    if (left == 1)
+                        push(b ^ 1, to, h);
+                }
+            }
+            double t = m->w[0] * x0;
+            const double t2 = t + m->w[1] * x1;
+            t = two ? t2 : t;
+            const double t3 = t + m->w[2] * x2;
+            t = three ? t3 : t;
+            const double n_k = m->n[comp];
+            const double p = quotient(t, dt, rdt) * n_k;
+            const int g = lane & ~3;
+            const double vn = __shfl_sync(0xffffffffu, p, g) + __shfl_sync(0xffffffffu, p, g + 1) +
+                              __shfl_sync(0xffffffffu, p, g + 2);
+            const double v_thre = 0.01, ms = m->ms, thr = m->thr;
+            const double Ic = vn > v_thre ? 0 : ms * fabs(vn) / 2;
+            double Ir = 0;
+            if (!(vn > thr))
+            {
+                const double Ir0 = m->ir0, Ir1 = ms * (thr - vn);
+                Ir = Ir0 < Ir1 ? Ir0 : Ir1;
+            }
+            const double I = Ic + Ir;
+            const double It = quotient(2 * I, m->den, m->rden);
+            const double q = quotient(m->a[comp] * It, ms, m->rms);
+            const double q0 = __shfl_sync(0xffffffffu, q, g), q1 = __shfl_sync(0xffffffffu, q, g + 1),
+                         q2 = __shfl_sync(0xffffffffu, q, g + 2);
+            const double post = m->post;
+            if (live && part < 3)
+            {
+                const double y0 = x0 + post * (q0 * n_k), y1 = x1 + post * (q1 * n_k),
+                             y2 = x2 + post * (q2 * n_k);
+                dxr[3 * size_t(v.x) + comp] = y0;
+                if (two)
+                    dxr[3 * size_t(v.y) + comp] = y1;
+                if (three)
+                    dxr[3 * size_t(v.z) + comp] = y2;
             }
         }
-        __syncthreads();
-        if (threadIdx.x == 0)
-            s_na = s_nb;
-        int *t = cur;
-        cur = nxt;
-        nxt = t;
+        done += na;
         rounds++;
         __syncthreads();
     }
     if (threadIdx.x == 0)
     {
         cw->rounds = rounds;
-        if (s_done != n)
+        if (done != n)
             cw->overflow = 1; // a contact never headed its lists (a lost list entry)
     }
 }
@@ -1328,6 +1424,8 @@ int collide_alloc(cloth_s *c)
         c->ctx->bytes -= w->bytes;
         w->mem = nullptr;
     }
+    CCK(cudaFuncSetAttribute(k_col_repulse, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             int(kRepSmem)));
     const int nlist = std::max(std::max(nv, ne), max_bnv);
     Layout L;
     const size_t o_ctlo = L.take<double>(3 * size_t(nt)), o_cthi = L.take<double>(3 * size_t(nt)),
@@ -1337,7 +1435,7 @@ int collide_alloc(cloth_s *c)
                  o_lst = L.take<int>(size_t(nlist) + 1), o_pt = L.take<PtContact>(size_t(cap_pt)),
                  o_ee = L.take<EeContact>(size_t(cap_ee)),
                  o_incoff = L.take<int>(size_t(nv) + 1), o_inccur = L.take<int>(size_t(nv)),
-                 o_inc = L.take<int>(size_t(cap_inc)), o_rptr = L.take<int>(size_t(nv)),
+                 o_inc = L.take<int>(size_t(cap_inc)),
                  o_cst = L.take<int>(size_t(cap_pt + cap_ee)),
                  o_wa = L.take<int>(size_t(cap_pt + cap_ee)), o_wb = L.take<int>(size_t(cap_pt + cap_ee)),
                  o_dxr = L.take<double>(3 * size_t(nv)),
@@ -1372,7 +1470,6 @@ int collide_alloc(cloth_s *c)
     w->inc_off = reinterpret_cast<int *>(base + o_incoff);
     w->inc_cur = reinterpret_cast<int *>(base + o_inccur);
     w->inc = reinterpret_cast<int *>(base + o_inc);
-    w->rptr = reinterpret_cast<int *>(base + o_rptr);
     w->cstate = reinterpret_cast<int *>(base + o_cst);
     w->wa = reinterpret_cast<int *>(base + o_wa);
     w->wb = reinterpret_cast<int *>(base + o_wb);
@@ -1533,11 +1630,16 @@ int cloth::detail::collide_repulse(cloth_s *c)
     const int nv = c->tab.nv;
     const float kmean = ((c->mat.stretch_k[0] + c->mat.stretch_k[1]) + c->mat.stretch_k[2]) / 3.0f;
     const double K = double(kmean) * 1;
-    k_col_dxr<<<grid_blocks(ctx, std::max(nv, w->cap_pt + w->cap_ee)), kColBlock, 0, s>>>(
-        nv, c->h.dx, w->dxr, w->rptr, w->cap_pt + w->cap_ee, w->cstate);
-    k_col_repulse<<<1, kRepBlock, 0, s>>>(w->cnt, w->cap_pt, w->cap_ee, w->pt, w->ee,
-                                          w->cverts, w->clpos, w->csucc, w->mass64, w->rptr,
-                                          w->cstate, w->wa, w->wb, w->dxr, c->dt_set, K, w->cnt);
+    k_col_dxr<<<grid_blocks(ctx, nv), kColBlock, 0, s>>>(nv, c->h.dx, w->dxr);
+    // (the pair list is free until the next detection)
+    Impulse *rec = reinterpret_cast<Impulse *>(w->tp);
+    const int cap_rec = int(size_t(w->cap_pairs) * sizeof(int) / sizeof(Impulse));
+    k_col_rep_prep<<<grid_blocks(ctx, std::max(w->cap_pt, w->cap_ee)), kColBlock, 0, s>>>(
+        w->cnt, w->cap_pt, w->cap_ee, w->pt, w->ee, w->cverts, w->csucc, w->mass64, c->dt_set, K,
+        rec, cap_rec);
+    k_col_repulse<<<1, kRepBlock, kRepSmem, s>>>(
+        w->cnt, w->cap_pt, w->cap_ee, w->pt, w->ee, w->cverts, w->clpos, w->csucc, w->mass64,
+        w->cstate, w->wa, w->wb, w->dxr, c->dt_set, K, rec, cap_rec, w->cnt);
     CCK(cudaGetLastError());
     return CLOTH_OK;
 }
