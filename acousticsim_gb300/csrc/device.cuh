@@ -65,6 +65,27 @@ struct EeContact
 // point-triangle index with this bit set (so a sorted list runs in the
 // reference's repulsion order: edge-edge contacts first).
 constexpr int kPtTag = 0x40000000;
+// A point-triangle contact's Hessian blocks (xx xy xz yy yz zz) by pairs of its cloth
+// vertices: 00 01 02 11 12 22.
+struct alignas(16) ContactHess
+{
+    int4 v; // cloth vertices (-1: none) and their count
+    float h[6][6];
+};
+#ifdef __CUDACC__
+// One such block: 1e-2 (w_i N)(w_j N)^T, the two orders of its factors averaged.
+__device__ __forceinline__ void contact_block(double wi, double wj, const double *n, float *h)
+{
+    const int pa[6] = {0, 0, 0, 1, 1, 2}, pb[6] = {0, 1, 2, 1, 2, 2};
+#pragma unroll
+    for (int q = 0; q < 6; q++)
+    {
+        const double u = (wi * n[pa[q]]) * (wj * n[pb[q]]);
+        const double v = (wi * n[pb[q]]) * (wj * n[pa[q]]);
+        h[q] = float(1e-2 * (0.5 * (u + v)));
+    }
+}
+#endif
 struct CollideCounts
 {
     int n_pt, n_ee;   // contacts so far
@@ -157,6 +178,8 @@ struct InstDesc
     const int *cinc_off;  // nv+1 per-vertex contact list ranges
     const int *cinc;      // per-vertex contact lists (sorted)
     const CollideCounts *ccount;
+    const ContactHess *chess; // blocks of the first n_chess point-triangle contacts
+    long long n_chess;
     double *dxr;          // nv*3: dx after the repulsion (FP64), used by the advance
     float4 *M0; // block-Jacobi inverse, symmetric: (00 01 02 11)
     float2 *M1; // (12 22)

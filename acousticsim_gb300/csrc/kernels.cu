@@ -466,7 +466,22 @@ __global__ void __launch_bounds__(kTile) k_row(InstDesc *const *descs,
             const int len = info & 255, ds = (info >> 8) & 255;
             const float4 xv = d.x32[row];
             const bool fixv = xv.w != 0.f;
-            const int ncinc = d.ccount ? d.ccount->cap_inc : 0;
+            // the row's point-triangle contacts: the end of its (ascending) list
+            int cpt0 = 0, cpt1 = 0;
+            if (d.cinc_off)
+            {
+                const int ncinc = d.ccount ? d.ccount->cap_inc : 0;
+                cpt0 = d.cinc_off[row];
+                cpt1 = min(d.cinc_off[row + 1], ncinc);
+                for (int e = cpt1; cpt0 < e;)
+                {
+                    const int mid = (cpt0 + e) >> 1;
+                    if (d.cinc[mid] & kPtTag)
+                        e = mid;
+                    else
+                        cpt0 = mid + 1;
+                }
+            }
             const float m = d.mass[row];
             float3 f = make_float3(0, 0, 0);
             for (int k = d.fptr[row]; k < d.fptr[row + 1]; k++)
@@ -520,57 +535,63 @@ __global__ void __launch_bounds__(kTile) k_row(InstDesc *const *descs,
                     A[k] = d.c_stiff * K[k];
                 float4 Aw = make_float4(d.c_stiff * wv[0], d.c_stiff * wv[1], d.c_stiff * wv[2],
                                         0.f);
-                // contact Hessian (PrepareCollisionHessian, BaraffCloth.cpp:928-990):
-                // 1e-2 (w_i N)(w_j N)^T per point-triangle contact holding row
-                // and c, w = 1 at a cloth point, -b at a cloth triangle's
-                // vertices; added to the system matrix unscaled, formed
-                // symmetrically so both rows of a pair hold the same block
+                // contact Hessian (PrepareCollisionHessian, BaraffCloth.cpp:928-990): a
+                // block per point-triangle contact holding row and c, added to the
+                // system matrix unscaled
                 float Hc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-                if (d.cinc_off)
-                    for (int k = d.cinc_off[row]; k < min(d.cinc_off[row + 1], ncinc); k++)
+                for (int k = cpt0; k < cpt1; k++)
+                {
+                    const int ci = d.cinc[k] & ~kPtTag;
+                    if (ci < d.n_chess)
                     {
-                        const int tag = d.cinc[k];
-                        if (!(tag & kPtTag))
+                        const ContactHess &ch = d.chess[ci];
+                        const int4 v = ch.v;
+                        const int i = v.z == row ? 2 : v.y == row ? 1 : 0;
+                        const int j = v.z == c ? 2 : v.y == c ? 1 : v.x == c ? 0 : -1;
+                        if (j < 0)
                             continue;
-                        const PtContact &pc = d.cpt[tag & ~kPtTag];
-                        double wi = 0.0, wj = 0.0;
-                        bool hit = false;
-                        if (pc.cloth_point)
+                        const int lo = min(i, j), hi = max(i, j);
+                        const float *h = ch.h[lo + hi + (lo > 0)];
+#pragma unroll
+                        for (int q = 0; q < 6; q++)
+                            Hc[q] += h[q];
+                        continue;
+                    }
+                    const PtContact &pc = d.cpt[ci];
+                    double wi = 0.0, wj = 0.0;
+                    bool hit = false;
+                    if (pc.cloth_point)
+                    {
+                        if (c == row)
                         {
-                            if (c == row)
+                            wi = wj = 1.0;
+                            hit = true;
+                        }
+                    }
+                    else
+                    {
+                        const int4 tv = d.tri[pc.t];
+                        const int vv[3] = {tv.x, tv.y, tv.z};
+#pragma unroll
+                        for (int q = 0; q < 3; q++)
+                        {
+                            if (vv[q] == row)
+                                wi = -double(pc.bary[q]);
+                            if (vv[q] == c)
                             {
-                                wi = wj = 1.0;
+                                wj = -double(pc.bary[q]);
                                 hit = true;
                             }
                         }
-                        else
-                        {
-                            const int4 tv = d.tri[pc.t];
-                            const int vv[3] = {tv.x, tv.y, tv.z};
-#pragma unroll
-                            for (int q = 0; q < 3; q++)
-                            {
-                                if (vv[q] == row)
-                                    wi = -double(pc.bary[q]);
-                                if (vv[q] == c)
-                                {
-                                    wj = -double(pc.bary[q]);
-                                    hit = true;
-                                }
-                            }
-                        }
-                        if (!hit)
-                            continue;
-                        const double N[3] = {pc.n[0], pc.n[1], pc.n[2]};
-                        const int pa[6] = {0, 0, 0, 1, 1, 2}, pb[6] = {0, 1, 2, 1, 2, 2};
-#pragma unroll
-                        for (int q = 0; q < 6; q++)
-                        {
-                            const double u = (wi * N[pa[q]]) * (wj * N[pb[q]]);
-                            const double v = (wi * N[pb[q]]) * (wj * N[pa[q]]);
-                            Hc[q] += float(1e-2 * (0.5 * (u + v)));
-                        }
                     }
+                    if (!hit)
+                        continue;
+                    float h[6];
+                    contact_block(wi, wj, pc.n, h);
+#pragma unroll
+                    for (int q = 0; q < 6; q++)
+                        Hc[q] += h[q];
+                }
                 bool zero = false;
                 if (s == ds)
                 {
