@@ -62,7 +62,7 @@ namespace detail {
 struct PersistLaunch
 {
     const void *func = nullptr;
-    bool on_chip = false; // k_pcg_team or k_pcg_half (their arguments)
+    bool on_chip = false; // k_pcg_team, k_pcg_half or k_pcg_wide (their arguments)
     int cluster = 0;      // teams are clusters of this many blocks (0: all blocks resident)
     int grid = 0, block = 0;
     size_t smem = 0;
@@ -902,12 +902,13 @@ TeamBlock team_block(const Tables &t, int inst, int rank, int r0, int r1)
     return w;
 }
 
-// An on-chip kernel: k_pcg_team or k_pcg_half (half) with K rows a thread (0:
-// one, without blocks in registers).
+// An on-chip kernel: k_pcg_team or (half) k_pcg_half, or above four k_pcg_wide, with
+// K rows a thread (0: one, without blocks in registers).
 struct TeamKernel
 {
     int K;
     bool half;
+    bool wide() const { return half && K > 4; }
 };
 
 // Adds cloth c as instance i to an on-chip kernel's work list in at most `blocks`
@@ -922,7 +923,7 @@ bool team_split(const cloth_s *c, int i, bool skew_kernel, int blocks, TeamKerne
     const size_t first = work.size();
     const int rows =
         ((t.nv + blocks - 1) / blocks + kRedRows - 1) / kRedRows * kRedRows;
-    if (rows > std::max(tk.K, 1) * kTeamWorkers || (tk.half && h.width_up > 15))
+    if (rows > std::max(tk.K, 1) * kTeamWorkers || (tk.half && !tk.wide() && h.width_up > 15))
         return false;
     size_t most = 0;
     for (int r0 = 0; r0 < t.nv; r0 += rows)
@@ -932,7 +933,9 @@ bool team_split(const cloth_s *c, int i, bool skew_kernel, int blocks, TeamKerne
         const int halo = w.halo1 - w.halo0, nr = w.row1 - w.row0;
         size_t bytes = 0;
         bool fits = halo <= 65535;
-        if (tk.half)
+        if (tk.wide())
+            bytes = wide_smem_bytes(halo, nr, tk.K);
+        else if (tk.half)
         {
             // as many planes of stored blocks as fit: all, or those from the
             // first upper one on (the diagonal's serves no lower slot)
@@ -1198,9 +1201,9 @@ int plan_persistent(cloth_ctx *ctx, Batch *b)
         if (most <= kClusterMax * kTeamWorkers && plan_queue(ctx, b, &rc))
             return rc;
         // Teams over the whole GPU: the whole matrix on chip where it fits (256^2:
-        // 4.2 us with one row a thread), else the stored blocks (300^2: 6.8, the
-        // kernel that reads the matrix from L2 13.0; 512^2: 15.8 and 21.4), with
-        // as few rows a thread as hold the set (362^2: 7.8 with two, 8.6 with
+        // 4.2 us with one row a thread), else the stored blocks (300^2: 6.4, the
+        // kernel that reads the matrix from L2 13.0; 512^2: 13.8 and 21.4), with
+        // as few rows a thread as hold the set (362^2: 7.3 with two, 8.6 with
         // three)
         for (TeamKernel k : {one, TeamKernel{1, false}, TeamKernel{2, false}, TeamKernel{2, true},
                              TeamKernel{3, true}, TeamKernel{4, true}})
@@ -1208,6 +1211,13 @@ int plan_persistent(cloth_ctx *ctx, Batch *b)
                 return add_launch(b, l, work, sizeof(TeamSync), alignof(TeamSync) * 64);
         if (plan_queue(ctx, b, &rc))
             return rc;
+        // The matrix read from memory, with as few rows a thread as hold the set
+        // (640^2: 26.6 us per iteration, the older kernel 44.4; 760^2: 48.3 and 59.7;
+        // with 15 rows a thread 900^2: 75.7 and 84.1, 1024^2: 99.7 and 100.3)
+        if (!b->skew)
+            for (int k : {kWideRows, kWidestRows})
+                if (plan_team(ctx, b, TeamKernel{k, true}, work, l))
+                    return add_launch(b, l, work, sizeof(TeamSync), alignof(TeamSync) * 64);
     }
     work.clear();
     const size_t smem_cap_bytes =

@@ -321,6 +321,15 @@ __host__ __device__ inline size_t half_smem_bytes(int halo, int rows, int ext, i
     return size_t(half_p_quads(halo) + (cluster ? halo - rows : 0)) * 16 +
            size_t(planes) * (rp + ext) * (skew ? 40 : 24) + size_t(words) * rp * 2;
 }
+// k_pcg_wide: rows per thread of its two variants (the first holds dx and the inverse
+// diagonal blocks on chip), and a block's dynamic shared memory.
+constexpr int kWideRows = 8, kWidestRows = 15;
+__host__ __device__ constexpr bool wide_hold(int k) { return k <= kWideRows; }
+__host__ __device__ inline size_t wide_smem_bytes(int halo, int rows, int k)
+{
+    return size_t(half_p_quads(halo)) * 16 +
+           size_t((rows + 31) / 32) * 32 * (wide_hold(k) ? 36 : 12);
+}
 // A team that is one thread-block cluster: its most blocks, and a block whose
 // halo holds rows [row0, row1) of this one (row i of z goes to z + 16 i in the
 // cluster's shared memory, counted on its barrier bar).

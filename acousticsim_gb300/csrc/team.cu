@@ -25,7 +25,7 @@
 // Measured (one GB300, us per PCG iteration over a whole step, before: the
 // kernel that reads the matrix from L2 and forms the scalars in FP64): 16x16
 // 13.1 -> 2.2, 64x64 12.2 -> 2.6, 97x61 11.8 -> 3.3, 193x255 12.4 -> 4.0,
-// 256x256 12.7 -> 4.2, 512x512 21.5 -> 15.8, 128x128 with dihedral bending
+// 256x256 12.7 -> 4.2, 512x512 21.5 -> 13.8, 128x128 with dihedral bending
 // 14.1 -> 3.8.
 #include "internal.h"
 #include "pcg_math.cuh"
@@ -175,10 +175,10 @@ __device__ __forceinline__ double value(const Raw &r)
     return fx_value((unsigned long long)r.hi << 16 | r.lo >> 32, r.lo & 0xffffffffull, r.s);
 }
 
-// Adds 32-row chunks' FP32 sums to the block's digits, one sum per group of 8
-// lanes (v, its scale s and its quantity's digits dig[0 .. 3] are theirs; dig[4]
-// counts sums out of range).
-__device__ __forceinline__ void chunk_add(int *dig, float v, int s, bool on)
+// A 32-row chunk's FP32 sum as digits, one sum per group of 8 lanes (v and its scale
+// s are theirs): lane j's part of digit j, lane 4 counting sums out of range; false
+// where the lane has none.
+__device__ __forceinline__ bool chunk_digit(float v, int s, int &x)
 {
     const unsigned bits = __float_as_uint(v);
     const int e = int((bits >> 23) & 0xffu), j = threadIdx.x & 7;
@@ -200,17 +200,40 @@ __device__ __forceinline__ void chunk_add(int *dig, float v, int s, bool on)
         sh = min(sh, 71);
     }
     const int k = (sh * 43) >> 10, off = sh - 24 * k; // sh / 24, sh % 24
-    int x = j == k ? int((m << off) & 0xffffffu) : int(m >> (24 - off));
+    x = j == k ? int((m << off) & 0xffffffu) : int(m >> (24 - off));
     const int sign = int(bits) >> 31;
     x = (x ^ sign) - sign;
-    bool add = on && unsigned(j - k) < 2u;
+    bool has = unsigned(j - k) < 2u;
     if (bad)
     {
         x = 1;
-        add = on && j == 4;
+        has = j == 4;
     }
-    if (add)
-        atomicAdd(dig + j, x);
+    return has;
+}
+// Adds the sums to the block's digits dig[0 .. 4] of their quantity.
+__device__ __forceinline__ void chunk_add(int *dig, float v, int s, bool on)
+{
+    int x;
+    if (chunk_digit(v, s, x) && on)
+        atomicAdd(dig + (threadIdx.x & 7), x);
+}
+// Adds the digits that groups of 8 lanes gathered (up to 16 chunks a warp) to the
+// block's: the low ones carried first, a top one that 15 warps could sum out of 32
+// bits counted as out of range.
+__device__ __forceinline__ void digits_add(int *dig, int d, bool on)
+{
+    const int j = threadIdx.x & 7;
+    const int c = j < 3 ? d >> 24 : 0;
+    const int below = __shfl_up_sync(kFull, c, 1);
+    if (j < 3)
+        d &= 0xffffff;
+    if (j >= 1 && j <= 3)
+        d += below;
+    if (on && j == 3 && (d >= 1 << 27 || d <= -(1 << 27)))
+        atomicAdd(dig + 4, 1);
+    if (on && j < 5 && d != 0)
+        atomicAdd(dig + j, d);
 }
 // The sums of a warp's K chunks (the same in every lane; zero where it has
 // none): p.q.
@@ -1666,6 +1689,413 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
         cluster_sync();
 }
 
+// The same solve for blocks with more rows than k_pcg_half takes, the matrix read
+// from memory (sets without skew parts).  On chip are p over the halo and q, then z,
+// in one place of shared memory, r in registers, and up to kWideRows rows a thread dx
+// in registers and the inverse diagonal blocks in shared memory as well.  z goes to
+// memory only for rows that another block's columns touch.  K: most rows per thread.
+//
+// What bounds it: reading the stored blocks and the columns (220 bytes a row of a
+// grid) and the transposed rows' blocks again, from L2 and past ~650^2 from HBM, by as
+// many warps as the registers allow.  So a warp has a group's loads in flight
+// together: the upper planes' addresses need no column, and a chunk's lower references
+// are fetched one chunk ahead.  (Groups of 4 spill: 640^2 28.0 us, 26.6 with 3; two
+// groups in flight in turn cost more instructions than the latency they hide: 52.0.)
+// us per iteration, before (k_pcg_persistent_gm): 545^2 27.5 -> 18.9, 640^2 44.4 ->
+// 26.6, 760^2 59.7 -> 48.3, 900^2 84.1 -> 75.7, 1024^2 100.3 -> 99.7.
+template <int K>
+__global__ void __launch_bounds__(kTeamThreads, 1)
+    k_pcg_wide(InstDesc *const *descs, const TeamBlock *work, TeamSync *sync, SpinCfg sc)
+{
+    constexpr int kAll = kTeamThreads;
+    constexpr bool kHold = wide_hold(K); // dx and the inverse diagonal blocks on chip
+    extern __shared__ float4 sm_dyn[];
+    __shared__ InstDesc d;
+    __shared__ int s_dig[3][8];
+    __shared__ int s_scale[3];
+    __shared__ Shared<false> sh;
+    const TeamBlock w = work[blockIdx.x];
+    if (!team_begin(descs, w, d, sh))
+        return;
+    InstState *st = d.st;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, grp = lane >> 3;
+    const int nrow = w.row1 - w.row0, nch = (nrow + 31) >> 5, rp = nch << 5;
+    const int nh = w.halo1 - w.halo0, nhalo = nh - nrow;
+    const bool multi = w.nblk > 1 || sc.extra != 0u;
+    const int it0 = __ldcg(&st->iter);
+    const int wl = d.width_lo, wu = d.width_up;
+    float2 *spx = reinterpret_cast<float2 *>(sm_dyn);
+    float *spz = reinterpret_cast<float *>(spx + nh);
+    auto p_get = [&](int j) {
+        const float2 v = spx[j];
+        return make_float3(v.x, v.y, spz[j]);
+    };
+    auto p_set = [&](int j, float3 v) {
+        spx[j] = make_float2(v.x, v.y);
+        spz[j] = v.z;
+    };
+    float2 *sqx = reinterpret_cast<float2 *>(sm_dyn + half_p_quads(nh));
+    float *sqz = reinterpret_cast<float *>(sqx + rp);
+    auto q_get = [&](int j) {
+        const float2 v = sqx[j];
+        return make_float3(v.x, v.y, sqz[j]);
+    };
+    auto q_set = [&](int j, float3 v) {
+        sqx[j] = make_float2(v.x, v.y);
+        sqz[j] = v.z;
+    };
+    float2 *sM = reinterpret_cast<float2 *>(sqz + rp); // three of rp
+    if (warp == kWarps)
+    {
+        control_warp<false>(d, w, sync, sc, it0, multi, sh, s_dig, s_scale);
+        return;
+    }
+    const int own0 = w.row0 - w.halo0;
+    // rows below need0 or from need1 on have readers in other blocks
+    int need0 = w.row0, need1 = w.row1;
+    for (int j = lane; j < w.nblk; j += 32)
+    {
+        const TeamBlock &o = work[int(blockIdx.x) - w.rank + j];
+        if (o.row1 <= w.row0)
+            need0 = max(need0, o.halo1);
+        else if (o.row0 >= w.row1)
+            need1 = min(need1, o.halo0);
+    }
+    need0 = __reduce_max_sync(kFull, need0);
+    need1 = __reduce_min_sync(kFull, need1);
+    float3 x[kHold ? K : 1], r[K];
+    const float4 *pold = (it0 & 1) ? d.p1 : d.p0;
+#pragma unroll
+    for (int k = 0; k < K; k++)
+    {
+        const int li = (k * kWarps + warp) * 32 + lane, row = w.row0 + li;
+        r[k] = make_float3(0.f, 0.f, 0.f);
+        if constexpr (kHold)
+            x[k] = r[k];
+        if (li < nrow)
+        {
+            r[k] = xyz(d.r[row]);
+            q_set(li, xyz(d.z[row]));
+            if constexpr (kHold)
+            {
+                x[k] = xyz(d.dx[row]);
+                const float4 m0 = d.M0[row];
+                sM[li] = make_float2(m0.x, m0.y);
+                sM[rp + li] = make_float2(m0.z, m0.w);
+                sM[2 * rp + li] = d.M1[row];
+            }
+        }
+    }
+    if (it0 > 0) // a solve handed over in its middle
+        for (int i = tid; i < nh; i += kWorkers)
+            p_set(i, xyz(__ldcg(pold + w.halo0 + i)));
+    bar_sync(1, kWorkers);
+    // halo rows of z of the first iteration (written before this launch)
+    float3 hz[kHaloAhead];
+#pragma unroll
+    for (int u = 0; u < kHaloAhead; u++)
+    {
+        const int i = tid + u * kWorkers;
+        hz[u] = make_float3(0.f, 0.f, 0.f);
+        if (i < nhalo)
+            hz[u] = xyz(__ldcg(d.z + w.halo0 + (i < own0 ? i : i + nrow)));
+    }
+    float bf = float(__ldcg(&st->beta));
+    bar_sync(6, kAll);
+    for (unsigned tag = unsigned(it0);; tag++)
+    {
+        // ---- p = z + beta p_old over the halo and the own rows
+        const bool first = bf == 0.f;
+        for (int i = tid, u = 0; i < nhalo; i += kWorkers, u++)
+        {
+            const int j = i < own0 ? i : i + nrow;
+            float3 zz;
+            if (u < kHaloAhead)
+                zz = u == 0 ? hz[0] : u == 1 ? hz[1] : hz[2];
+            else if (tag == unsigned(it0))
+                zz = xyz(__ldcg(d.z + w.halo0 + j));
+            else
+                zz = poll_row(d.z + w.halo0 + j, tag, sc.limit, &sh.err);
+            p_set(j, first ? zz : pform(zz, bf, p_get(j)));
+        }
+        // (a thread's first row, formed anew: else the addresses and bounds of all its
+        // rows are kept in registers from one iteration to the next)
+        int li0 = warp * 32 + lane;
+        asm volatile("" : "+r"(li0));
+#pragma unroll
+        for (int k = 0; k < K; k++)
+        {
+            const int li = k * kWorkers + li0;
+            if (li < nrow)
+            {
+                const float3 z = q_get(li);
+                p_set(own0 + li, first ? z : pform(z, bf, p_get(own0 + li)));
+            }
+        }
+        // (the first chunk's references, in flight over the barrier)
+        constexpr int G = 3, kRef = 2 * G;
+        uint32_t next_ref[kRef];
+        int next_info = 0;
+        auto fetch = [&](int ch) {
+            const int row = min(w.row0 + ch * 32 + lane, w.row1 - 1);
+            next_info = __ldg(d.rowinfo + row);
+#pragma unroll
+            for (int i = 0; i < kRef; i++)
+                next_ref[i] = i < wl ? __ldg(d.lref + lo_idx(i, row, wl)) : 0u;
+        };
+        fetch(min(warp, nch - 1));
+        bar_sync(1, kWorkers);
+        // ---- q = A p; p.q per 32-row chunk
+        int dig = 0;
+        float v4 = 0.f; // four chunks' sums, one per group of 8 lanes
+#pragma unroll 1
+        for (int k = 0; k < K; k++)
+        {
+            const int ch = k * kWarps + warp, li = ch * 32 + lane, row = w.row0 + li;
+            if (ch >= nch)
+                break;
+            const int inf = li < nrow ? next_info : 0;
+            const int ds = (inf >> 8) & 255, ne = (inf & 255) - ds;
+            struct Block
+            {
+                float4 a0;
+                float2 a1;
+            };
+            float3 q = make_float3(0.f, 0.f, 0.f);
+            auto load = [&](Block &b, bool on, uint32_t oa) {
+                b.a0 = make_float4(0.f, 0.f, 0.f, 0.f);
+                b.a1 = make_float2(0.f, 0.f);
+                if (on)
+                {
+                    b.a0 = __ldg(d.A0 + oa);
+                    b.a1 = __ldg(d.A1 + oa);
+                }
+            };
+            auto add = [&](const Block &b, float3 pc, bool on) {
+                const float A[6] = {b.a0.x, b.a0.y, b.a0.z, b.a0.w, b.a1.x, b.a1.y};
+                q = pick(on, q + symv(A, pc), q);
+            };
+            // the upper planes' first group and the lower ones' first two groups
+            // know their addresses
+            Block up[G], lo[G];
+            int cu[G], cl[G];
+            auto lower = [&](int i, bool on, uint32_t ref) {
+                load(lo[i], on, lref_block(ref, wu));
+                cl[i] = on ? lref_col(ref) - w.halo0 : own0;
+            };
+            auto upper = [&](int i, int u) {
+                const uint32_t oa = up_idx(u, row, wu);
+                load(up[i], u < ne, oa);
+                cu[i] = u < ne ? __ldg(d.colu + oa) - w.halo0 : own0;
+            };
+            uint32_t ref[kRef];
+#pragma unroll
+            for (int i = 0; i < kRef; i++)
+                ref[i] = next_ref[i];
+#pragma unroll
+            for (int i = 0; i < G; i++)
+                lower(i, i < ds, ref[i]);
+#pragma unroll
+            for (int i = 0; i < G; i++)
+                upper(i, i);
+            fetch(min(ch + kWarps, nch - 1));
+#pragma unroll
+            for (int i = 0; i < G; i++)
+                add(lo[i], p_get(cl[i]), i < ds);
+            if (wl > G)
+            {
+#pragma unroll
+                for (int i = 0; i < G; i++)
+                    lower(i, G + i < ds, ref[G + i]);
+#pragma unroll
+                for (int i = 0; i < G; i++)
+                    add(lo[i], p_get(cl[i]), G + i < ds);
+            }
+            for (int s = kRef; s < wl; s++)
+            {
+                lower(0, s < ds, s < ds ? __ldg(d.lref + lo_idx(s, row, wl)) : 0u);
+                add(lo[0], p_get(cl[0]), s < ds);
+            }
+            for (int u = 0;;)
+            {
+#pragma unroll
+                for (int i = 0; i < G; i++)
+                    add(up[i], p_get(cu[i]), u + i < ne);
+                u += G;
+                if (u >= wu)
+                    break;
+#pragma unroll
+                for (int i = 0; i < G; i++)
+                    if (u + i < wu)
+                        upper(i, u + i);
+            }
+            q_set(li, q);
+            const float3 pv = p_get(own0 + min(li, nrow - 1));
+            const float part = warp_sum(li < nrow ? fdot(pv, q) : 0.f);
+            v4 = grp == (k & 3) ? part : v4;
+            if ((k & 3) == 3 || k == K - 1 || ch + kWarps >= nch)
+            {
+                int t;
+                if (chunk_digit(v4, s_scale[0], t) && grp <= (k & 3))
+                    dig += t;
+            }
+        }
+        dig += __shfl_xor_sync(kFull, dig, 8);
+        dig += __shfl_xor_sync(kFull, dig, 16);
+        digits_add(s_dig[0], dig, grp == 0);
+        bar_arrive(2, kAll);
+        if (multi && w.rank == 0 && warp == kWarps - 1)
+        {
+            // the sum words of iteration it + 2 (see k_pcg_team)
+            if (lane < 16)
+                sync[blockIdx.x].words[(tag + 2u) & 3u][lane] = 0ull;
+            __threadfence();
+        }
+        // (not on chip: kAhead rows' inverse diagonal blocks in flight)
+        constexpr int kAhead = 3;
+        float4 m0[kAhead];
+        float2 m1[kAhead];
+        auto fetch_m = [&](int k) {
+            const int row = w.row0 + min((k * kWarps + warp) * 32 + lane, nrow - 1);
+            m0[k % kAhead] = __ldg(d.M0 + row);
+            m1[k % kAhead] = __ldg(d.M1 + row);
+        };
+        if constexpr (!kHold)
+#pragma unroll
+            for (int k = 0; k < kAhead; k++)
+                fetch_m(k);
+        bar_sync(3, kAll);
+        if (*(volatile int *)&sh.stop)
+            break;
+        const float af = *(volatile float *)&sh.af;
+        // ---- r -= alpha q, z = M^-1 r; r.z and r.r per chunk (dx += alpha p
+        // once they are on their way)
+        dig = 0;
+        const int s2 = s_scale[1 + (grp >> 1)];
+        float last = 0.f;
+        int own = nrow - li0;
+        asm volatile("" : "+r"(li0), "+r"(own));
+#pragma unroll
+        for (int k = 0; k < K; k++)
+        {
+            const int li = k * kWorkers + li0, row = w.row0 + li;
+            float part = 0.f;
+            if (k * kWorkers - lane < own) // the warp's chunk has rows
+            {
+                float pr = 0.f, prr = 0.f;
+                if (k * kWorkers < own)
+                {
+                    const float3 q = q_get(li);
+                    r[k] = make_float3(fmaf(-af, q.x, r[k].x), fmaf(-af, q.y, r[k].y),
+                                       fmaf(-af, q.z, r[k].z));
+                    float M[6];
+                    if constexpr (kHold)
+                    {
+                        const float2 m0 = sM[li], m1 = sM[rp + li], m2 = sM[2 * rp + li];
+                        M[0] = m0.x;
+                        M[1] = m0.y;
+                        M[2] = m1.x;
+                        M[3] = m1.y;
+                        M[4] = m2.x;
+                        M[5] = m2.y;
+                    }
+                    else
+                    {
+                        M[0] = m0[k % kAhead].x;
+                        M[1] = m0[k % kAhead].y;
+                        M[2] = m0[k % kAhead].z;
+                        M[3] = m0[k % kAhead].w;
+                        M[4] = m1[k % kAhead].x;
+                        M[5] = m1[k % kAhead].y;
+                    }
+                    const float3 z = symv(M, r[k]);
+                    q_set(li, z);
+                    if (row < need0 || row >= need1)
+                        st_row(d.z + row, z, tag + 1u);
+                    pr = fdot(r[k], z);
+                    prr = fdot(r[k], r[k]);
+                }
+                part = warp_sum2(pr, prr);
+            }
+            if constexpr (!kHold)
+                if (k + kAhead < K)
+                    fetch_m(k + kAhead);
+            if (k & 1 || k == K - 1)
+            {
+                int t;
+                if (chunk_digit(k & 1 ? (grp & 1 ? part : last) : part, s2, t) &&
+                    (k & 1 || !(grp & 1)))
+                    dig += t;
+            }
+            last = part;
+        }
+        dig += __shfl_xor_sync(kFull, dig, 8);
+        digits_add(s_dig[1 + (grp >> 1)], dig, !(grp & 1));
+        bar_arrive(4, kAll);
+        if constexpr (kHold)
+        {
+#pragma unroll
+            for (int k = 0; k < K; k++)
+            {
+                const int li = (k * kWarps + warp) * 32 + lane;
+                if (li < nrow)
+                {
+                    const float3 p = p_get(own0 + li);
+                    x[k] = make_float3(fmaf(af, p.x, x[k].x), fmaf(af, p.y, x[k].y),
+                                       fmaf(af, p.z, x[k].z));
+                }
+            }
+        }
+        else
+        {
+            constexpr int kX = 4;
+#pragma unroll 1
+            for (int k0 = 0; k0 * kWarps + warp < nch; k0 += kX)
+            {
+                float4 v[kX];
+#pragma unroll
+                for (int k = 0; k < kX; k++)
+                    v[k] = d.dx[w.row0 + min(((k0 + k) * kWarps + warp) * 32 + lane, nrow - 1)];
+#pragma unroll
+                for (int k = 0; k < kX; k++)
+                {
+                    const int li = ((k0 + k) * kWarps + warp) * 32 + lane;
+                    if (li < nrow)
+                    {
+                        const float3 p = p_get(own0 + li);
+                        d.dx[w.row0 + li] = make_float4(fmaf(af, p.x, v[k].x), fmaf(af, p.y, v[k].y),
+                                                        fmaf(af, p.z, v[k].z), 0.f);
+                    }
+                }
+            }
+        }
+        // the halo rows of the new z, while the sums are under way
+#pragma unroll
+        for (int u = 0; u < kHaloAhead; u++)
+        {
+            const int i = tid + u * kWorkers;
+            if (i < nhalo)
+                hz[u] = poll_row(d.z + w.halo0 + (i < own0 ? i : i + nrow), tag + 1u, sc.limit,
+                                 &sh.err);
+        }
+        bar_sync(5, kAll);
+        bf = *(volatile float *)&sh.bf;
+    }
+#pragma unroll
+    for (int k = 0; k < K; k++)
+    {
+        const int li = (k * kWarps + warp) * 32 + lane, row = w.row0 + li;
+        if (li < nrow)
+        {
+            if constexpr (kHold)
+                d.dx[row] = f4(x[k]);
+            d.r[row] = f4(r[k]);
+            if (*(volatile int *)&sh.stop == kLeave)
+                d.z[row] = f4(p_get(own0 + li));
+        }
+    }
+}
+
 template <int K> const void *half_kernel(bool skew, bool cluster)
 {
     return cluster ? (skew ? (const void *)k_pcg_half<K, true, true>
@@ -1685,6 +2115,9 @@ template <int K> const void *row_kernel(bool skew, bool cluster)
 
 const void *team_kernel(int k, bool half, bool skew, bool cluster)
 {
+    if (half && k > 4)
+        return k == kWideRows ? (const void *)k_pcg_wide<kWideRows>
+                              : (const void *)k_pcg_wide<kWidestRows>;
     if (half)
         return k <= 2   ? half_kernel<2>(skew, cluster)
                : k == 3 ? half_kernel<3>(skew, cluster)

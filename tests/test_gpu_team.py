@@ -20,14 +20,14 @@ def _conf(h, w, model):
             "constraints": {"static_point": [[-0.5, 0.5], [0.5, 0.5]]}}
 
 
-# one row short of, at and past a 32-row chunk; the most rows of one row per
-# thread in a single block (512) and the fewest of two; the largest single
+# one row short of, at and past a 32-row chunk; around the most rows of one
+# row per thread in a single block (480); the largest single
 # block and the smallest team; a short last block; a set whose teams hold two
 # rows per thread; uneven teams in one launch; sets of cloths too large for the
 # whole matrix on chip: every stored block on chip, and a part of them (with
 # rows whose transposed blocks another block owns), two, three and four rows a
-# thread
-# more cloths than SMs, of every size of cluster, the largest with their stored
+# thread; the matrix in memory, up to eight rows a thread and more; a set of
+# those; more cloths than SMs, of every size of cluster, the largest with their stored
 # blocks alone
 MANY = [(3 + k % 5, 4 + k % 3) for k in range(160)] + [(22, 23), (30, 33), (44, 45), (62, 61),
                                                        (87, 88), (100, 100), (125, 128)]
@@ -39,7 +39,8 @@ MANY = [(3 + k % 5, 4 + k % 3) for k in range(160)] + [(22, 23), (30, 33), (44, 
                                     [(65, 64)], [(128, 129)],
                                     [(150, 150), (149, 150), (150, 149), (140, 150)],
                                     [(5, 5), (90, 31), (2, 40), (64, 64)], [(270, 300)],
-                                    [(300, 320), (5, 5)], [(400, 401)], [(470, 480)], MANY])
+                                    [(300, 320), (5, 5)], [(400, 401)], [(470, 480)], [(541, 560)],
+                                    [(760, 767)], [(771, 770)], [(520, 530), (9, 7), (350, 360)], MANY])
 def test_team_kernel_matches_graph_loop(ctx, shapes, model):
     from acousticsim_gb300 import BaraffClothGpu, params
     big = sum(h * w for h, w in shapes) > 40000  # a few iterations show it
