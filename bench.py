@@ -592,10 +592,8 @@ def headline_roofline(args, cloth, solver, prof, prof_iters) -> dict:
         survey_launch = survey_iter * n_it
         kname = ("k_pcg1_persistent (single-barrier PCG, all iterations of the step in one "
                  "cooperative launch)" if solver == "persistent_1b" else
-                 "k_pcg_persistent_sm (all PCG iterations of the step in one cooperative launch)")
-        if args.bending == "dihedral":
-            kname = ("k_pcg_persistent_sm_skew (all PCG iterations of the step in one "
-                     "cooperative launch; blocks with skew parts)")
+                 on_chip_kernel(nv, args.bending == "dihedral") +
+                 " (all PCG iterations of the step in one cooperative launch)")
     else:
         bytes_launch = graph_loop_bytes(nv, nnzb)
         survey_launch = survey_iter
@@ -620,9 +618,9 @@ def headline_roofline(args, cloth, solver, prof, prof_iters) -> dict:
             "avg_launch_ms": launch_ms,
             "us_per_pcg_iteration": 1e3 * sp["ms"] / max(1, sum(prof_iters)),
             "phase_share": shares, "solver": solver, "nnzb": nnzb,
-            "note": "the 512x512 PCG working set (~75 MB) stays in the 129 MB L2: the "
-                    "fraction is of the HBM copy peak, but the kernel is bound by L2 latency "
-                    "and its team barriers, not by DRAM"}
+            "note": "the 512x512 cloth's vectors and a part of its matrix are on chip and the "
+                    "rest (~40 MB) in the 129 MB L2: the fraction is of the HBM copy peak, but "
+                    "the kernel is bound by L2 reads of that rest and its team sums, not by DRAM"}
 
 
 # ---------------------------------------------------------------- batched
@@ -666,6 +664,19 @@ def stratified(keys, count: int) -> list[int]:
     return [int(order[k]) for k in pos]
 
 
+def on_chip_kernel(nv: int, skew: bool) -> str:
+    """The kernel that the persistent solver runs for one grid cloth of nv
+    vertices (rows per thread over 152 blocks of 480 workers)."""
+    rows = nv / (152 * 480)
+    if rows <= 1:
+        return "k_pcg_team"
+    if rows <= 4:
+        return "k_pcg_half"
+    if rows <= 15 and not skew:
+        return "k_pcg_wide"
+    return "k_pcg_persistent_gm_skew" if skew else "k_pcg_persistent_gm"
+
+
 def graph_loop_roofline(prof: dict, bytes_spmv: float, bytes_upd: float) -> dict:
     """Achieved bandwidth of the graph-loop kernels over a profiled solve:
     algorithmic bytes they moved (per instance: iterations x bytes per
@@ -677,6 +688,15 @@ def graph_loop_roofline(prof: dict, bytes_spmv: float, bytes_upd: float) -> dict
     for name, kname, nbytes in (("spmv_dot", "k_spmv (graph loop)", bytes_spmv),
                                 ("update_dot", "k_update_t", bytes_upd)):
         ms = prof[name]["ms"]
+        if name == "spmv_dot" and ms > 0 and prof["update_dot"]["ms"] == 0:
+            # on-chip launches (a cluster a cloth): all iterations in one phase
+            nb = bytes_spmv + bytes_upd
+            out["k_pcg_team, k_pcg_half (a cluster a cloth)"] = {
+                "bound": "latency (matrix and vectors on chip)", "achieved": nb / ms / 1e6,
+                "peak": peak["hbm_gbs"], "unit": "GB/s", "frac": nb / ms / 1e6 / peak["hbm_gbs"],
+                "launches": prof[name]["launches"], "ms_total": ms, "algorithmic_bytes": nb,
+                "traffic": None}
+            continue
         if ms > 0:
             gbs = nbytes / (ms * 1e-3) / 1e9
             # DRAM bytes per algorithmic byte of the committed ncu capture (all

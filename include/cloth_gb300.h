@@ -109,17 +109,18 @@ typedef struct {
     int solver;           /* CLOTH_SOLVER_PERSISTENT or CLOTH_SOLVER_GRAPH_LOOP */
 } cloth_solve_stats;
 
-/* PCG drivers. PERSISTENT: one cooperative launch runs all iterations of every
- * instance (team barriers between the SpMV and update phases); used whenever
- * the launch set fits in the resident blocks, else GRAPH_LOOP: two kernels per
- * iteration inside a CUDA-graph while loop with a device-side condition. */
+/* PCG drivers. PERSISTENT: a launch runs all iterations of its instances: teams
+ * of blocks over the whole GPU that meet at two sums per iteration, or, for sets
+ * of cloths that fit one, a thread-block cluster per cloth (sets of any number).
+ * Used whenever the launch set fits, else GRAPH_LOOP: two kernels per iteration
+ * inside a CUDA-graph while loop with a device-side condition. */
 #define CLOTH_SOLVER_PERSISTENT 0
 #define CLOTH_SOLVER_GRAPH_LOOP 1
 #define CLOTH_SOLVER_FP64 2       /* cloth_solve_fp64 */
 /* PERSISTENT_1B: the persistent launch with one team barrier per iteration
  * (the same PCG in the Chronopoulos-Gear arrangement: r.u, w.u and r.r summed
  * together), used where every block's halo fits in shared memory; stats report
- * which one ran. PERSISTENT_2B: only the two-barrier persistent kernel. */
+ * which one ran. PERSISTENT_2B: only the two-sum persistent kernels. */
 #define CLOTH_SOLVER_PERSISTENT_1B 3
 #define CLOTH_SOLVER_PERSISTENT_2B 4
 /* ESCALATED: the step's FP32 PCG ended in NaN or breakdown (a system beyond
@@ -149,7 +150,8 @@ int cloth_ctx_get_profile(cloth_ctx *ctx, double *ms_total, long long *launches)
 int cloth_ctx_reset_profile(cloth_ctx *ctx);
 /* Preferred PCG driver for launch sets built after the call. */
 int cloth_ctx_set_solver(cloth_ctx *ctx, int solver);
-/* Launch sets of more cloths than fit one persistent launch run the graph
+/* Launch sets of more cloths than blocks are resident at once, with one among
+ * them that no thread-block cluster holds (above ~16,000 vertices), run the graph
  * loop; with the persistent solver (two barriers) chosen, such a set hands
  * its last max_instances iterating cloths to the persistent kernel, whose
  * arithmetic is the graph loop's bit for bit (results do not change; the few
