@@ -1211,13 +1211,24 @@ int plan_persistent(cloth_ctx *ctx, Batch *b)
                 return add_launch(b, l, work, sizeof(TeamSync), alignof(TeamSync) * 64);
         if (plan_queue(ctx, b, &rc))
             return rc;
-        // The matrix read from memory, with as few rows a thread as hold the set
-        // (640^2: 26.6 us per iteration, the older kernel 44.4; 760^2: 48.3 and 59.7;
-        // with 15 rows a thread 900^2: 75.7 and 84.1, 1024^2: 99.7 and 100.3)
+        // The matrix read from memory: r and dx on chip while three quarters of L2 hold
+        // the matrix (640^2, 90 MB: 26.6 us per iteration, 30.5 without, the older kernel
+        // 44.4), else read too, for more loads in flight (680^2, 102 MB: 35.4; 760^2: 42.3,
+        // 48.3 with them on chip, 59.7; 1024^2: 92.0, the older kernel 100.3)
         if (!b->skew)
+        {
+            size_t matrix = 0;
+            for (auto *c : b->members)
+                matrix += size_t(c->tab.nv) * (size_t(c->h.width_up) * 28 + size_t(c->h.width_lo) * 4);
+            int l2 = 0;
+            const bool kept = cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, ctx->device) ==
+                                  cudaSuccess &&
+                              matrix <= size_t(l2) / 4 * 3;
             for (int k : {kWideRows, kWidestRows})
-                if (plan_team(ctx, b, TeamKernel{k, true}, work, l))
+                if ((kept || k == kWidestRows) &&
+                    plan_team(ctx, b, TeamKernel{k, true}, work, l))
                     return add_launch(b, l, work, sizeof(TeamSync), alignof(TeamSync) * 64);
+        }
     }
     work.clear();
     const size_t smem_cap_bytes =

@@ -321,8 +321,8 @@ __host__ __device__ inline size_t half_smem_bytes(int halo, int rows, int ext, i
     return size_t(half_p_quads(halo) + (cluster ? halo - rows : 0)) * 16 +
            size_t(planes) * (rp + ext) * (skew ? 40 : 24) + size_t(words) * rp * 2;
 }
-// k_pcg_wide: rows per thread of its two variants (the first holds dx and the inverse
-// diagonal blocks on chip), and a block's dynamic shared memory.
+// k_pcg_wide: rows per thread of its two variants (the first holds r, dx and the
+// inverse diagonal blocks on chip), and a block's dynamic shared memory.
 constexpr int kWideRows = 8, kWidestRows = 15;
 __host__ __device__ constexpr bool wide_hold(int k) { return k <= kWideRows; }
 __host__ __device__ inline size_t wide_smem_bytes(int halo, int rows, int k)

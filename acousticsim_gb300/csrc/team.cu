@@ -1691,24 +1691,26 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
 
 // The same solve for blocks with more rows than k_pcg_half takes, the matrix read
 // from memory (sets without skew parts).  On chip are p over the halo and q, then z,
-// in one place of shared memory, r in registers, and up to kWideRows rows a thread dx
-// in registers and the inverse diagonal blocks in shared memory as well.  z goes to
+// in one place of shared memory, and up to kWideRows rows a thread r and dx in
+// registers and the inverse diagonal blocks in shared memory as well.  z goes to
 // memory only for rows that another block's columns touch.  K: most rows per thread.
 //
 // What bounds it: reading the stored blocks and the columns (220 bytes a row of a
 // grid) and the transposed rows' blocks again, from L2 and past ~650^2 from HBM, by as
-// many warps as the registers allow.  So a warp has a group's loads in flight
+// many loads as the registers hold.  So a warp has a group's loads in flight
 // together: the upper planes' addresses need no column, and a chunk's lower references
-// are fetched one chunk ahead.  (Groups of 4 spill: 640^2 28.0 us, 26.6 with 3; two
-// groups in flight in turn cost more instructions than the latency they hide: 52.0.)
+// are fetched one chunk ahead.  Groups of 3 next to r and dx in registers (groups of 4
+// spill: 640^2 28.0 us per iteration, 26.6 with 3); where the matrix does not stay in
+// L2 r and dx are better read as well and the registers hold groups of 6: 1024^2 92.0
+// us (4: 98.7, 5: 95.1; 3 with r in registers 99.7), 760^2 42.3 (48.3).
 // us per iteration, before (k_pcg_persistent_gm): 545^2 27.5 -> 18.9, 640^2 44.4 ->
-// 26.6, 760^2 59.7 -> 48.3, 900^2 84.1 -> 75.7, 1024^2 100.3 -> 99.7.
+// 26.6, 680^2 47.9 -> 35.4, 760^2 59.7 -> 42.3, 800^2 69.3 -> 46.9, 1024^2 100.3 -> 92.0.
 template <int K>
 __global__ void __launch_bounds__(kTeamThreads, 1)
     k_pcg_wide(InstDesc *const *descs, const TeamBlock *work, TeamSync *sync, SpinCfg sc)
 {
     constexpr int kAll = kTeamThreads;
-    constexpr bool kHold = wide_hold(K); // dx and the inverse diagonal blocks on chip
+    constexpr bool kHold = wide_hold(K); // r, dx and the inverse diagonal blocks on chip
     extern __shared__ float4 sm_dyn[];
     __shared__ InstDesc d;
     __shared__ int s_dig[3][8];
@@ -1763,21 +1765,20 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
     }
     need0 = __reduce_max_sync(kFull, need0);
     need1 = __reduce_min_sync(kFull, need1);
-    float3 x[kHold ? K : 1], r[K];
+    float3 x[kHold ? K : 1], r[kHold ? K : 1];
     const float4 *pold = (it0 & 1) ? d.p1 : d.p0;
 #pragma unroll
     for (int k = 0; k < K; k++)
     {
         const int li = (k * kWarps + warp) * 32 + lane, row = w.row0 + li;
-        r[k] = make_float3(0.f, 0.f, 0.f);
         if constexpr (kHold)
-            x[k] = r[k];
+            x[k] = r[k] = make_float3(0.f, 0.f, 0.f);
         if (li < nrow)
         {
-            r[k] = xyz(d.r[row]);
             q_set(li, xyz(d.z[row]));
             if constexpr (kHold)
             {
+                r[k] = xyz(d.r[row]);
                 x[k] = xyz(d.dx[row]);
                 const float4 m0 = d.M0[row];
                 sM[li] = make_float2(m0.x, m0.y);
@@ -1833,7 +1834,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
             }
         }
         // (the first chunk's references, in flight over the barrier)
-        constexpr int G = 3, kRef = 2 * G;
+        constexpr int G = kHold ? 3 : 6, kRef = kHold ? 2 * G : G;
         uint32_t next_ref[kRef];
         int next_info = 0;
         auto fetch = [&](int ch) {
@@ -1902,15 +1903,16 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
 #pragma unroll
             for (int i = 0; i < G; i++)
                 add(lo[i], p_get(cl[i]), i < ds);
-            if (wl > G)
-            {
+            if constexpr (kRef > G)
+                if (wl > G)
+                {
 #pragma unroll
-                for (int i = 0; i < G; i++)
-                    lower(i, G + i < ds, ref[G + i]);
+                    for (int i = 0; i < G; i++)
+                        lower(i, G + i < ds, ref[G + i]);
 #pragma unroll
-                for (int i = 0; i < G; i++)
-                    add(lo[i], p_get(cl[i]), G + i < ds);
-            }
+                    for (int i = 0; i < G; i++)
+                        add(lo[i], p_get(cl[i]), G + i < ds);
+                }
             for (int s = kRef; s < wl; s++)
             {
                 lower(0, s < ds, s < ds ? __ldg(d.lref + lo_idx(s, row, wl)) : 0u);
@@ -1951,14 +1953,16 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
                 sync[blockIdx.x].words[(tag + 2u) & 3u][lane] = 0ull;
             __threadfence();
         }
-        // (not on chip: kAhead rows' inverse diagonal blocks in flight)
-        constexpr int kAhead = 3;
+        // (not on chip: kAhead rows' inverse diagonal blocks and r in flight)
+        constexpr int kAhead = 6;
         float4 m0[kAhead];
         float2 m1[kAhead];
+        float4 rr[kAhead];
         auto fetch_m = [&](int k) {
             const int row = w.row0 + min((k * kWarps + warp) * 32 + lane, nrow - 1);
             m0[k % kAhead] = __ldg(d.M0 + row);
             m1[k % kAhead] = __ldg(d.M1 + row);
+            rr[k % kAhead] = d.r[row];
         };
         if constexpr (!kHold)
 #pragma unroll
@@ -1986,8 +1990,13 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
                 if (k * kWorkers < own)
                 {
                     const float3 q = q_get(li);
-                    r[k] = make_float3(fmaf(-af, q.x, r[k].x), fmaf(-af, q.y, r[k].y),
-                                       fmaf(-af, q.z, r[k].z));
+                    float3 &rv = r[kHold ? k : 0];
+                    if constexpr (!kHold)
+                        rv = xyz(rr[k % kAhead]);
+                    rv = make_float3(fmaf(-af, q.x, rv.x), fmaf(-af, q.y, rv.y),
+                                     fmaf(-af, q.z, rv.z));
+                    if constexpr (!kHold)
+                        d.r[row] = f4(rv);
                     float M[6];
                     if constexpr (kHold)
                     {
@@ -2008,12 +2017,12 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
                         M[4] = m1[k % kAhead].x;
                         M[5] = m1[k % kAhead].y;
                     }
-                    const float3 z = symv(M, r[k]);
+                    const float3 z = symv(M, rv);
                     q_set(li, z);
                     if (row < need0 || row >= need1)
                         st_row(d.z + row, z, tag + 1u);
-                    pr = fdot(r[k], z);
-                    prr = fdot(r[k], r[k]);
+                    pr = fdot(rv, z);
+                    prr = fdot(rv, rv);
                 }
                 part = warp_sum2(pr, prr);
             }
@@ -2088,8 +2097,10 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
         if (li < nrow)
         {
             if constexpr (kHold)
+            {
                 d.dx[row] = f4(x[k]);
-            d.r[row] = f4(r[k]);
+                d.r[row] = f4(r[k]);
+            }
             if (*(volatile int *)&sh.stop == kLeave)
                 d.z[row] = f4(p_get(own0 + li));
         }
