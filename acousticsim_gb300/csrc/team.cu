@@ -139,15 +139,20 @@ __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, unsigne
 }
 
 // ---- team sums.  A sum is the exact total V of fixed-point chunk sums, in
-// units of 2^-s, kept as signed 24-bit digits d0 .. d3 (each chunk adds to two
-// of them).  Four words carry it, one per digit: the digit's sum, biased per
-// block, with the number of blocks that added to the word in its top byte;
-// bits 44-55 of the first count the blocks that saw a chunk out of range (or
-// Inf / NaN).
-constexpr int kCountShift = 56, kBadShift = 44;
+// units of 2^-s, kept as signed 24-bit digits d0 .. d4 (each chunk adds to two
+// of them).  V itself has to lie within 2^95 units; its chunks may be up to
+// 2^15 times larger and cancel, as those of an indefinite system's p.q do (a
+// 20 x 20 cloth of negative stiffness has p.q of a hundredth of a chunk's).
+// Four words carry it, one per digit (d4 in d3's): the digit's sum, biased per
+// block, with the number of blocks that added to the word in its top byte.  A block
+// that saw a chunk out of range (or Inf / NaN) adds kTopBad in place of d4, which no
+// others' digits outweigh.
+constexpr int kChunkBits = 86; // a chunk's lowest bit lies below this place
+constexpr int kTopBad = 1 << 21;
+constexpr int kCountShift = 56;
 constexpr unsigned long long kOne = 1ull << kCountShift;
-constexpr unsigned long long kBias = 1ull << 32;
-constexpr unsigned long long kSumMask = (1ull << kBadShift) - 1;
+constexpr unsigned long long kBias = 1ull << 47;
+constexpr unsigned long long kSumMask = kOne - 1;
 
 // V = hi 2^48 + lo, 0 <= lo < 2^48.
 struct Raw
@@ -176,7 +181,7 @@ __device__ __forceinline__ double value(const Raw &r)
 }
 
 // A 32-row chunk's FP32 sum as digits, one sum per group of 8 lanes (v and its scale
-// s are theirs): lane j's part of digit j, lane 4 counting sums out of range; false
+// s are theirs): lane j's part of digit j, lane 5 counting sums out of range; false
 // where the lane has none.
 __device__ __forceinline__ bool chunk_digit(float v, int s, int &x)
 {
@@ -185,19 +190,19 @@ __device__ __forceinline__ bool chunk_digit(float v, int s, int &x)
     unsigned m = (bits & 0x7fffffu) | 0x800000u;
     int sh = e - 150 + s; // |v| = m 2^sh units
     bool bad = false;
-    if (__any_sync(kFull, unsigned(sh) >= 72u || unsigned(e - 1) >= 254u))
+    if (__any_sync(kFull, unsigned(sh) >= unsigned(kChunkBits) || unsigned(e - 1) >= 254u))
     {
         // zero or subnormal (below any scale in use), Inf / NaN, out of range,
         // or digits below the unit
         if (e == 0)
             m = 0u;
-        bad = e == 255 || (e != 0 && sh >= 72);
+        bad = e == 255 || (e != 0 && sh >= kChunkBits);
         if (sh < 0)
         {
             m = sh > -25 ? (m + (1u << (-sh - 1))) >> -sh : 0u;
             sh = 0;
         }
-        sh = min(sh, 71);
+        sh = min(sh, kChunkBits - 1);
     }
     const int k = (sh * 43) >> 10, off = sh - 24 * k; // sh / 24, sh % 24
     x = j == k ? int((m << off) & 0xffffffu) : int(m >> (24 - off));
@@ -207,11 +212,11 @@ __device__ __forceinline__ bool chunk_digit(float v, int s, int &x)
     if (bad)
     {
         x = 1;
-        has = j == 4;
+        has = j == 5;
     }
     return has;
 }
-// Adds the sums to the block's digits dig[0 .. 4] of their quantity.
+// Adds the sums to the block's digits dig[0 .. 5] of their quantity.
 __device__ __forceinline__ void chunk_add(int *dig, float v, int s, bool on)
 {
     int x;
@@ -219,20 +224,17 @@ __device__ __forceinline__ void chunk_add(int *dig, float v, int s, bool on)
         atomicAdd(dig + (threadIdx.x & 7), x);
 }
 // Adds the digits that groups of 8 lanes gathered (up to 16 chunks a warp) to the
-// block's: the low ones carried first, a top one that 15 warps could sum out of 32
-// bits counted as out of range.
+// block's, carried first, so that 15 warps sum them in 32 bits.
 __device__ __forceinline__ void digits_add(int *dig, int d, bool on)
 {
     const int j = threadIdx.x & 7;
-    const int c = j < 3 ? d >> 24 : 0;
+    const int c = j < 4 ? d >> 24 : 0;
     const int below = __shfl_up_sync(kFull, c, 1);
-    if (j < 3)
+    if (j < 4)
         d &= 0xffffff;
-    if (j >= 1 && j <= 3)
+    if (j >= 1 && j <= 4)
         d += below;
-    if (on && j == 3 && (d >= 1 << 27 || d <= -(1 << 27)))
-        atomicAdd(dig + 4, 1);
-    if (on && j < 5 && d != 0)
+    if (on && j < 6 && d != 0)
         atomicAdd(dig + j, d);
 }
 // The sums of a warp's K chunks (the same in every lane; zero where it has
@@ -272,7 +274,7 @@ __device__ __forceinline__ float warp_sum2(float a, float b)
     return v;
 }
 
-// V from its digits; true when it is out of the 96-bit range.
+// V from its digits (d4 in d3's higher bits); true when it is out of the 96-bit range.
 __device__ __forceinline__ bool combine(long long d0, long long d1, long long d2, long long d3,
                                         int s, Raw &r)
 {
@@ -280,40 +282,55 @@ __device__ __forceinline__ bool combine(long long d0, long long d1, long long d2
     r.hi = d2 + d3 * (1ll << 24) + (lo >> 48);
     r.lo = (unsigned long long)lo & 0xffffffffffffull;
     r.s = s;
-    return r.hi >= (1ll << 47) || r.hi < -(1ll << 47);
+    const long long top = d3 + ((d2 + (lo >> 48)) >> 24);
+    return top >= (1ll << 23) || top < -(1ll << 23);
 }
 
-// A block's digits dig[0 .. 4], read and cleared by the control warp.
+// A block's digits dig[0 .. 5], read and cleared by the control warp.
 struct Digits
 {
     int4 d;
-    int bad;
+    int top; // d4, or the mark of a chunk out of range
 };
 __device__ __forceinline__ Digits take(int *dig)
 {
-    const volatile int *v = dig;
-    Digits r{make_int4(v[0], v[1], v[2], v[3]), v[4]};
+    Digits r;
+    int bad;
+    const unsigned at = smem_u32(dig);
+    asm volatile("ld.volatile.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r.d.x), "=r"(r.d.y), "=r"(r.d.z), "=r"(r.d.w)
+                 : "r"(at)
+                 : "memory");
+    asm volatile("ld.volatile.shared.v2.u32 {%0, %1}, [%2];"
+                 : "=r"(r.top), "=r"(bad)
+                 : "r"(at + 16u)
+                 : "memory");
+    if (bad)
+        r.top = kTopBad;
     __syncwarp();
-    if ((threadIdx.x & 31) < 5)
+    if ((threadIdx.x & 31) < 6)
         dig[threadIdx.x & 31] = 0;
     return r;
 }
 __device__ __forceinline__ bool decode(const Digits &v, int s, Raw &r)
 {
-    return combine(v.d.x, v.d.y, v.d.z, v.d.w, s, r) || v.bad != 0;
+    return combine(v.d.x, v.d.y, v.d.z, v.d.w + (long long)v.top * (1ll << 24), s, r);
 }
 
-// The same digits carried into [0, 2^24) (the last one signed), bit 31 of the
-// first marking a sum out of range: a cluster's 16 add up in 32 bits.
+// The same digits as a record, carried so that a cluster's 16 add up in 32 bits: what
+// is above d3's 24 bits (a block's 60 chunks: below 2^20, or kTopBad) is in the
+// upper bytes of the first three, bit 31 of the first saying that it is not zero.
 __device__ __forceinline__ int4 carried(const Digits &v)
 {
+    const int up = v.top + (v.d.w >> 24);
+    const unsigned f = (unsigned(up) & 0x7fffffu) | (up != 0 ? 0x800000u : 0u);
     int4 c = v.d;
     c.y += c.x >> 24;
-    c.x = (c.x & 0xffffff) | (v.bad ? int(0x80000000u) : 0);
     c.z += c.y >> 24;
-    c.y &= 0xffffff;
-    c.w += c.z >> 24;
-    c.z &= 0xffffff;
+    c.w = (c.w & 0xffffff) + (c.z >> 24);
+    c.x = int(unsigned(c.x & 0xffffff) | (f & 0xff0000u) << 8);
+    c.y = int(unsigned(c.y & 0xffffff) | (f & 0xff00u) << 16);
+    c.z = int(unsigned(c.z & 0xffffff) | f << 24);
     return c;
 }
 // Total of a cluster's nblk records.
@@ -322,18 +339,28 @@ __device__ __forceinline__ bool decode(const int4 *rec, int nblk, int s, Raw &r)
     int4 c = make_int4(0, 0, 0, 0);
     if ((threadIdx.x & 31) < nblk)
         c = rec[threadIdx.x & 31];
-    const bool bad = __any_sync(kFull, c.x < 0) != 0;
-    const int d0 = __reduce_add_sync(kFull, c.x & 0xffffff), d1 = __reduce_add_sync(kFull, c.y),
+    int up = 0;
+    if (__any_sync(kFull, c.x < 0))
+    {
+        const unsigned f = (unsigned(c.x) >> 8 & 0x7f0000u) | (unsigned(c.y) >> 16 & 0xff00u) |
+                           unsigned(c.z) >> 24;
+        up = __reduce_add_sync(kFull, int(f << 9) >> 9);
+        c.x &= 0xffffff;
+        c.y &= 0xffffff;
+        c.z &= 0xffffff;
+    }
+    const int d0 = __reduce_add_sync(kFull, c.x), d1 = __reduce_add_sync(kFull, c.y),
               d2 = __reduce_add_sync(kFull, c.z), d3 = __reduce_add_sync(kFull, c.w);
-    return combine(d0, d1, d2, d3, s, r) || bad;
+    return combine(d0, d1, d2, d3 + (long long)up * (1ll << 24), s, r);
 }
 
 // Word k of a block's sum: added to the team's by lane k.
 __device__ __forceinline__ void word_add(unsigned long long *words, const Digits &v, int k)
 {
     const int d = k == 0 ? v.d.x : k == 1 ? v.d.y : k == 2 ? v.d.z : v.d.w;
-    const unsigned long long w = kOne + kBias + (unsigned long long)(long long)d +
-                                 (k == 0 && v.bad ? 1ull << kBadShift : 0ull);
+    const unsigned long long w =
+        kOne + kBias +
+        (unsigned long long)(d + (long long)(k == 3 ? v.top : 0) * (1ll << 24));
     asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(words + k), "l"(w)
                  : "memory");
 }
@@ -360,8 +387,7 @@ struct Words
         const unsigned long long b = (unsigned long long)nblk * kBias;
         return combine((long long)((w[0] & kSumMask) - b), (long long)((w[1] & kSumMask) - b),
                        (long long)((w[2] & kSumMask) - b), (long long)((w[3] & kSumMask) - b), s,
-                       r) ||
-               ((w[0] >> kBadShift) & 0xfffu) != 0;
+                       r);
     }
 };
 
@@ -846,7 +872,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
     constexpr int RC = RW > 0 ? 5 : 0; // slots past the RW whose offsets of p are in registers
     extern __shared__ float4 sm_dyn[];
     __shared__ InstDesc d;
-    __shared__ int s_dig[3][8];  // digits of the block's sums: p.q, r.z, r.r
+    alignas(16) __shared__ int s_dig[3][8]; // digits of the block's sums: p.q, r.z, r.r
     __shared__ int s_scale[3];   // and their scales
     __shared__ Shared<CLUSTER> sh;
     const TeamBlock w = work[blockIdx.x];
@@ -1243,7 +1269,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
     constexpr int kAll = kTeamThreads;
     extern __shared__ float4 sm_dyn[];
     __shared__ InstDesc d;
-    __shared__ int s_dig[3][8];
+    alignas(16) __shared__ int s_dig[3][8];
     __shared__ int s_scale[3];
     __shared__ Shared<CLUSTER> sh;
     const TeamBlock w = work[blockIdx.x];
@@ -1713,7 +1739,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
     constexpr bool kHold = wide_hold(K); // r, dx and the inverse diagonal blocks on chip
     extern __shared__ float4 sm_dyn[];
     __shared__ InstDesc d;
-    __shared__ int s_dig[3][8];
+    alignas(16) __shared__ int s_dig[3][8];
     __shared__ int s_scale[3];
     __shared__ Shared<false> sh;
     const TeamBlock w = work[blockIdx.x];
