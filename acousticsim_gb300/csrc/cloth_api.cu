@@ -977,6 +977,35 @@ bool team_split(const cloth_s *c, int i, bool skew_kernel, int blocks, TeamKerne
 // Most dynamic shared memory of a block of a cluster.
 size_t cluster_smem_cap(const cloth_ctx *ctx) { return size_t(ctx->max_smem_optin) - 6144; }
 
+// How many clusters of C blocks of an on-chip kernel can be resident together (0:
+// none, also where the device refuses such a cluster); sets the kernel's attributes.
+int resident_clusters(const cloth_ctx *ctx, const void *f, int C, size_t blocks, size_t smem)
+{
+    cudaLaunchConfig_t cfg;
+    std::memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3(unsigned(blocks));
+    cfg.blockDim = dim3(kTeamThreads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute at;
+    std::memset(&at, 0, sizeof(at));
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = unsigned(C);
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int active = 0;
+    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             int(cluster_smem_cap(ctx))) != cudaSuccess ||
+        cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
+            cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&active, f, &cfg) != cudaSuccess)
+    {
+        cudaGetLastError();
+        return 0;
+    }
+    return active;
+}
+
 // Plan of an on-chip kernel over some members, its teams clusters of C blocks
 // (at_once: all of them resident together).
 bool plan_cluster(cloth_ctx *ctx, const Batch *b, std::vector<int> which, TeamKernel tk, int C,
@@ -1011,29 +1040,7 @@ bool plan_cluster(cloth_ctx *ctx, const Batch *b, std::vector<int> which, TeamKe
     l.cluster = C;
     l.block = kTeamThreads;
     l.smem = smem;
-    cudaLaunchConfig_t cfg;
-    std::memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3(unsigned(work.size()));
-    cfg.blockDim = dim3(kTeamThreads);
-    cfg.dynamicSmemBytes = smem;
-    cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = unsigned(C);
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    int active = 0;
-    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, int(cap)) !=
-            cudaSuccess ||
-        cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
-            cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&active, f, &cfg) != cudaSuccess ||
-        active < (at_once ? n : 1))
-    {
-        cudaGetLastError();
-        return false;
-    }
-    return true;
+    return resident_clusters(ctx, f, C, work.size(), smem) >= (at_once ? n : 1);
 }
 
 // Plan of k_pcg_team with K rows per thread and teams of any number of blocks,
@@ -2098,15 +2105,13 @@ bool cloth::detail::cluster_plan(cloth_ctx *ctx, const cloth_s *c, ClusterPlan &
     out.func = team_kernel(ch.k.K, ch.k.half, skew, true);
     out.cluster = ch.C;
     out.block = kTeamThreads;
-    if (cudaFuncSetAttribute(out.func, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             int(cluster_smem_cap(ctx))) != cudaSuccess ||
-        cudaFuncSetAttribute(out.func, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
-            cudaSuccess)
-    {
-        cudaGetLastError();
-        return false;
-    }
-    return true;
+    return cluster_resident(ctx, out.func, out.cluster, out.smem);
+}
+
+bool cloth::detail::cluster_resident(const cloth_ctx *ctx, const void *func, int cluster,
+                                     size_t smem)
+{
+    return resident_clusters(ctx, func, cluster, size_t(cluster), smem) >= 1;
 }
 
 int cloth::detail::inner_solve(cloth_s *c, const double *rhs64, const cloth_solve_params *p,

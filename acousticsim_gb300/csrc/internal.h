@@ -231,8 +231,11 @@ struct ClusterPlan
     size_t smem = 0;
     std::vector<TeamBlock> blocks;
 };
-// The smallest cluster that holds the cloth; false when none does.
+// The smallest cluster that holds the cloth; false when none does, or the device
+// cannot run that one.
 bool cluster_plan(cloth_ctx *ctx, const cloth_s *c, ClusterPlan &out);
+// Whether the device can run a cluster of an on-chip kernel with that shared memory.
+bool cluster_resident(const cloth_ctx *ctx, const void *func, int cluster, size_t smem);
 
 // Points the scratch fields of h at base (null: clears them).
 void bind_scratch(const cloth_s *c, InstDesc &h, char *base);

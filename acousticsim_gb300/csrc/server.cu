@@ -511,6 +511,18 @@ size_t plan_clusters(cloth_server_s *s)
         g.smem = std::max(g.smem, cr.plan.smem);
         blocks += cr.plan.blocks.size();
     }
+    // a group's launch takes the shared memory of its largest cloth
+    for (size_t k = 0; k < s->groups.size(); k++)
+    {
+        const SrvGroup &g = s->groups[k];
+        if (!cluster_resident(s->ctx, g.func, g.cluster, g.smem))
+            for (SrvCloth &cr : s->cl)
+                if (cr.group == int(k))
+                {
+                    cr.group = -1;
+                    cr.plan.blocks.clear();
+                }
+    }
     return align_up(blocks * sizeof(TeamBlock), 256);
 }
 
