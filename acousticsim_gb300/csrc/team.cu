@@ -844,7 +844,21 @@ __device__ __forceinline__ void control_warp(const InstDesc &d, const TeamBlock 
         }
     }
     if (CLUSTER)
+    {
+        // (a block that gave up leaves its shared memory to the peers' stores that
+        // are still on their way)
+        if (stop == 9)
+            for (int i = 0; i < 32; i++)
+                __nanosleep(1000);
         cluster_sync();
+        // a wait of another block alone gave up, after the first one's last sum: the
+        // solve is not to go on from that block's rows
+        if (lane == 0 && w.rank == 0 && stop != 9 && atomicAdd(&st->bar_err, 0) != 0)
+        {
+            st->status = 9;
+            st->active = 0;
+        }
+    }
 }
 
 __device__ __forceinline__ float3 pick(bool on, float3 a, float3 b)
