@@ -2923,8 +2923,9 @@ __global__ void __launch_bounds__(kPBlock, 1)
             bc_s[2] = fx_scale(rr);
             if (w.rank == 0)
             {
-                // the buffer of the next sums was last read two iterations ago
-                const int nb = (bq + 1) % 3;
+                // the buffer of the sums after the next was last read one iteration
+                // ago, and no block adds to it before the next barrier
+                const int nb = (bq + 2) % 3;
                 for (int q = 0; q < 3; q++)
                 {
                     st->acc[nb][q][0] = 0ull;
