@@ -117,8 +117,12 @@ struct InstState
     // exact fixed-point team sums of the persistent solver, triple-buffered by
     // iteration: [buffer][quantity: p.q, r.z, r.r][limb: units of 2^32, units]
     unsigned long long acc[3][3][2];
-    float acc_chk[3][3];  // FP32 magnitude check of the same sums
-    float pad2[3];
+    // what their 96 bits do not tell: the chunks of 2^75 units and more (fx_note), in
+    // units of 2^72, and whether one was out of range or not finite; and the
+    // magnitudes (fx_mag) of the first two's chunks
+    unsigned long long acc_top[3][3], acc_mag[3][2];
+    int acc_bad[3][3];
+    int pad2;
 };
 
 struct InstDesc
@@ -278,7 +282,7 @@ struct SpinCfg
 // k_pcg_team: worker threads (one row each, or two) and the control warp - 16
 // warps, four on each quarter of an SM, so a thread may have 128 registers; a
 // team's sum words, four iterations deep (p.q in words 0-3, r.z in 4-7, r.r in
-// 8-11), zeroed before every launch.
+// 8-11, the first two's magnitudes in 12-13), zeroed before every launch.
 constexpr int kTeamWorkers = 480;
 constexpr int kTeamThreads = kTeamWorkers + 32;
 constexpr int kTeamAloneRows = 320; // instances up to this size: a team of one block

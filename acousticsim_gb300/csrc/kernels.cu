@@ -191,12 +191,7 @@ __device__ __forceinline__ void begin_solve(const InstDesc &d, const double (&to
     st.bar_err = 0;
     st.open = 1;
     for (int bq = 0; bq < 3; bq++)
-        for (int q = 0; q < 3; q++)
-        {
-            st.acc[bq][q][0] = 0ull;
-            st.acc[bq][q][1] = 0ull;
-            st.acc_chk[bq][q] = 0.f;
-        }
+        fx_clear(&st, bq);
     if (!isfinite(tot[0]) || !isfinite(tot[1]) || !isfinite(tot[2]))
     {
         st.status = 6; // CLOTH_ERR_NAN
@@ -751,7 +746,7 @@ __device__ __forceinline__ void tile_fx_add(const float (&vf)[R][N], InstState *
             tsum[r][k] = warp_sum(vf[r][k]);
     long long hh = 0;
     unsigned long long ll = 0ull;
-    float c = 0.f;
+    unsigned mag = 0u;
 #pragma unroll
     for (int r = 0; r < R; r++)
 #pragma unroll
@@ -759,20 +754,23 @@ __device__ __forceinline__ void tile_fx_add(const float (&vf)[R][N], InstState *
             if (l == r * N + k)
             {
                 fx_split(tsum[r][k], sc[k], hh, ll);
-                c = tsum[r][k];
+                if (q0 + k < 2)
+                    mag = fx_mag(tsum[r][k], sc[k]);
+                fx_note(tsum[r][k], sc[k], st, bq, q0 + k);
             }
 #pragma unroll
     for (int o = (R / 2) * N; o >= N && o > 0; o >>= 1)
     {
         hh += __shfl_xor_sync(FULLM, hh, o);
         ll += __shfl_xor_sync(FULLM, ll, o);
-        c += __shfl_xor_sync(FULLM, c, o);
+        mag += __shfl_xor_sync(FULLM, mag, o);
     }
     if (l < N)
     {
         atomicAdd(&st->acc[bq][q0 + l][0], (unsigned long long)hh);
         atomicAdd(&st->acc[bq][q0 + l][1], ll);
-        atomicAdd(&st->acc_chk[bq][q0 + l], c);
+        if (q0 + l < 2)
+            atomicAdd(&st->acc_mag[bq][q0 + l], (unsigned long long)mag);
     }
 }
 
@@ -1665,21 +1663,22 @@ __global__ void __launch_bounds__(kBulkThreads, SKEW ? 1 : 2) k_spmv_bulk(InstDe
             {
                 long long hh;
                 unsigned long long ll;
+                const int bq = g.it % 3;
                 fx_split(g.v, g.s, hh, ll);
-                float c = g.v;
+                fx_note(g.v, g.s, g.st, bq, 0);
+                unsigned mag = fx_mag(g.v, g.s);
 #pragma unroll
                 for (int k = (kTile / 32) / 2; k > 0; k >>= 1)
                 {
                     hh += __shfl_xor_sync(M4, hh, k);
                     ll += __shfl_xor_sync(M4, ll, k);
-                    c += __shfl_xor_sync(M4, c, k);
+                    mag += __shfl_xor_sync(M4, mag, k);
                 }
                 if (lane == 0)
                 {
-                    const int bq = g.it % 3;
                     atomicAdd(&g.st->acc[bq][0][0], (unsigned long long)hh);
                     atomicAdd(&g.st->acc[bq][0][1], ll);
-                    atomicAdd(&g.st->acc_chk[bq][0], c);
+                    atomicAdd(&g.st->acc_mag[bq][0], (unsigned long long)mag);
                 }
             }
             __syncwarp();
@@ -1812,16 +1811,6 @@ __global__ void __launch_bounds__(kBulkThreads, SKEW ? 1 : 2) k_spmv_bulk(InstDe
 // iteration count and the convergence test; the next iteration's buffer
 // (last used two iterations ago) is cleared.
 namespace {
-__device__ __forceinline__ double loop_total(const InstState *st, int bq, int q, int s,
-                                             int *bad)
-{
-    const double v = fx_value(__ldcg(&st->acc[bq][q][0]), __ldcg(&st->acc[bq][q][1]), s);
-    const float chk = __ldcg(&st->acc_chk[bq][q]);
-    if (!isfinite(chk) || fabs(v - double(chk)) > 1e-3 * fabs(double(chk)) + 1e-30)
-        *bad = 1;
-    return v;
-}
-
 template <int KIND>
 __device__ __forceinline__ void reduce_body(InstDesc *const *descs, const int *inst_list,
                                             int ninst, const int *ninst_dev, BatchCtl *ctl,
@@ -1842,7 +1831,7 @@ __device__ __forceinline__ void reduce_body(InstDesc *const *descs, const int *i
         int bad = 0;
         if (KIND == 0)
         {
-            const double pq = loop_total(stp, bq, 0, fx_scale(st.pq), &bad);
+            const double pq = fx_total(stp, bq, 0, fx_scale(st.pq), &bad);
             st.pq = pq;
             if (bad || !isfinite(pq))
             {
@@ -1865,15 +1854,11 @@ __device__ __forceinline__ void reduce_body(InstDesc *const *descs, const int *i
         else
         {
             const double rho0 = st.rho;
-            const double rho_new = loop_total(stp, bq, 1, fx_scale(rho0), &bad);
-            const double rr = loop_total(stp, bq, 2, fx_scale(st.rr), &bad);
-            const int nb = (it0 + 1) % 3;
-            for (int q = 0; q < 3; q++)
-            {
-                st.acc[nb][q][0] = 0ull;
-                st.acc[nb][q][1] = 0ull;
-                st.acc_chk[nb][q] = 0.f;
-            }
+            const double rho_new = fx_total(stp, bq, 1, fx_scale(rho0), &bad);
+            const double rr = fx_total(stp, bq, 2, fx_scale(st.rr), &bad);
+            if (fx_cancels(stp, bq, 0) || fx_cancels(stp, bq, 1))
+                bad = 1;
+            fx_clear(stp, (it0 + 1) % 3);
             st.beta = (rho0 == 0.0) ? 0.0 : rho_new / rho0;
             st.rho = rho_new;
             st.rr = rr;
@@ -2167,7 +2152,7 @@ template <int NQ> struct WarpFx
 {
     long long H[NQ];
     unsigned long long L[NQ];
-    float chk[NQ];
+    unsigned mag[NQ];
     __device__ __forceinline__ void clear()
     {
 #pragma unroll
@@ -2175,17 +2160,18 @@ template <int NQ> struct WarpFx
         {
             H[q] = 0;
             L[q] = 0ull;
-            chk[q] = 0.f;
+            mag[q] = 0u;
         }
     }
-    __device__ __forceinline__ void add(int q, float v, int s)
+    __device__ __forceinline__ void add(int q, float v, int s, InstState *st, int bq)
     {
         long long h;
         unsigned long long l;
         fx_split(v, s, h, l);
+        fx_note(v, s, st, bq, q);
+        mag[q] += fx_mag(v, s);
         H[q] += h;
         L[q] += l;
-        chk[q] += v;
     }
 };
 
@@ -2286,30 +2272,31 @@ __device__ __forceinline__ void pcg_persistent_body(InstDesc *const *descs,
             const int q = warp;
             const int sq = q == 0 ? sc0 : sc1;
             {
-                unsigned long long h = 0ull, l = 0ull;
-                float c = 0.f;
+                unsigned long long h = 0ull, l = 0ull, mag = 0ull;
                 for (int ch = lane; ch < nch; ch += 32)
                 {
                     const float v = cpart[(q0 + q) * cps + ch];
                     long long hh;
                     unsigned long long ll;
                     fx_split(v, sq, hh, ll);
+                    fx_note(v, sq, st, bq, q0 + q);
+                    mag += fx_mag(v, sq);
                     h += (unsigned long long)hh;
                     l += ll;
-                    c += v;
                 }
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1)
                 {
                     h += __shfl_xor_sync(0xffffffffu, h, o);
                     l += __shfl_xor_sync(0xffffffffu, l, o);
-                    c += __shfl_xor_sync(0xffffffffu, c, o);
+                    mag += __shfl_xor_sync(0xffffffffu, mag, o);
                 }
                 if (lane == 0)
                 {
                     atomicAdd(&st->acc[bq][q0 + q][0], h);
                     atomicAdd(&st->acc[bq][q0 + q][1], l);
-                    atomicAdd(&st->acc_chk[bq][q0 + q], c);
+                    if (q0 + q < 2)
+                        atomicAdd(&st->acc_mag[bq][q0 + q], mag);
                 }
             }
         }
@@ -2317,14 +2304,9 @@ __device__ __forceinline__ void pcg_persistent_body(InstDesc *const *descs,
             s_nbar += (unsigned long long)w.nblk;
         return team_barrier_count(team_count(), s_nbar, st, w.nblk, sc);
     };
-    // Reads a team sum after the barrier; flags a fixed-point overflow when it
-    // disagrees with the FP32 magnitude check.
+    // Reads a team sum after the barrier.
     auto team_value = [&](int q, int bq, int s, int *bad) -> double {
-        const double v = fx_value(__ldcg(&st->acc[bq][q][0]), __ldcg(&st->acc[bq][q][1]), s);
-        const float chk = __ldcg(&st->acc_chk[bq][q]);
-        if (!isfinite(chk) || fabs(v - double(chk)) > 1e-3 * fabs(double(chk)) + 1e-30)
-            *bad = 1;
-        return v;
+        return fx_total(st, bq, q, s, bad);
     };
 
     for (;;)
@@ -2344,13 +2326,7 @@ __device__ __forceinline__ void pcg_persistent_body(InstDesc *const *descs,
             if (w.rank == 0)
             {
                 // the buffer of iteration it+1 was last read in iteration it-2
-                const int nb = (it + 1) % 3;
-                for (int q = 0; q < 3; q++)
-                {
-                    st->acc[nb][q][0] = 0ull;
-                    st->acc[nb][q][1] = 0ull;
-                    st->acc_chk[nb][q] = 0.f;
-                }
+                fx_clear(st, (it + 1) % 3);
             }
         }
         // ---- p = z + beta p_old over the staged range. The staged p of the
@@ -2598,6 +2574,8 @@ __device__ __forceinline__ void pcg_persistent_body(InstDesc *const *descs,
             int bad = 0;
             const double rho_new = team_value(1, bq, s1q, &bad);
             const double rr = team_value(2, bq, s2q, &bad);
+            if (fx_cancels(st, bq, 0) || fx_cancels(st, bq, 1))
+                bad = 1;
             s_beta = (s_rho == 0.0) ? 0.0 : rho_new / s_rho;
             s_rho = rho_new;
             s_rr = rr;
@@ -2713,7 +2691,7 @@ __global__ void __launch_bounds__(kPBlock, 1)
     extern __shared__ float4 sm_dyn[];
     __shared__ InstDesc d;
     __shared__ unsigned long long wsum_h[3][NW], wsum_l[3][NW];
-    __shared__ float wsum_c[3][NW];
+    __shared__ unsigned wsum_m[3][NW];
     // FP64 scalars: owned by thread 0, the block reads the FP32 copies
     __shared__ double s_gam, s_del, s_rr, s_alpha, s_beta;
     __shared__ float bc_af, bc_bf;
@@ -2772,32 +2750,28 @@ __global__ void __launch_bounds__(kPBlock, 1)
             {
                 wsum_h[q][warp] = (unsigned long long)wfx.H[q];
                 wsum_l[q][warp] = wfx.L[q];
-                wsum_c[q][warp] = wfx.chk[q];
+                wsum_m[q][warp] = wfx.mag[q];
             }
         __syncthreads();
         if (tid == 0)
             for (int q = 0; q < 3; q++)
             {
-                unsigned long long hh = 0ull, ll = 0ull;
-                float c = 0.f;
+                unsigned long long hh = 0ull, ll = 0ull, mag = 0ull;
                 for (int j = 0; j < NW; j++)
                 {
                     hh += wsum_h[q][j];
                     ll += wsum_l[q][j];
-                    c += wsum_c[q][j];
+                    mag += wsum_m[q][j];
                 }
                 atomicAdd(&st->acc[bq][q][0], hh);
                 atomicAdd(&st->acc[bq][q][1], ll);
-                atomicAdd(&st->acc_chk[bq][q], c);
+                if (q < 2)
+                    atomicAdd(&st->acc_mag[bq][q], mag);
             }
         return team_barrier(st, w.nblk, sc);
     };
     auto team_value = [&](int q, int bq, int s, int *bad) -> double {
-        const double v = fx_value(__ldcg(&st->acc[bq][q][0]), __ldcg(&st->acc[bq][q][1]), s);
-        const float chk = __ldcg(&st->acc_chk[bq][q]);
-        if (!isfinite(chk) || fabs(v - double(chk)) > 1e-3 * fabs(double(chk)) + 1e-30)
-            *bad = 1;
-        return v;
+        return fx_total(st, bq, q, s, bad);
     };
     // w = A u on an own row from the staged u; writes wbuf, returns w.u
     auto spmv_row = [&](int row, float3 uv, float4 *wbuf) -> float {
@@ -2872,9 +2846,9 @@ __global__ void __launch_bounds__(kPBlock, 1)
             pr = warp_sum(pr);
             if (lane == 0)
             {
-                f.add(0, pg, s0q);
-                f.add(1, pd, s1q);
-                f.add(2, pr, s2q);
+                f.add(0, pg, s0q, st, bq);
+                f.add(1, pd, s1q, st, bq);
+                f.add(2, pr, s2q, st, bq);
             }
         }
         if (!team_sum(f, bq))
@@ -2889,6 +2863,8 @@ __global__ void __launch_bounds__(kPBlock, 1)
             const double gam = team_value(0, bq, bc_s[0], &bad);
             const double del = team_value(1, bq, bc_s[1], &bad);
             const double rr = team_value(2, bq, bc_s[2], &bad);
+            if (fx_cancels(st, bq, 0) || fx_cancels(st, bq, 1))
+                bad = 1;
             int stop = 0; // 0 go on, 1 converged, else a status code
             double beta = 0.0, alpha = s_alpha;
             if (bad || !isfinite(gam) || !isfinite(del) || !isfinite(rr))
@@ -2925,13 +2901,7 @@ __global__ void __launch_bounds__(kPBlock, 1)
             {
                 // the buffer of the sums after the next was last read one iteration
                 // ago, and no block adds to it before the next barrier
-                const int nb = (bq + 2) % 3;
-                for (int q = 0; q < 3; q++)
-                {
-                    st->acc[nb][q][0] = 0ull;
-                    st->acc[nb][q][1] = 0ull;
-                    st->acc_chk[nb][q] = 0.f;
-                }
+                fx_clear(st, (bq + 2) % 3);
             }
         }
         __syncthreads();
@@ -2942,7 +2912,7 @@ __global__ void __launch_bounds__(kPBlock, 1)
         }
         const float af = bc_af, bf = bc_bf;
         const bool first = (it == 0);
-        const int cur = it & 1, nxt = cur ^ 1;
+        const int cur = it & 1, nxt = cur ^ 1, nbq = (bq + 1) % 3;
         const int s0q = bc_s[0], s1q = bc_s[1], s2q = bc_s[2];
         WarpFx<3> f;
         f.clear();
@@ -2985,8 +2955,8 @@ __global__ void __launch_bounds__(kPBlock, 1)
             pr = warp_sum(pr);
             if (lane == 0)
             {
-                f.add(0, pg, s0q);
-                f.add(2, pr, s2q);
+                f.add(0, pg, s0q, st, nbq);
+                f.add(2, pr, s2q, st, nbq);
             }
         }
         // ---- halo rows owned by other blocks: the same u from their r, w, s
@@ -3015,9 +2985,9 @@ __global__ void __launch_bounds__(kPBlock, 1)
                 pd = spmv_row(row, xyz(su[row - h0]), wb[nxt]);
             pd = warp_sum(pd);
             if (lane == 0)
-                f.add(1, pd, s1q);
+                f.add(1, pd, s1q, st, nbq);
         }
-        bq = (bq + 1) % 3;
+        bq = nbq;
         it++;
         if (!team_sum(f, bq))
         {

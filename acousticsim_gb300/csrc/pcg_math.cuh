@@ -101,13 +101,13 @@ __device__ __forceinline__ void fx_split(float v, int s, long long &H,
     H = 0;
     L = 0;
     if (e == 0 || e == 255)
-        return; // zero, subnormal (below any scale in use) or Inf/NaN (check sum)
+        return; // zero, subnormal (below any scale in use) or Inf/NaN (fx_note)
     const unsigned long long m = (bits & 0x7fffffu) | 0x800000u;
     const int sh = e - 150 + s; // |v| = m * 2^(e - 150)
     unsigned long long fh = 0ull, fl = 0ull;
     if (sh >= 104)
     {
-        fh = 0x3fffffffffffffffull; // saturate; the check sum flags it
+        fh = 0x3fffffffffffffffull; // out of range: fx_note flags it
         fl = ~0ull;
     }
     else if (sh >= 64)
@@ -128,6 +128,66 @@ __device__ __forceinline__ void fx_split(float v, int s, long long &H,
     }
     L = fl & 0xffffffffull;
     H = (long long)((fh << 32) | (fl >> 32));
+}
+
+// Which sums count, in every driver alike: each 32-row chunk below 2^(kChunkBits + 24)
+// units and finite, their exact total within 2^95, and (p.q and r.z, judged at the end
+// of the iteration) the total not so far below the sum of the chunks' magnitudes that
+// the chunks' FP32 rounding leaves nothing of it.
+//
+// The limbs hold the total modulo 2^96, so chunks of 2^75 units and more, which are
+// rare (a sum's last value has about 2^70), are counted in units of 2^72 too; the
+// others' part of 2^19 chunks (16 million rows) stays in range.
+constexpr int kChunkBits = 86, kChunkBig = 52, kTopUnit = 72;
+__device__ __forceinline__ void fx_note(float v, int s, InstState *st, int bq, int q)
+{
+    const unsigned bits = __float_as_uint(v);
+    const int e = int((bits >> 23) & 0xffu), sh = e - 150 + s;
+    if (e == 0 || (sh < kChunkBig && e != 255))
+        return;
+    if (e == 255 || sh >= kChunkBits)
+    {
+        atomicOr(&st->acc_bad[bq][q], 1);
+        return;
+    }
+    long long m = (long long)((bits & 0x7fffffu) | 0x800000u);
+    if (bits & 0x80000000u)
+        m = -m;
+    m = sh >= kTopUnit ? m * (1ll << (sh - kTopUnit)) : m >> (kTopUnit - sh);
+    atomicAdd(&st->acc_top[bq][q], (unsigned long long)m);
+}
+// A chunk's magnitude m 2^sh in units of 2^66, at most 2^18; and whether a total, floor(V
+// / 2^kCancelUnit), is below 2^-kCancelBits of its chunks' magnitudes: p.q of an
+// indefinite system, or r.z where diagonal blocks are, once FP32 (rows of 2^-24, and
+// more in their sums) no longer resolves it.  alpha and beta are then noise and the solve
+// stalls until max_iters (256x256 with stiff dihedral bending: a residual of 0.4 after
+// 20,000 iterations); ended as NaN, a step escalates it to FP64.  Solves that converge
+// stay far from it (small negative stiffness: p.q a hundredth of a chunk).
+constexpr int kCancelBits = 13, kCancelUnit = 66 - kCancelBits;
+__device__ __forceinline__ unsigned fx_mag(unsigned m, int sh)
+{
+    return min(m >> min(max(66 - sh, 0), 31), 1u << 18);
+}
+__device__ __forceinline__ unsigned fx_mag(float v, int s)
+{
+    const unsigned bits = __float_as_uint(v);
+    const int e = int((bits >> 23) & 0xffu);
+    return e == 0 || e == 255 ? 0u : fx_mag((bits & 0x7fffffu) | 0x800000u, e - 150 + s);
+}
+__device__ __forceinline__ bool fx_cancels(long long total, unsigned long long mag)
+{
+    return (unsigned long long)(total ^ (total >> 63)) < mag;
+}
+__device__ __forceinline__ void fx_clear(InstState *st, int bq)
+{
+    for (int q = 0; q < 3; q++)
+    {
+        st->acc[bq][q][0] = 0ull;
+        st->acc[bq][q][1] = 0ull;
+        st->acc_top[bq][q] = 0ull;
+        st->acc_bad[bq][q] = 0;
+    }
+    st->acc_mag[bq][0] = st->acc_mag[bq][1] = 0ull;
 }
 
 // Scale exponent for an estimate of a sum (from the double's exponent bits).
@@ -151,6 +211,25 @@ __device__ __forceinline__ double fx_value(unsigned long long H, unsigned long l
                                            int s)
 {
     return double((long long)H) * pow2(32 - s) + double(L) * pow2(-s);
+}
+
+__device__ __forceinline__ bool fx_cancels(const InstState *st, int bq, int q)
+{
+    const long long H = (long long)(__ldcg(&st->acc[bq][q][0]) + (__ldcg(&st->acc[bq][q][1]) >> 32));
+    return fx_cancels(H >> (kCancelUnit - 32), __ldcg(&st->acc_mag[bq][q]));
+}
+// A sum's total; *bad where it is out of range.
+__device__ __forceinline__ double fx_total(const InstState *st, int bq, int q, int s, int *bad)
+{
+    const unsigned long long L = __ldcg(&st->acc[bq][q][1]);
+    const unsigned long long H = __ldcg(&st->acc[bq][q][0]) + (L >> 32);
+    const long long top = (long long)__ldcg(&st->acc_top[bq][q]);
+    // the total over 2^72, as the limbs have it (24 bits) and as it is
+    const long long hi = (long long)H >> (kTopUnit - 32);
+    const long long rest = (long long)((unsigned long long)(hi - top) << 40) >> 40;
+    if (__ldcg(&st->acc_bad[bq][q]) != 0 || top + rest != hi)
+        *bad = 1;
+    return fx_value(H, L & 0xffffffffull, s);
 }
 
 } // namespace cloth

@@ -146,8 +146,10 @@ __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, unsigne
 // Four words carry it, one per digit (d4 in d3's): the digit's sum, biased per
 // block, with the number of blocks that added to the word in its top byte.  A block
 // that saw a chunk out of range (or Inf / NaN) adds kTopBad in place of d4, which no
-// others' digits outweigh.
-constexpr int kChunkBits = 86; // a chunk's lowest bit lies below this place
+// others' digits outweigh.  The magnitudes of p.q's and r.z's chunks (fx_mag) go beside
+// p.q and r.r and are looked at off the chain: what they say is told at the end of the
+// iteration (us per iteration, without them -> with: 16x16 2.62 -> 2.63, 64x64 2.77 ->
+// 2.82, 97x61 2.99 -> 3.02, 193x255 3.89 -> 3.96, 512x512 14.31 -> 14.41).
 constexpr int kTopBad = 1 << 21;
 constexpr int kCountShift = 56;
 constexpr unsigned long long kOne = 1ull << kCountShift;
@@ -181,8 +183,8 @@ __device__ __forceinline__ double value(const Raw &r)
 }
 
 // A 32-row chunk's FP32 sum as digits, one sum per group of 8 lanes (v and its scale
-// s are theirs): lane j's part of digit j, lane 5 counting sums out of range; false
-// where the lane has none.
+// s are theirs): lane j's part of digit j, lane 5 counting sums out of range, lane 6 the
+// magnitude; false where the lane has none.
 __device__ __forceinline__ bool chunk_digit(float v, int s, int &x)
 {
     const unsigned bits = __float_as_uint(v);
@@ -195,8 +197,11 @@ __device__ __forceinline__ bool chunk_digit(float v, int s, int &x)
         // zero or subnormal (below any scale in use), Inf / NaN, out of range,
         // or digits below the unit
         if (e == 0)
+        {
             m = 0u;
-        bad = e == 255 || (e != 0 && sh >= kChunkBits);
+            sh = 0;
+        }
+        bad = e == 255 || sh >= kChunkBits;
         if (sh < 0)
         {
             m = sh > -25 ? (m + (1u << (-sh - 1))) >> -sh : 0u;
@@ -208,7 +213,9 @@ __device__ __forceinline__ bool chunk_digit(float v, int s, int &x)
     x = j == k ? int((m << off) & 0xffffffu) : int(m >> (24 - off));
     const int sign = int(bits) >> 31;
     x = (x ^ sign) - sign;
-    bool has = unsigned(j - k) < 2u;
+    const int mag = int(fx_mag(m, sh)); // (no branch: k_pcg_wide spilled)
+    x = j == 6 ? mag : x;
+    bool has = unsigned(j - k) < 2u || j == 6;
     if (bad)
     {
         x = 1;
@@ -216,7 +223,7 @@ __device__ __forceinline__ bool chunk_digit(float v, int s, int &x)
     }
     return has;
 }
-// Adds the sums to the block's digits dig[0 .. 5] of their quantity.
+// Adds the sums to the block's digits dig[0 .. 6] of their quantity.
 __device__ __forceinline__ void chunk_add(int *dig, float v, int s, bool on)
 {
     int x;
@@ -234,7 +241,7 @@ __device__ __forceinline__ void digits_add(int *dig, int d, bool on)
         d &= 0xffffff;
     if (j >= 1 && j <= 4)
         d += below;
-    if (on && j < 6 && d != 0)
+    if (on && j < 7 && d != 0)
         atomicAdd(dig + j, d);
 }
 // The sums of a warp's K chunks (the same in every lane; zero where it has
@@ -286,29 +293,31 @@ __device__ __forceinline__ bool combine(long long d0, long long d1, long long d2
     return top >= (1ll << 23) || top < -(1ll << 23);
 }
 
-// A block's digits dig[0 .. 5], read and cleared by the control warp.
+// A block's digits dig[0 .. 6], read and cleared by the control warp.
 struct Digits
 {
     int4 d;
     int top; // d4, or the mark of a chunk out of range
+    int mag; // the chunks' magnitudes (225: below 2^26, in a cluster 60: below 2^24)
 };
 __device__ __forceinline__ Digits take(int *dig)
 {
     Digits r;
     int bad;
+    [[maybe_unused]] int pad;
     const unsigned at = smem_u32(dig);
     asm volatile("ld.volatile.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
                  : "=r"(r.d.x), "=r"(r.d.y), "=r"(r.d.z), "=r"(r.d.w)
                  : "r"(at)
                  : "memory");
-    asm volatile("ld.volatile.shared.v2.u32 {%0, %1}, [%2];"
-                 : "=r"(r.top), "=r"(bad)
+    asm volatile("ld.volatile.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r.top), "=r"(bad), "=r"(r.mag), "=r"(pad)
                  : "r"(at + 16u)
                  : "memory");
     if (bad)
         r.top = kTopBad;
     __syncwarp();
-    if ((threadIdx.x & 31) < 6)
+    if ((threadIdx.x & 31) < 7)
         dig[threadIdx.x & 31] = 0;
     return r;
 }
@@ -332,6 +341,33 @@ __device__ __forceinline__ int4 carried(const Digits &v)
     c.y = int(unsigned(c.y & 0xffffff) | (f & 0xff00u) << 16);
     c.z = int(unsigned(c.z & 0xffffff) | f << 24);
     return c;
+}
+// The same of r.r, in which nothing cancels: a block's sum past d3's 24 bits makes the
+// total out of range by itself, so the upper bytes are free for r.z's magnitudes.
+__device__ __forceinline__ int4 carried_with(const Digits &v, int mag)
+{
+    int4 c = v.d;
+    c.y += c.x >> 24;
+    c.z += c.y >> 24;
+    c.w += c.z >> 24;
+    if ((v.top | (v.d.w >> 24)) != 0)
+        c.w = 1 << 26;
+    c.x = (c.x & 0xffffff) | mag << 24;
+    c.y = (c.y & 0xffffff) | (mag >> 8) << 24;
+    c.z = (c.z & 0xffffff) | (mag >> 16) << 24;
+    return c;
+}
+__device__ __forceinline__ bool decode_with(const int4 *rec, int nblk, int s, Raw &r,
+                                            unsigned long long &mag)
+{
+    int4 c = make_int4(0, 0, 0, 0);
+    if ((threadIdx.x & 31) < nblk)
+        c = rec[threadIdx.x & 31];
+    mag = __reduce_add_sync(kFull, __byte_perm(__byte_perm(c.x, c.y, 0x73), c.z, 0x3710) & 0xffffffu);
+    const int d0 = __reduce_add_sync(kFull, c.x & 0xffffff),
+              d1 = __reduce_add_sync(kFull, c.y & 0xffffff),
+              d2 = __reduce_add_sync(kFull, c.z & 0xffffff), d3 = __reduce_add_sync(kFull, c.w);
+    return combine(d0, d1, d2, d3, s, r);
 }
 // Total of a cluster's nblk records.
 __device__ __forceinline__ bool decode(const int4 *rec, int nblk, int s, Raw &r)
@@ -364,6 +400,22 @@ __device__ __forceinline__ void word_add(unsigned long long *words, const Digits
     asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(words + k), "l"(w)
                  : "memory");
 }
+// The magnitudes: a word each.
+__device__ __forceinline__ void mag_add(unsigned long long *word, int mag)
+{
+    asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(word),
+                 "l"(kOne + (unsigned long long)mag)
+                 : "memory");
+}
+__device__ __forceinline__ bool mags_in(const unsigned long long *p, unsigned long long target,
+                                        unsigned long long (&m)[2])
+{
+    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];"
+                 : "=l"(m[0]), "=l"(m[1])
+                 : "l"(p)
+                 : "memory");
+    return min(m[0] >> kCountShift, m[1] >> kCountShift) >= target;
+}
 // A team's sum words, the same in every lane (one 32-byte request a poll: the
 // team's polls and reductions queue at one L2 slice).
 struct Words
@@ -390,6 +442,12 @@ struct Words
                        r);
     }
 };
+
+__device__ __forceinline__ bool is_noise(const Raw &v, unsigned long long mag)
+{
+    static_assert(kCancelUnit >= 48, "the upper part holds it");
+    return fx_cancels(v.hi >> (kCancelUnit - 48), mag);
+}
 
 // ---- scalars without the FP64 pipe.  |value| = (hi + lo 2^-24) 2^e with hi
 // in [2^23, 2^24): its top 48 bits, the rest dropped (relative error 2^-47).
@@ -486,11 +544,11 @@ __device__ __forceinline__ float ratio(const Top48 &a, const Top48 &b, float rb,
 }
 
 // What the warps of a block share; in a cluster also the blocks' sum records
-// (p.q; r.z; r.r), the barriers they and the z rows are counted on, and where a
-// row of z goes: the blocks whose columns touch rows of this one.
+// (p.q; r.z; r.r; p.q's magnitudes), the barriers they and the z rows are counted on,
+// and where a row of z goes: the blocks whose columns touch rows of this one.
 template <bool CLUSTER> struct Shared
 {
-    alignas(16) int4 rec[3][CLUSTER ? kClusterMax : 1];
+    alignas(16) int4 rec[4][CLUSTER ? kClusterMax : 1];
     alignas(8) unsigned long long bar[3];
     TeamPeer peer[CLUSTER ? kClusterMax : 1];
     int npeer;
@@ -582,14 +640,14 @@ __device__ __forceinline__ void control_warp(const InstDesc &d, const TeamBlock 
     constexpr int kAll = kTeamThreads;
     unsigned long long(*words)[16] = CLUSTER ? nullptr : sync[blockIdx.x - w.rank].words;
     const unsigned bar_p = smem_u32(sh.bar), bar_z = smem_u32(sh.bar + 1);
-    // this lane's peer: block lane % 16, sum lane / 16 (r.z, r.r)
+    // this lane's peer: block lane % 16, sum lane / 16 (p.q and its magnitudes; r.z and r.r)
     const int pr_ = lane & (kClusterMax - 1), pq_ = lane / kClusterMax;
     unsigned to_p = 0, to_z = 0, at_p = 0, at_z = 0;
     if (CLUSTER && pr_ < w.nblk)
     {
         to_p = peer_addr(bar_p, pr_);
         to_z = peer_addr(bar_z, pr_);
-        at_p = peer_addr(smem_u32(&sh.rec[0][w.rank]), pr_);
+        at_p = peer_addr(smem_u32(&sh.rec[3 * pq_][w.rank]), pr_);
         at_z = peer_addr(smem_u32(&sh.rec[1 + pq_][w.rank]), pr_);
     }
     unsigned phase = 0;
@@ -632,9 +690,11 @@ __device__ __forceinline__ void control_warp(const InstDesc &d, const TeamBlock 
             stop = 9;
         float af = 0.f;
         Top48 pq48 = rho48;
+        unsigned long long mag[2] = {0ull, 0ull};
         if (!stop)
         {
             const Digits v = take(dig[0]);
+            mag[0] = (unsigned long long)v.mag;
             bool bad = false;
             if (!multi)
                 bad = decode(v, s_pq, pq);
@@ -642,10 +702,10 @@ __device__ __forceinline__ void control_warp(const InstDesc &d, const TeamBlock 
             {
                 const int4 c = carried(v);
                 if (lane == 0)
-                    mbar_expect(bar_p, 16u * (unsigned(w.nblk) + sc.extra));
+                    mbar_expect(bar_p, 32u * (unsigned(w.nblk) + sc.extra));
                 __syncwarp();
-                if (lane < w.nblk)
-                    peer_store(at_p, to_p, c.x, c.y, c.z, c.w);
+                if (pr_ < w.nblk)
+                    peer_store(at_p, to_p, pq_ ? v.mag : c.x, c.y, c.z, c.w);
                 if (mbar_wait(bar_p, phase, sc.limit))
                     bad = decode(sh.rec[0], w.nblk, s_pq, pq);
                 else
@@ -703,6 +763,14 @@ __device__ __forceinline__ void control_warp(const InstDesc &d, const TeamBlock 
         s_pq = scale_of(pq, pq48);
         if (lane == 0)
             scale[0] = s_pq;
+        bool noise = false;
+        if (CLUSTER) // (while the workers form z)
+        {
+            if (multi)
+                mag[0] = __reduce_add_sync(kFull,
+                                           lane < w.nblk ? unsigned(sh.rec[3][lane].x) : 0u);
+            noise = is_noise(pq, mag[0]);
+        }
         // ---- r.z, r.r and beta
         bar_sync(4, kAll);
         if (*(volatile int *)&sh.err)
@@ -718,11 +786,12 @@ __device__ __forceinline__ void control_warp(const InstDesc &d, const TeamBlock 
         {
             const Digits v1 = take(dig[1]);
             v2 = take(dig[2]);
+            mag[1] = (unsigned long long)v1.mag;
             if (!multi)
                 bad = decode(v1, s_rho, rz);
             else if (CLUSTER)
             {
-                const int4 c1 = carried(v1), c2 = carried(v2);
+                const int4 c1 = carried(v1), c2 = carried_with(v2, v1.mag);
                 const int4 c = pq_ ? c2 : c1;
                 if (lane == 0)
                     mbar_expect(bar_z, 32u * (unsigned(w.nblk) + sc.extra));
@@ -739,6 +808,8 @@ __device__ __forceinline__ void control_warp(const InstDesc &d, const TeamBlock 
             {
                 if (lane < 8)
                     word_add(wd + 4 + (lane & 4), lane < 4 ? v1 : v2, lane & 3);
+                else if (lane < 10)
+                    mag_add(wd + 4 + lane, lane == 8 ? int(mag[0]) : v1.mag);
                 for (;;)
                 {
                     x.load(wd + 4);
@@ -776,7 +847,7 @@ __device__ __forceinline__ void control_warp(const InstDesc &d, const TeamBlock 
             for (;;)
             {
                 y.load(wd + 8);
-                if (y.all_in(target))
+                if (mags_in(wd + 12, target, mag) && y.all_in(target))
                     break;
                 if (++n > sc.limit)
                 {
@@ -787,8 +858,12 @@ __device__ __forceinline__ void control_warp(const InstDesc &d, const TeamBlock 
         if (stop)
             continue; // a wait gave up: told at the next alpha
         bad |= !multi    ? decode(v2, s_rr, rr)
-               : CLUSTER ? decode(sh.rec[2], w.nblk, s_rr, rr)
+               : CLUSTER ? decode_with(sh.rec[2], w.nblk, s_rr, rr, mag[1])
                          : y.decode(w.nblk, s_rr, rr);
+        if (!CLUSTER)
+            noise = is_noise(pq, mag[0] & kSumMask);
+        // (no branches: these are between two exchanges)
+        bad = (int(bad) | int(noise) | int(is_noise(rz, mag[1] & kSumMask))) != 0;
         it++;
         rho_b = rho;
         have_b = true;
