@@ -902,6 +902,13 @@ TeamBlock team_block(const Tables &t, int inst, int rank, int r0, int r1)
     return w;
 }
 
+// Whether a block's rows touch most of its cloth.
+bool numbered_far(const Tables &t, const TeamBlock &w)
+{
+    const int halo = w.halo1 - w.halo0;
+    return halo - (w.row1 - w.row0) > kFarRows && 2 * halo > t.nv;
+}
+
 // An on-chip kernel: k_pcg_team or (half) k_pcg_half, or above four k_pcg_wide, with
 // K rows a thread (0: one, without blocks in registers).
 struct TeamKernel
@@ -961,6 +968,14 @@ bool team_split(const cloth_s *c, int i, bool skew_kernel, int blocks, TeamKerne
         else
             bytes = team_smem_bytes(halo, nr, h.width, skew, team_reg_slots(tk.K, skew_kernel),
                                     cluster);
+        // k_pcg_half and k_pcg_wide over the whole GPU poll the z rows of the halo 480 at a
+        // time, the older kernel stages them behind a barrier: faster where a block
+        // touches most of its cloth (random order, us per iteration: 136^2 23.2, the older
+        // one 19.9; 64 x 64^2 57.2, 39.7; 20 x 125^2 121.6, 70.1; with a third of the
+        // columns or less k_pcg_wide is as fast or faster: 400^2 shuffled within 5,000
+        // rows 32.8, 37.3)
+        if (tk.half && !cluster && numbered_far(t, w))
+            fits = false;
         if (!fits || bytes > cap)
         {
             work.resize(first);
@@ -1055,17 +1070,25 @@ bool plan_team(cloth_ctx *ctx, const Batch *b, TeamKernel tk, std::vector<TeamBl
     if (n > G)
         return false;
     const size_t cap = size_t(ctx->max_smem_optin) - 4096;
+    // blocks in proportion to the rows, at least one; where the ones that this gives to
+    // small cloths leave too few, in proportion to what they leave
     long long total = 0;
     for (auto *c : b->members)
         total += c->tab.nv;
+    auto share = [&](int blocks, int i) {
+        const int nv = b->members[i]->tab.nv;
+        const long long s = (long long)blocks * nv / std::max(1ll, total);
+        return std::max(1, std::min<int>(int(s), (nv + kTeamMinRows - 1) / kTeamMinRows));
+    };
+    int all = 0, shared = G;
+    for (int i = 0; i < n; i++)
+        all += share(G, i);
+    if (all > G)
+        shared = G - (n - 1);
     work.clear();
     for (int i = 0; i < n; i++)
     {
-        const int nv = b->members[i]->tab.nv;
-        const long long share =
-            std::max(1ll, (long long)(G - (n - 1)) * nv / std::max(1ll, total));
-        const int want =
-            std::max(1, std::min<int>(int(share), (nv + kTeamMinRows - 1) / kTeamMinRows));
+        const int want = share(shared, i);
         if (!team_split(b->members[i], i, b->skew, want, tk, false, cap, work, smem))
             return false;
     }
@@ -1124,9 +1147,15 @@ ClusterChoice cluster_choice(const cloth_ctx *ctx, const cloth_s *c, bool skew_k
 // Plan of a set as one launch per size of cluster, side by side, each cloth with
 // cluster_choice's; clusters start, the longest solves first, as SMs come free.
 // While the set leaves SMs idle the clusters are doubled.  False when a cloth fits
-// no cluster.
-bool plan_queue(cloth_ctx *ctx, Batch *b, int *rc)
+// no cluster, or one numbered without locality would wait for clusters of 16 to end: a
+// cluster's iteration is then 6.5 us at 64^2 and 8.8 at 80^2 (in grid order 2.8 and 3.0),
+// and the kernels that run the set at once are faster (30 x 64^2: 32.5 us as a queue, 20.0;
+// 160 x 64^2: 150, the graph loop 126).  rows: those of a block, wave after wave.
+using QueuePlan = std::vector<std::pair<PersistLaunch, std::vector<TeamBlock>>>;
+bool plan_queue(cloth_ctx *ctx, const Batch *b, QueuePlan &plans, long long *rows)
 {
+    plans.clear();
+    *rows = 0;
     const int n = int(b->members.size());
     std::vector<ClusterChoice> choice(n);
     std::vector<TeamBlock> work;
@@ -1159,19 +1188,36 @@ bool plan_queue(cloth_ctx *ctx, Batch *b, int *rc)
     std::map<std::tuple<int, int, int>, std::vector<int>> groups;
     for (int i = 0; i < n; i++)
         groups[std::make_tuple(-choice[i].C, -int(choice[i].k.half), -choice[i].k.K)].push_back(i);
-    std::vector<std::pair<PersistLaunch, std::vector<TeamBlock>>> plans;
     for (auto &g : groups)
     {
         PersistLaunch l;
         const ClusterChoice &c = choice[g.second[0]];
         if (!plan_cluster(ctx, b, g.second, c.k, c.C, false, work, l))
             return false;
+        const int at_once = resident_clusters(ctx, l.func, c.C, work.size(), l.smem);
+        const int waves = (int(g.second.size()) + at_once - 1) / at_once;
+        int most = 0;
+        bool far = false;
+        for (const TeamBlock &w : work)
+        {
+            most = std::max(most, w.row1 - w.row0);
+            far = far || (w.inst >= 0 && numbered_far(b->members[size_t(w.inst)]->tab, w));
+        }
+        if (far && c.C == kClusterMax && waves > 1)
+            return false;
+        *rows += (long long)waves * most;
         plans.emplace_back(l, work);
     }
-    for (auto &p : plans)
-        if (*rc == CLOTH_OK)
-            *rc = add_launch(b, p.first, p.second, sizeof(unsigned long long), sizeof(TeamBlock));
     return true;
+}
+
+int add_queue(Batch *b, const QueuePlan &plans)
+{
+    int rc = CLOTH_OK;
+    for (auto &p : plans)
+        if (rc == CLOTH_OK)
+            rc = add_launch(b, p.first, p.second, sizeof(unsigned long long), sizeof(TeamBlock));
+    return rc;
 }
 
 // Team plan of the persistent solver: every instance gets blocks in
@@ -1204,9 +1250,10 @@ int plan_persistent(cloth_ctx *ctx, Batch *b)
         const TeamKernel one{b->skew ? 0 : 1, false};
         if (plan_cluster(ctx, b, all, one, C, true, work, l))
             return add_launch(b, l, work, sizeof(unsigned long long), sizeof(TeamBlock));
-        int rc = CLOTH_OK;
-        if (most <= kClusterMax * kTeamWorkers && plan_queue(ctx, b, &rc))
-            return rc;
+        QueuePlan queue;
+        long long queue_rows = 0;
+        if (most <= kClusterMax * kTeamWorkers && plan_queue(ctx, b, queue, &queue_rows))
+            return add_queue(b, queue);
         // Teams over the whole GPU: the whole matrix on chip where it fits (256^2:
         // 4.2 us with one row a thread), else the stored blocks (300^2: 6.4, the
         // kernel that reads the matrix from L2 13.0; 512^2: 13.8 and 21.4), with
@@ -1216,26 +1263,32 @@ int plan_persistent(cloth_ctx *ctx, Batch *b)
                              TeamKernel{3, true}, TeamKernel{4, true}})
             if (plan_team(ctx, b, k, work, l))
                 return add_launch(b, l, work, sizeof(TeamSync), alignof(TeamSync) * 64);
-        if (plan_queue(ctx, b, &rc))
-            return rc;
         // The matrix read from memory: r and dx on chip while three quarters of L2 hold
         // the matrix (640^2, 90 MB: 26.6 us per iteration, 30.5 without, the older kernel
         // 44.4), else read too, for more loads in flight (680^2, 102 MB: 35.4; 760^2: 42.3,
         // 48.3 with them on chip, 59.7; 1024^2: 92.0, the older kernel 100.3)
-        if (!b->skew)
-        {
-            size_t matrix = 0;
-            for (auto *c : b->members)
-                matrix += size_t(c->tab.nv) * (size_t(c->h.width_up) * 28 + size_t(c->h.width_lo) * 4);
-            int l2 = 0;
-            const bool kept = cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, ctx->device) ==
-                                  cudaSuccess &&
-                              matrix <= size_t(l2) / 4 * 3;
-            for (int k : {kWideRows, kWidestRows})
-                if ((kept || k == kWidestRows) &&
-                    plan_team(ctx, b, TeamKernel{k, true}, work, l))
-                    return add_launch(b, l, work, sizeof(TeamSync), alignof(TeamSync) * 64);
-        }
+        size_t matrix = 0;
+        for (auto *c : b->members)
+            matrix += size_t(c->tab.nv) * (size_t(c->h.width_up) * 28 + size_t(c->h.width_lo) * 4);
+        int l2 = 0;
+        const bool kept =
+            cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, ctx->device) == cudaSuccess &&
+            matrix <= size_t(l2) / 4 * 3;
+        bool wide = !b->skew && kept && plan_team(ctx, b, TeamKernel{kWideRows, true}, work, l);
+        // Cloths that clusters hold, as a queue, unless its last wave leaves too much of
+        // the GPU idle: a row of a block is 10 to 11 ns of k_pcg_wide's iteration and 7 to 8
+        // of k_pcg_half's in a cluster (10 x 172^2: 28.3 us as a queue, 21.9; 19 x 125^2:
+        // 24.5, 22.1; 14 x 172^2: 28.7, 35.1)
+        long long wide_rows = 0;
+        if (wide)
+            for (const TeamBlock &w : work)
+                wide_rows = std::max(wide_rows, (long long)(w.row1 - w.row0));
+        if (plan_queue(ctx, b, queue, &queue_rows) && !(wide && 4 * wide_rows <= 3 * queue_rows))
+            return add_queue(b, queue);
+        if (!wide)
+            wide = !b->skew && plan_team(ctx, b, TeamKernel{kWidestRows, true}, work, l);
+        if (wide)
+            return add_launch(b, l, work, sizeof(TeamSync), alignof(TeamSync) * 64);
     }
     work.clear();
     const size_t smem_cap_bytes =

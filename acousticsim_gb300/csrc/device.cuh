@@ -328,6 +328,9 @@ __host__ __device__ inline size_t half_smem_bytes(int halo, int rows, int ext, i
 // k_pcg_wide: rows per thread of its two variants (the first holds r, dx and the
 // inverse diagonal blocks on chip), and a block's dynamic shared memory.
 constexpr int kWideRows = 8, kWidestRows = 15;
+// Halo rows of other blocks above which a block's rows count as numbered without
+// locality where they touch more than half of its cloth.
+constexpr int kFarRows = 2048;
 __host__ __device__ constexpr bool wide_hold(int k) { return k <= kWideRows; }
 __host__ __device__ inline size_t wide_smem_bytes(int halo, int rows, int k)
 {
