@@ -68,8 +68,9 @@ __global__ void k_pcg_persistent_gm_skew(InstDesc *const *descs, const TeamBlock
 __global__ void k_pcg1_persistent(InstDesc *const *descs, const TeamBlock *work, int halo_cap,
                                   int rows_cap, SpinCfg sc);
 
-// k_pcg_team (1 or 2 rows per thread; 0: one, no blocks in registers) or
-// k_pcg_half (half; 2 to 4), its teams clusters or not; arguments (descs, work, sync, spin)
+// k_pcg_team (1 or 2 rows per thread; 0: one, no blocks in registers), k_pcg_half (half;
+// 2 to 4) or k_pcg_wide (half; kWideRows or kWidestRows, no clusters, no skew parts), its
+// teams clusters or not; arguments (descs, work, sync, spin)
 const void *team_kernel(int k, bool half, bool skew, bool cluster);
 
 // ---------------------------------------------------------------- plain path

@@ -2,10 +2,11 @@
 //
 // One cooperative launch runs every PCG iteration of every instance of a
 // launch set.  A block owns a contiguous row range of one instance and keeps
-// everything it iterates on next to its SM: the rows' 3x3 blocks and local
-// column indices and p over the block's column range (halo) in shared memory,
-// dx, r, z, p and the inverse diagonal block of its rows in registers.  Per
-// iteration only boundary rows of z and two team sums cross the L2.
+// everything it iterates on next to its SM: the rows' 3x3 blocks, local column
+// indices and inverse diagonal blocks and p over the block's column range (halo)
+// in shared memory (the first blocks of a row in registers), dx, r, z and p of its
+// rows in registers.  Per iteration its rows of z are stored to the L2, those of
+// its halo read from there, and two team sums exchanged.
 //
 // What bounds it: with the matrix on chip an iteration is a chain of
 // latencies - two team sums (an L2 reduction and its poll, ~1,400 cycles each)
@@ -18,8 +19,8 @@
 //     polls the rows it needs while the r.z sum is under way;
 //   * a control warp folds the chunk sums, talks to the team and forms alpha
 //     and beta from integers and FP32 (FP64 division costs ~1,000 cycles on
-//     this GPU's narrow FP64 pipe); the FP64 scalars that the next fixed-point
-//     scales and the result need are formed while the other warps compute.
+//     this GPU's narrow FP64 pipe) unless that leaves their rounding open, and the
+//     next fixed-point scales from exponents; the FP64 scalars are formed at the end.
 // The arithmetic is that of the other PCG drivers, bit for bit.
 //
 // Measured (one GB300, us per PCG iteration over a whole step, before: the
@@ -1614,7 +1615,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
                 }
                 return b;
             };
-            // upper planes that are not on chip: the first three in flight from here
+            // upper planes that are not on chip: the first kPre in flight from here
             constexpr int kPre = 2;
             Block f[kPre];
 #pragma unroll
