@@ -1216,7 +1216,7 @@ int add_queue(Batch *b, const QueuePlan &plans)
     int rc = CLOTH_OK;
     for (auto &p : plans)
         if (rc == CLOTH_OK)
-            rc = add_launch(b, p.first, p.second, sizeof(unsigned long long), sizeof(TeamBlock));
+            rc = add_launch(b, p.first, p.second, 0, sizeof(TeamBlock));
     return rc;
 }
 
@@ -1249,7 +1249,7 @@ int plan_persistent(cloth_ctx *ctx, Batch *b)
         const int C = most <= kTeamAloneRows ? 1 : kClusterMax;
         const TeamKernel one{b->skew ? 0 : 1, false};
         if (plan_cluster(ctx, b, all, one, C, true, work, l))
-            return add_launch(b, l, work, sizeof(unsigned long long), sizeof(TeamBlock));
+            return add_launch(b, l, work, 0, sizeof(TeamBlock));
         QueuePlan queue;
         long long queue_rows = 0;
         if (most <= kClusterMax * kTeamWorkers && plan_queue(ctx, b, queue, &queue_rows))
@@ -1532,6 +1532,7 @@ int build_graph(Batch *b, bool full, cudaGraphExec_t *exec)
             if (rc != CLOTH_OK)
                 break;
             PersistArgs args(b, l);
+            // (clusters have none)
             cudaMemsetParams mp;
             std::memset(&mp, 0, sizeof(mp));
             mp.dst = l.d_sync;
@@ -1539,9 +1540,10 @@ int build_graph(Batch *b, bool full, cudaGraphExec_t *exec)
             mp.elementSize = 4;
             mp.width = l.sync_bytes / 4;
             mp.height = 1;
-            cudaGraphNode_t m = nullptr;
-            if (cudaGraphAddMemsetNode(&m, g, root ? &root : nullptr, root ? 1 : 0, &mp) !=
-                cudaSuccess)
+            cudaGraphNode_t m = root;
+            if (l.sync_bytes &&
+                cudaGraphAddMemsetNode(&m, g, root ? &root : nullptr, root ? 1 : 0, &mp) !=
+                    cudaSuccess)
             {
                 rc = fail(CLOTH_ERR_CUDA, "cudaGraphAddMemsetNode failed");
                 break;
@@ -1553,7 +1555,7 @@ int build_graph(Batch *b, bool full, cudaGraphExec_t *exec)
             p.blockDim = dim3(l.block);
             p.sharedMemBytes = unsigned(l.smem);
             p.kernelParams = args.of(l);
-            if (cudaGraphAddKernelNode(&n, g, &m, 1, &p) != cudaSuccess)
+            if (cudaGraphAddKernelNode(&n, g, m ? &m : nullptr, m ? 1 : 0, &p) != cudaSuccess)
                 rc = fail(CLOTH_ERR_CUDA, "cudaGraphAddKernelNode(persistent) failed");
             else
             {
@@ -1655,7 +1657,8 @@ int launch_persistent(Batch *b)
     for (auto &l : b->launches)
     {
         PersistArgs args(b, l);
-        CK(cudaMemsetAsync(l.d_sync, 0, l.sync_bytes, ctx->stream));
+        if (l.sync_bytes)
+            CK(cudaMemsetAsync(l.d_sync, 0, l.sync_bytes, ctx->stream));
         cudaLaunchAttribute at = persist_attribute(l);
         cudaLaunchConfig_t cfg;
         std::memset(&cfg, 0, sizeof(cfg));

@@ -602,7 +602,8 @@ def headline_roofline(args, cloth, solver, prof, prof_iters) -> dict:
     ach_survey = survey_launch / (launch_ms * 1e-3) / 1e9
     kshort = kname.split()[0]
     dram_it = ncu_dram_per_iteration(kshort)
-    return {"bound": "hbm", "kernel": kname,
+    resident = bool(dram_it is not None and dram_it < 0.2 * per_iter)
+    return {"bound": "l2 and team sums" if resident else "hbm", "kernel": kname,
             "achieved": achieved, "peak": peak["hbm_gbs"], "unit": "GB/s",
             "frac": achieved / peak["hbm_gbs"], "peak_source": f"{peak['source']} hbm_gbs",
             "achieved_survey_bytes": ach_survey,
@@ -611,7 +612,7 @@ def headline_roofline(args, cloth, solver, prof, prof_iters) -> dict:
             "traffic_source": "profiles/ncu_traffic.json (ncu capture of this workload, DRAM "
                               "bytes per PCG iteration, scaled by iterations)",
             "dram_bytes_per_iteration": dram_it,
-            "l2_resident": bool(dram_it is not None and dram_it < 0.2 * per_iter),
+            "l2_resident": resident,
             "algorithmic_bytes_per_launch": bytes_launch,
             "algorithmic_bytes_per_iteration": per_iter,
             "survey_bytes_per_iteration": survey_iter,
@@ -664,13 +665,18 @@ def stratified(keys, count: int) -> list[int]:
     return [int(order[k]) for k in pos]
 
 
+TEAM_WORKERS = 480  # worker threads of an on-chip PCG block (kTeamWorkers)
+
+
 def on_chip_kernel(nv: int, skew: bool) -> str:
     """The kernel that the persistent solver runs for one grid cloth of nv
-    vertices (rows per thread over 152 blocks of 480 workers)."""
-    rows = nv / (152 * 480)
+    vertices, by rows per thread over the GPU (skew parts leave shared memory
+    for three of k_pcg_half's four)."""
+    import torch
+    rows = nv / (torch.cuda.get_device_properties(0).multi_processor_count * TEAM_WORKERS)
     if rows <= 1:
         return "k_pcg_team"
-    if rows <= 4:
+    if rows <= (3 if skew else 4):
         return "k_pcg_half"
     if rows <= 15 and not skew:
         return "k_pcg_wide"
