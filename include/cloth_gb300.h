@@ -33,7 +33,8 @@ enum cloth_status {
     CLOTH_ERR_OOM = 3,         /* device allocation failed */
     CLOTH_ERR_BUDGET = 4,      /* admission refused: device-memory budget */
     CLOTH_ERR_MESH = 5,        /* mesh unsupported (non-manifold edge, row wider than 32) */
-    CLOTH_ERR_NAN = 6,         /* NaN/Inf met in the solve (per-instance status) */
+    CLOTH_ERR_NAN = 6,         /* NaN/Inf met in the solve, or a sum that FP32 does not
+                                  resolve (per-instance status) */
     CLOTH_ERR_BREAKDOWN = 7,   /* PCG denominator was zero (alpha or beta clamped) */
     CLOTH_ERR_MAXITER = 8,     /* solve stopped at max_iters above tolerance (per-instance status) */
     CLOTH_ERR_TIMEOUT = 9,     /* a bounded device wait gave up */
@@ -151,7 +152,7 @@ int cloth_ctx_reset_profile(cloth_ctx *ctx);
 /* Preferred PCG driver for launch sets built after the call. */
 int cloth_ctx_set_solver(cloth_ctx *ctx, int solver);
 /* Launch sets of more cloths than blocks are resident at once, with one among
- * them that no thread-block cluster holds (above ~16,000 vertices), run the graph
+ * them that no thread-block cluster holds (above ~30,000 vertices), run the graph
  * loop; with the persistent solver (two barriers) chosen, such a set hands
  * its last max_instances iterating cloths to the persistent kernel, whose
  * arithmetic is the graph loop's bit for bit (results do not change; the few
