@@ -20,7 +20,7 @@
 //   k_srv_status  one record per request on the GPU; ended ones are closed
 //
 // 48 cloths of 16^2 to 128^2 vertices, all at once, with their positions set and
-// read: 17.7 ms when every request ran in the graph loop, 8.9 ms now.
+// read: 17.7 ms when every request ran in the graph loop, 9.2 ms now.
 //
 // Up to two chunks are in flight: while chunk k runs, the host reads the
 // status of chunk k-1, retires the requests that ended (their pool memory is
