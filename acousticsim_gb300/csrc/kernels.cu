@@ -1856,7 +1856,8 @@ __device__ __forceinline__ void reduce_body(InstDesc *const *descs, const int *i
             const double rho0 = st.rho;
             const double rho_new = fx_total(stp, bq, 1, fx_scale(rho0), &bad);
             const double rr = fx_total(stp, bq, 2, fx_scale(st.rr), &bad);
-            if (fx_cancels(stp, bq, 0) || fx_cancels(stp, bq, 1))
+            if (fx_cancels(stp, bq, 0) || fx_cancels(stp, bq, 1) || fx_from_zero(rho0, rho_new) ||
+                fx_from_zero(st.rr, rr))
                 bad = 1;
             fx_clear(stp, (it0 + 1) % 3);
             st.beta = (rho0 == 0.0) ? 0.0 : rho_new / rho0;
@@ -2574,7 +2575,8 @@ __device__ __forceinline__ void pcg_persistent_body(InstDesc *const *descs,
             int bad = 0;
             const double rho_new = team_value(1, bq, s1q, &bad);
             const double rr = team_value(2, bq, s2q, &bad);
-            if (fx_cancels(st, bq, 0) || fx_cancels(st, bq, 1))
+            if (fx_cancels(st, bq, 0) || fx_cancels(st, bq, 1) || fx_from_zero(s_rho, rho_new) ||
+                fx_from_zero(s_rr, rr))
                 bad = 1;
             s_beta = (s_rho == 0.0) ? 0.0 : rho_new / s_rho;
             s_rho = rho_new;
@@ -2863,7 +2865,8 @@ __global__ void __launch_bounds__(kPBlock, 1)
             const double gam = team_value(0, bq, bc_s[0], &bad);
             const double del = team_value(1, bq, bc_s[1], &bad);
             const double rr = team_value(2, bq, bc_s[2], &bad);
-            if (fx_cancels(st, bq, 0) || fx_cancels(st, bq, 1))
+            if (fx_cancels(st, bq, 0) || fx_cancels(st, bq, 1) || fx_from_zero(s_gam, gam) ||
+                fx_from_zero(s_rr, rr))
                 bad = 1;
             int stop = 0; // 0 go on, 1 converged, else a status code
             double beta = 0.0, alpha = s_alpha;

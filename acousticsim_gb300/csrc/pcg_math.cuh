@@ -133,7 +133,8 @@ __device__ __forceinline__ void fx_split(float v, int s, long long &H,
 // Which sums count, in every driver alike: each 32-row chunk below 2^(kChunkBits + 24)
 // units and finite, their exact total within 2^95, and (p.q and r.z, judged at the end
 // of the iteration) the total not so far below the sum of the chunks' magnitudes that
-// the chunks' FP32 rounding leaves nothing of it.
+// the chunks' FP32 rounding leaves nothing of it, nor (r.z and r.r) one that rises
+// from zero.
 //
 // The limbs hold the total modulo 2^96, so chunks of 2^75 units and more, which are
 // rare (a sum's last value has about 2^70), are counted in units of 2^72 too; the
@@ -217,6 +218,12 @@ __device__ __forceinline__ bool fx_cancels(const InstState *st, int bq, int q)
 {
     const long long H = (long long)(__ldcg(&st->acc[bq][q][0]) + (__ldcg(&st->acc[bq][q][1]) >> 32));
     return fx_cancels(H >> (kCancelUnit - 32), __ldcg(&st->acc_mag[bq][q]));
+}
+// A residual that had gone below FP32's range and comes back (a solve without tolerances
+// that goes on past its end): rounding noise, which grows without bound.
+__device__ __forceinline__ bool fx_from_zero(double last, double now)
+{
+    return last == 0.0 && now != 0.0;
 }
 // A sum's total; *bad where it is out of range.
 __device__ __forceinline__ double fx_total(const InstState *st, int bq, int q, int s, int *bad)

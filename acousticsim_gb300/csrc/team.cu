@@ -671,6 +671,7 @@ __device__ __forceinline__ void control_warp(const InstDesc &d, const TeamBlock 
     int to_check = check_every - 1 - (it0 + check_every - 1) % check_every;
     Top48 rho48 = top48(rho);
     float rb_rho = recip(rho48);
+    bool rr_was_zero = rr.hi == 0 && rr.lo == 0ull;
     int s_pq = fx_scale(__ldcg(&st->pq)), s_rho = fx_scale(__ldcg(&st->rho)),
         s_rr = fx_scale(__ldcg(&st->rr));
     const unsigned long long target = (unsigned long long)w.nblk + sc.extra;
@@ -864,7 +865,9 @@ __device__ __forceinline__ void control_warp(const InstDesc &d, const TeamBlock 
         if (!CLUSTER)
             noise = is_noise(pq, mag[0] & kSumMask);
         // (no branches: these are between two exchanges)
-        bad = (int(bad) | int(noise) | int(is_noise(rz, mag[1] & kSumMask))) != 0;
+        bad = (int(bad) | int(noise) | int(is_noise(rz, mag[1] & kSumMask)) |
+               int(rho48.hi == 0u && new48.hi != 0u) |
+               int(rr_was_zero && (rr.hi | (long long)rr.lo) != 0)) != 0;
         it++;
         rho_b = rho;
         have_b = true;
@@ -872,6 +875,7 @@ __device__ __forceinline__ void control_warp(const InstDesc &d, const TeamBlock 
         rho48 = new48;
         rb_rho = recip(rho48);
         const Top48 r48 = top48(rr);
+        rr_was_zero = r48.hi == 0u;
         s_rho = scale_of(rho, rho48);
         s_rr = scale_of(rr, r48);
         if (lane == 0)

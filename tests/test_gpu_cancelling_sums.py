@@ -54,3 +54,22 @@ def test_on_chip_solve_that_stalls_is_escalated(built, n, kb, noise):
     ctx.close()
     assert st["status"] == "OK" and st["solver"] == "escalated_fp64", st
     assert st["rel_residual"] <= 1e-6 and np.isfinite(x).all()
+
+
+# without tolerances a solve goes on past its end: the residual leaves FP32's range, and
+# noise comes back.  A strip and a square, the older kernels among the drivers
+@pytest.mark.parametrize("h,w,density", [(5, 122, 0.0125), (24, 24, 0.1)])
+def test_residual_that_comes_back_from_zero(built, h, w, density):
+    from acousticsim_gb300 import ClothContext, params
+    conf = dict(_conf(2, 350.0), subdivision=[h - 1, w - 1], cloth_density=density,
+                cloth_bending_model="dihedral", cloth_bending_stiffness=[3e-4, 3e-4])
+    p = params(max_iters=6000, rel_tol=0.0, abs_tol=0.0)
+    ctx = ClothContext(0)
+    ctx.set_escalation(False)
+    st = [_step(ctx, s, conf, 1e-3, p)[0] for s in ("persistent", "graph_loop")]
+    assert st[0]["status"] == st[1]["status"] == "NAN", st
+    assert st[0]["iters"] == st[1]["iters"]
+    ctx.set_escalation(True)
+    for s in ("persistent", "graph_loop", "persistent_1b"):
+        assert _step(ctx, s, conf, 1e-3, p)[0]["status"] == "OK"
+    ctx.close()
