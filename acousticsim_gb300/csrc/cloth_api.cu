@@ -696,7 +696,9 @@ int cloth::detail::sync_desc(cloth_s *c)
 {
     if (!c->desc_dirty)
         return CLOTH_OK;
-    CK(cudaMemcpy(c->d_desc, &c->h, sizeof(InstDesc), cudaMemcpyHostToDevice));
+    // (in the stream's order: the kernels of an earlier call may still be reading it)
+    CK(cudaMemcpyAsync(c->d_desc, &c->h, sizeof(InstDesc), cudaMemcpyHostToDevice,
+                       c->ctx->stream));
     c->desc_dirty = false;
     return CLOTH_OK;
 }
@@ -796,13 +798,14 @@ int make_batch(cloth_ctx *ctx, const std::vector<cloth_s *> &members,
     b->d_tt = reinterpret_cast<Tile *>(b->mem + o_tt);
     b->d_ctl = reinterpret_cast<BatchCtl *>(b->mem + o_c);
     BatchCtl ctl = {0, b->n_rt, b->n_tt, 0, 0, {0, 0, 0}};
-    CK(cudaMemcpy(b->d_descs, descs.data(), descs.size() * sizeof(InstDesc *),
-                  cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(b->d_inst, inst.data(), inst.size() * sizeof(int),
-                  cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(b->d_rt, rt.data(), rt.size() * sizeof(Tile), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(b->d_tt, tt.data(), tt.size() * sizeof(Tile), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(b->d_ctl, &ctl, sizeof(ctl), cudaMemcpyHostToDevice));
+    const cudaStream_t st = ctx->stream;
+    CK(cudaMemcpyAsync(b->d_descs, descs.data(), descs.size() * sizeof(InstDesc *),
+                       cudaMemcpyHostToDevice, st));
+    CK(cudaMemcpyAsync(b->d_inst, inst.data(), inst.size() * sizeof(int),
+                       cudaMemcpyHostToDevice, st));
+    CK(cudaMemcpyAsync(b->d_rt, rt.data(), rt.size() * sizeof(Tile), cudaMemcpyHostToDevice, st));
+    CK(cudaMemcpyAsync(b->d_tt, tt.data(), tt.size() * sizeof(Tile), cudaMemcpyHostToDevice, st));
+    CK(cudaMemcpyAsync(b->d_ctl, &ctl, sizeof(ctl), cudaMemcpyHostToDevice, st));
     // one tile per block while that fits in a few waves; grid-stride beyond
     auto cap = [&](int occ) { return std::max(1, ctx->num_sms * occ * 8); };
     b->grid_tri = std::max(1, std::min(b->n_tt, cap(ctx->occ_tri)));
@@ -822,7 +825,7 @@ int make_batch(cloth_ctx *ctx, const std::vector<cloth_s *> &members,
         (ctx->solver == CLOTH_SOLVER_PERSISTENT || ctx->solver == CLOTH_SOLVER_PERSISTENT_2B))
     {
         b->hand_off = ho;
-        CK(cudaMemcpy(&b->d_ctl->hand_off, &ho, sizeof(int), cudaMemcpyHostToDevice));
+        CK(cudaMemcpyAsync(&b->d_ctl->hand_off, &ho, sizeof(int), cudaMemcpyHostToDevice, st));
     }
     out = std::move(b);
     return CLOTH_OK;
@@ -882,8 +885,8 @@ int add_launch(Batch *b, PersistLaunch l, const std::vector<TeamBlock> &work, si
     l.grid = int(work.size());
     b->launches.push_back(l);
     b->persist_ok = true;
-    CK(cudaMemcpy(l.d_work, work.data(), work.size() * sizeof(TeamBlock),
-                  cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(l.d_work, work.data(), work.size() * sizeof(TeamBlock),
+                       cudaMemcpyHostToDevice, b->ctx->stream));
     return CLOTH_OK;
 }
 
@@ -2800,13 +2803,14 @@ int cloth_set_material(cloth_t *c, const cloth_material *mat)
         for (int v = 0; v < t.nv; v++)
             for (int s = 0; s < t.rowptr[v + 1] - t.rowptr[v]; s++)
                 kb[size_t(s) * c->h.stride + v] = t.kbend[size_t(t.rowptr[v]) + s];
-        CK(cudaMemcpy(const_cast<float *>(c->h.kb), kb.data(), kb.size() * sizeof(float),
-                      cudaMemcpyHostToDevice));
+        CK(cudaMemcpyAsync(const_cast<float *>(c->h.kb), kb.data(), kb.size() * sizeof(float),
+                           cudaMemcpyHostToDevice, c->ctx->stream));
         if (mt.bending_model == 1 && c->tab.n_dih > 0)
         {
             rebuild_dihedral_factor(c->mesh, mt, c->tab);
-            CK(cudaMemcpy(const_cast<double *>(c->h.dfac), c->tab.dih_factor.data(),
-                          c->tab.dih_factor.size() * sizeof(double), cudaMemcpyHostToDevice));
+            CK(cudaMemcpyAsync(const_cast<double *>(c->h.dfac), c->tab.dih_factor.data(),
+                               c->tab.dih_factor.size() * sizeof(double),
+                               cudaMemcpyHostToDevice, c->ctx->stream));
         }
     }
     set_material_fields(c);
@@ -3372,8 +3376,10 @@ int cloth_step_plain(cloth_t *c, double dt, const cloth_solve_params *params,
     if (rc != CLOTH_OK)
         return rc;
     // keep the library's device state in step, so GetPos and the fast path see it
-    CK(cudaMemcpy(c->h.x64, c->plain_x.data(), c->plain_x.size() * 8, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(c->h.xp64, c->plain_xp.data(), c->plain_xp.size() * 8, cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(c->h.x64, c->plain_x.data(), c->plain_x.size() * 8,
+                       cudaMemcpyHostToDevice, c->ctx->stream));
+    CK(cudaMemcpyAsync(c->h.xp64, c->plain_xp.data(), c->plain_xp.size() * 8,
+                       cudaMemcpyHostToDevice, c->ctx->stream));
     k_sync_x32<<<std::min(1024, (n + 255) / 256), 256, 0, c->ctx->stream>>>(c->d_desc);
     CK(cudaGetLastError());
     if (c->drag_vid >= 0)
